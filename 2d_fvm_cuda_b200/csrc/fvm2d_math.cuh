@@ -273,7 +273,7 @@ __device__ __forceinline__ Cell<Real> conservative_update(const Cell<Real> &U, c
 //
 // RefOrder: the reference's expressions in the reference's order (above).
 // Hoisted:  the same mathematics with the reciprocals hoisted and shared
-//           (1/rho_l and 1/rho_r from one division; 1/(rho a) per side as
+//           (1/rho of the contact's side only; 1/(rho a) per side as
 //           1/sqrt(g p rho), with a = g p/(rho a); the second side's 1/c and
 //           1/(c_l + c_r) from one division; 1/c of the first side and
 //           1/rho_star: 4 divisions and 2 reciprocal square roots per
@@ -395,14 +395,15 @@ __device__ __forceinline__ Real limited_slope_hoisted(Real m, Real c, Real p, Re
 // implies dc d2 > 0: d1, d2 nonzero of one sign puts m, c, p in strict order,
 // so dc = fl(p - m) has that sign and |dc| >= |d1| (rounding is monotonic),
 // hence |dc d2| >= |d1 d2| > 0; then dc != 0 and the result takes its sign.
-// The branch skips the minima where the slope is zero (constant regions):
-// measured 2.4% off the FP64 step at 4096^2, where computing them
-// unconditionally (a select) cost 7%.
+// The minima are formed for every cell and selected: four fields without a
+// branch between them overlap their chains (4096^2 step of a varied flow in
+// tiles: 1627 -> 1587 us; a branch around the minima pays only where the
+// flow is constant).
 __device__ __forceinline__ double limited_slope_hoisted(double m, double c, double p, double hrh, double rha)
 {
     const double d1 = c - m, d2 = p - c, dc = p - m;
-    if (d1 * d2 > 0.0) return copysign(rmin(fabs(dc) * hrh, rha * rmin(fabs(d1), fabs(d2))), dc);
-    return 0.0;
+    const double a = rmin(fabs(dc) * hrh, rha * rmin(fabs(d1), fabs(d2)));
+    return d1 * d2 > 0.0 ? copysign(a, dc) : 0.0;
 }
 
 // Single precision: the same choices with the min/max and sign instructions
@@ -415,23 +416,49 @@ __device__ __forceinline__ float limited_slope_hoisted(float m, float c, float p
     return d1 * d2 > 0.f ? copysignf(a, dc) : 0.f;
 }
 
+// Products of the constants of a sweep, formed where they are used; a kernel
+// that keeps its constants in memory keeps the products there (TileConsts in
+// fvm2d_tile.cuh) and overloads these.
+template <typename Real>
+__device__ __forceinline__ Real half_h(const SweepConsts<Real> &K) { return K.h * Real(0.5); }
+template <typename Real>
+__device__ __forceinline__ Real half_rh(const SweepConsts<Real> &K) { return K.rh * Real(0.5); }
+template <typename Real>
+__device__ __forceinline__ Real alpha_rh(const SweepConsts<Real> &K) { return K.rh * K.alpha; }
+template <typename Real>
+__device__ __forceinline__ Real half_k(const SweepConsts<Real> &K) { return K.k * Real(0.5); }
+
+// Every sum of a product below is written as an fma or as two roundings, and
+// the FP64 build is compiled without contraction, so each copy of this
+// arithmetic (walkers, tiles, batches, taped steps) rounds alike.
 struct Hoisted {
-    template <typename Real>
+    template <typename Real, class Consts>
     __device__ static __forceinline__ Cell<Real> slope(const Cell<Real> &m, const Cell<Real> &c, const Cell<Real> &p,
-                                                       const SweepConsts<Real> &K)
+                                                       const Consts &K)
     {
         Cell<Real> s;
-        const Real hrh = K.rh * Real(0.5), rha = K.rh * K.alpha;
+        const Real hrh = half_rh(K), rha = alpha_rh(K);
         s.rho = limited_slope_hoisted(m.rho, c.rho, p.rho, hrh, rha);
         s.p = limited_slope_hoisted(m.p, c.p, p.p, hrh, rha);
         s.un = limited_slope_hoisted(m.un, c.un, p.un, hrh, rha);
         s.ut = limited_slope_hoisted(m.ut, c.ut, p.ut, hrh, rha);
         return s;
     }
-    template <typename Real>
+    // The reference's formulas (src/basicFuns.cuh:86-189) with common parts
+    // taken out.  With k_l, k_r as there and s = c / rho, its d_l = 2 s_l k_l
+    // and d_r = 2 s_r k_r, so Dpi_Dt = (c_r s_l k_l - c_l s_r k_r) / (c_l + c_r).
+    // On the side of the contact (c, the face's rho, u, ...; sg = 1 on the
+    // right, -1 on the left) z = 1 / (sg (u_s - u) + c / rho_s) is the star
+    // density over c; with w = u z and h = 1 + sg w
+    //   rho_t = z (z h Dpi_Dt - w (rho / rho_s) S),
+    //   S     = s^2 rho_x - sg c u_x + 3/2 (u - u_s) c_x,
+    // and u rho / c = w in the factors of p_t and u_t: about 125 operations from
+    // the face states to the star region's derivatives, where the formulas term
+    // by term take about 165.
+    template <typename Real, class Consts>
     __device__ static __forceinline__ Interface<Real> grp(const Cell<Real> &L, const Cell<Real> &R,
                                                           const Cell<Real> &sL, const Cell<Real> &sR,
-                                                          const SweepConsts<Real> &K)
+                                                          const Consts &K)
     {
         const Real one = Real(1), half = Real(0.5), zero = Real(0);
         const Real g = K.g, igm1 = K.igm1, kappa = K.kappa;
@@ -440,100 +467,127 @@ struct Hoisted {
         const Real rho_lx = sL.rho, pi_lx = sL.p, u_lx = sL.un, v_lx = sL.ut;
         const Real rho_rx = sR.rho, pi_rx = sR.p, u_rx = sR.un, v_rx = sR.ut;
 
-        // 1/rho_l and 1/rho_r from one division
-        const Real irlr = rrcp(rho_l * rho_r);
-        const Real irl = rho_r * irlr, irr = rho_l * irlr;
-        const Real e_l = pi_l * irl * igm1, e_r = pi_r * irr * igm1;
-        const Real e_lx = (pi_lx - pi_l * rho_lx * irl) * irl * igm1;
-        const Real e_rx = (pi_rx - pi_r * rho_rx * irr) * irr * igm1;
         // 1/(rho a) = 1/sqrt(g p rho) and a = sqrt(g p / rho) = g p / sqrt(g p rho):
         // one reciprocal square root per side
-        const Real il = rrsqrt(g * pi_l * rho_l), ir = rrsqrt(g * pi_r * rho_r);
-        const Real a_l = g * pi_l * il, a_r = g * pi_r * ir;
-        const Real c_lx = half * g * (pi_l * rho_lx + rho_l * pi_lx) * il;
-        const Real c_rx = half * g * (pi_r * rho_rx + rho_r * pi_rx) * ir;
-        const Real du = u_l - u_r;
+        const Real gpl = g * pi_l, gpr = g * pi_r;
+        const Real il = rrsqrt(gpl * rho_l), ir = rrsqrt(gpr * rho_r);
+        const Real a_l = gpl * il, a_r = gpr * ir;
+        const Real hg = half * g;
+        const Real c_lx = fma(pi_l, rho_lx, rho_l * pi_lx) * (hg * il);
+        const Real c_rx = fma(pi_r, rho_rx, rho_r * pi_rx) * (hg * ir);
+        const Real du = u_l - u_r, dp = pi_r - pi_l;
         // the side computed second gets its reciprocal and 1/(c_l + c_r)
         // from one division
-        Real c_l, c_r, icl, icr, isum;
+        Real c_l, c_r, icl, icr, isum, sl, sr;  // s = c/rho: the fan's edge speeds relative to u
         if (pi_r >= pi_l) {
-            c_l = rho_l * (a_l + kappa * rmax(zero, (pi_r - pi_l) * ir + du));
+            sl = fma(kappa, rmax(zero, fma(dp, ir, du)), a_l);
+            c_l = rho_l * sl;
             icl = rrcp(c_l);
-            c_r = rho_r * (a_r + kappa * rmax(zero, (pi_l - pi_r) * icl + du));
+            sr = fma(kappa, rmax(zero, fma(-dp, icl, du)), a_r);
+            c_r = rho_r * sr;
             const Real sc = c_l + c_r, q = rrcp(c_r * sc);
             icr = sc * q;
             isum = c_r * q;
         } else {
-            c_r = rho_r * (a_r + kappa * rmax(zero, (pi_l - pi_r) * il + du));
+            sr = fma(kappa, rmax(zero, fma(-dp, il, du)), a_r);
+            c_r = rho_r * sr;
             icr = rrcp(c_r);
-            c_l = rho_l * (a_l + kappa * rmax(zero, (pi_r - pi_l) * icr + du));
+            sl = fma(kappa, rmax(zero, fma(dp, icr, du)), a_l);
+            c_l = rho_l * sl;
             const Real sc = c_l + c_r, q = rrcp(c_l * sc);
             icl = sc * q;
             isum = c_l * q;
         }
-        const Real sl = c_l * irl, sr = c_r * irr;  // c/rho: the fan's edge speeds relative to u
         Interface<Real> o;
         if (u_l - sl >= zero) {
-            o.rho = rho_l; o.p = pi_l; o.un = u_l; o.ut = v_l; o.e = e_l;
-            o.rho_t = -rho_l * u_lx - u_l * rho_lx;
-            o.un_t = -u_l * u_lx - pi_lx * irl;
-            o.e_t = -u_l * e_lx - pi_l * irl * u_lx;
-            o.ut_t = -u_l * v_lx;
-            o.p_t = -u_l * pi_lx - c_l * sl * u_lx;
+            const Real irl = rrcp(rho_l), iri = irl * igm1, tp = pi_l * irl;
+            o.rho = rho_l; o.p = pi_l; o.un = u_l; o.ut = v_l; o.e = pi_l * iri;
+            o.rho_t = -fma(rho_l, u_lx, u_l * rho_lx);
+            o.un_t = -fma(u_l, u_lx, pi_lx * irl);
+            o.e_t = -fma(u_l, fma(-tp, rho_lx, pi_lx) * iri, tp * u_lx);
+            o.ut_t = -(u_l * v_lx);
+            o.p_t = -fma(u_l, pi_lx, (c_l * sl) * u_lx);
         } else if (u_r + sr <= zero) {
-            o.rho = rho_r; o.p = pi_r; o.un = u_r; o.ut = v_r; o.e = e_r;
-            o.rho_t = -rho_r * u_rx - u_r * rho_rx;
-            o.un_t = -u_r * u_rx - pi_rx * irr;
-            o.e_t = -u_r * e_rx - pi_r * irr * u_rx;
-            o.ut_t = -u_r * v_rx;
-            o.p_t = -u_r * pi_rx - c_r * sr * u_rx;
+            const Real irr = rrcp(rho_r), iri = irr * igm1, tp = pi_r * irr;
+            o.rho = rho_r; o.p = pi_r; o.un = u_r; o.ut = v_r; o.e = pi_r * iri;
+            o.rho_t = -fma(rho_r, u_rx, u_r * rho_rx);
+            o.un_t = -fma(u_r, u_rx, pi_rx * irr);
+            o.e_t = -fma(u_r, fma(-tp, rho_rx, pi_rx) * iri, tp * u_rx);
+            o.ut_t = -(u_r * v_rx);
+            o.p_t = -fma(u_r, pi_rx, (c_r * sr) * u_rx);
         } else {
-            const Real u = (u_l * c_l + u_r * c_r + pi_l - pi_r) * isum;
-            const Real pm = (du * c_l * c_r + c_l * pi_r + c_r * pi_l) * isum;
-            const Real k_l = -pi_lx - c_l * u_lx - half * u_l * c_lx;
-            const Real k_r = -pi_rx + c_r * u_rx + half * u_r * c_rx;
-            const Real d_l = sl * (Real(-2) * (c_l * u_lx + pi_lx) - u_l * c_lx);
-            const Real d_r = sr * (Real(2) * (c_r * u_rx - pi_rx) + u_r * c_rx);
-            const Real Dp = (c_r * d_l - c_l * d_r) * half * isum;
+            const Real u = (fma(u_l, c_l, u_r * c_r) - dp) * isum;
+            const Real pm = fma(du * c_l, c_r, fma(c_l, pi_r, c_r * pi_l)) * isum;
+            // b_l = -s_l k_l, b_r = s_r k_r, nDp = -Dpi_Dt
+            const Real b_l = sl * fma(half * u_l, c_lx, fma(c_l, u_lx, pi_lx));
+            const Real b_r = sr * fma(half * u_r, c_rx, fma(c_r, u_rx, -pi_rx));
+            const Real nDp = fma(c_r, b_l, c_l * b_r) * isum;
             o.p = pm;
             o.un = u;
             if (u <= zero) {
-                const Real irho = (u_r - u + sr) * icr;
-                const Real rho = rrcp(irho);
-                const Real icr2 = icr * icr;
-                const Real e = e_r + (pm - pi_r) * (pm + pi_r) * half * icr2;
-                const Real rho3 = rho * rho * rho, urho = u * rho;
-                o.rho = rho; o.e = e; o.ut = v_r;
-                o.rho_t = -u * rho3 * irr * icr2 * (sr * sr * rho_rx - c_r * u_rx + Real(1.5) * (u - u_r) * c_rx) +
-                          rho3 * icr2 * icr * (u + c_r * irho) * Dp;
-                o.p_t = isum * (c_r * sl * (one + urho * icr) * k_l - c_l * sr * (one - urho * icl) * k_r);
-                o.un_t = isum * (sl * (one + urho * icr) * k_l + sr * (one - urho * c_l * icr2) * k_r);
-                o.e_t = -urho * irr * (e_rx - pi_r * pi_rx * icr2 + Real(2) * (e_r - e) * c_rx * icr) + pm * icr2 * o.p_t;
-                o.ut_t = -urho * irr * v_rx;
+                const Real irr = rrcp(rho_r), z = rrcp((u_r - u) + sr);
+                const Real rho = c_r * z, w = u * z, h = one + w, q = rho * irr;
+                const Real S = fma(sr * sr, rho_rx, fma(-c_r, u_rx, (Real(1.5) * (u - u_r)) * c_rx));
+                const Real P = b_l * h;
+                const Real icr2 = icr * icr, E2 = (pm - pi_r) * (pm + pi_r) * icr2;
+                const Real iri = irr * igm1, tp = pi_r * irr;
+                const Real G = fma(-icr, fma(E2, c_rx, (icr * pi_r) * pi_rx), fma(-tp, rho_rx, pi_rx) * iri);
+                const Real uq = u * q;
+                o.rho = rho;
+                o.e = fma(half, E2, pi_r * iri);
+                o.ut = v_r;
+                o.rho_t = -(z * fma(z * h, nDp, (w * q) * S));
+                o.p_t = -(isum * fma(c_r, P, b_r * fma(-u, rho, c_l)));
+                o.un_t = isum * fma(b_r, fma(-(w * c_l), icr, one), -P);
+                o.e_t = fma(pm * icr2, o.p_t, -(uq * G));
+                o.ut_t = -(uq * v_rx);
             } else {
-                const Real irho = (u - u_l + sl) * icl;
-                const Real rho = rrcp(irho);
-                const Real icl2 = icl * icl;
-                const Real e = e_l + (pm - pi_l) * (pm + pi_l) * half * icl2;
-                const Real rho3 = rho * rho * rho, urho = u * rho;
-                o.rho = rho; o.e = e; o.ut = v_l;
-                o.rho_t = -u * rho3 * irl * icl2 * (sl * sl * rho_lx + c_l * u_lx + Real(1.5) * (u - u_l) * c_lx) -
-                          rho3 * icl2 * icl * (u - c_l * irho) * Dp;
-                o.p_t = isum * (c_r * sl * (one + urho * icr) * k_l - c_l * sr * (one - urho * icl) * k_r);
-                o.un_t = isum * (sl * (one + urho * c_r * icl2) * k_l + sr * (one - urho * icl) * k_r);
-                o.e_t = -urho * irl * (e_lx - pi_l * pi_lx * icl2 + Real(2) * (e_l - e) * c_lx * icl) + pm * icl2 * o.p_t;
-                o.ut_t = -urho * irl * v_lx;
+                const Real irl = rrcp(rho_l), z = rrcp((u - u_l) + sl);
+                const Real rho = c_l * z, w = u * z, h = one - w, q = rho * irl;
+                const Real S = fma(sl * sl, rho_lx, fma(c_l, u_lx, (Real(1.5) * (u - u_l)) * c_lx));
+                const Real P = b_r * h;
+                const Real icl2 = icl * icl, E2 = (pm - pi_l) * (pm + pi_l) * icl2;
+                const Real iri = irl * igm1, tp = pi_l * irl;
+                const Real G = fma(-icl, fma(E2, c_lx, (icl * pi_l) * pi_lx), fma(-tp, rho_lx, pi_lx) * iri);
+                const Real uq = u * q;
+                o.rho = rho;
+                o.e = fma(half, E2, pi_l * iri);
+                o.ut = v_l;
+                o.rho_t = -(z * fma(z * h, nDp, (w * q) * S));
+                o.p_t = -(isum * fma(b_l, fma(u, rho, c_r), c_l * P));
+                o.un_t = isum * fma(-b_l, fma(w * c_r, icl, one), P);
+                o.e_t = fma(pm * icl2, o.p_t, -(uq * G));
+                o.ut_t = -(uq * v_lx);
             }
         }
         return o;
     }
 
-    template <typename Real>
+    // F + k/2 dF/dt through m = rho u and m_t = d(rho u)/dt (the product rule
+    // applied to src/basicFuns.cuh:28-33), gathered around the midpoint mass
+    // flux M = m + k/2 m_t and pressure Q = p + k/2 p_t.
+    template <typename Real, class Consts>
+    __device__ static __forceinline__ Cell<Real> flux_of(const Interface<Real> &w, const Consts &K)
+    {
+        const Real hk = half_k(K), half = Real(0.5);
+        const Real m = w.rho * w.un, m_t = fma(w.rho, w.un_t, w.un * w.rho_t);
+        const Real M = fma(hk, m_t, m), Q = fma(hk, w.p_t, w.p), hm = hk * m;
+        const Real es = fma(half, fma(w.un, w.un, w.ut * w.ut), w.e);
+        const Real et = fma(w.un, w.un_t, fma(w.ut, w.ut_t, w.e_t));
+        Cell<Real> F;
+        F.rho = M;
+        F.p = fma(M, w.un, fma(hm, w.un_t, Q));
+        F.un = fma(es, M, fma(hm, et, fma(w.un, Q, (hk * w.p) * w.un_t)));
+        F.ut = fma(M, w.ut, hm * w.ut_t);
+        return F;
+    }
+
+    template <typename Real, class Consts>
     __device__ static __forceinline__ Cell<Real> interface_flux(const Cell<Real> &UL, const Cell<Real> &UR,
                                                                 const Cell<Real> &sL, const Cell<Real> &sR,
-                                                                const SweepConsts<Real> &K)
+                                                                const Consts &K)
     {
-        const Real hh = K.h * Real(0.5);
+        const Real hh = half_h(K);
         Cell<Real> fL, fR;  // U_L + s_L h/2, U_R - s_R h/2 with h/2 folded in
         fL.rho = fma(sL.rho, hh, UL.rho);
         fL.p = fma(sL.p, hh, UL.p);
@@ -543,40 +597,26 @@ struct Hoisted {
         fR.p = fma(-sR.p, hh, UR.p);
         fR.un = fma(-sR.un, hh, UR.un);
         fR.ut = fma(-sR.ut, hh, UR.ut);
-        const Interface<Real> w = grp(fL, fR, sL, sR, K);
-        // F + k/2 dF/dt through m = rho u and m_t = d(rho u)/dt (the product
-        // rule applied to src/basicFuns.cuh:28-33)
-        const Real hk = K.k * Real(0.5);
-        const Real m = w.rho * w.un, m_t = w.rho * w.un_t + w.un * w.rho_t;
-        const Real es = w.e + Real(0.5) * (w.un * w.un + w.ut * w.ut);
-        Cell<Real> F;
-        F.rho = m + hk * m_t;
-        F.p = m * w.un + w.p + hk * (m_t * w.un + m * w.un_t + w.p_t);
-        F.un = m * es + w.p * w.un +
-               hk * (m_t * es + m * (w.e_t + w.un * w.un_t + w.ut * w.ut_t) + w.p_t * w.un + w.p * w.un_t);
-        F.ut = m * w.ut + hk * (m_t * w.ut + m * w.ut_t);
-        return F;
+        return flux_of(grp(fL, fR, sL, sR, K), K);
     }
 
-    template <typename Real>
+    template <typename Real, class Consts>
     __device__ static __forceinline__ Cell<Real> update(const Cell<Real> &U, const Cell<Real> &FL,
-                                                        const Cell<Real> &FR, const SweepConsts<Real> &K)
+                                                        const Cell<Real> &FR, const Consts &K)
     {
         const Real half = Real(0.5);
-        Real m0 = U.rho;
-        Real m1 = U.rho * U.un;
-        Real m2 = U.p * K.igm1 + half * U.rho * (U.un * U.un + U.ut * U.ut);
-        Real m3 = U.rho * U.ut;
-        m0 -= (FR.rho - FL.rho) * K.lambda;
-        m1 -= (FR.p - FL.p) * K.lambda;
-        m2 -= (FR.un - FL.un) * K.lambda;
-        m3 -= (FR.ut - FL.ut) * K.lambda;
+        const Real r1 = U.rho * U.un, r3 = U.rho * U.ut;
+        const Real r2 = fma(U.p, K.igm1, half * fma(r1, U.un, r3 * U.ut));
+        const Real m0 = fma(FL.rho - FR.rho, K.lambda, U.rho);
+        const Real m1 = fma(FL.p - FR.p, K.lambda, r1);
+        const Real m2 = fma(FL.un - FR.un, K.lambda, r2);
+        const Real m3 = fma(FL.ut - FR.ut, K.lambda, r3);
         const Real ir = rrcp(m0);
         Cell<Real> o;
         o.rho = m0;
         o.un = m1 * ir;
         o.ut = m3 * ir;
-        o.p = (K.g - Real(1)) * (m2 - half * (m1 * m1 + m3 * m3) * ir);
+        o.p = K.gm1 * fma(-(half * fma(m1, m1, m3 * m3)), ir, m2);
         return o;
     }
 };
@@ -606,9 +646,9 @@ __device__ __forceinline__ void two_prod(Real a, Real b, Real &p, Real &e)
 }
 
 struct HoistedCompensated : Hoisted {
-    template <typename Real>
+    template <typename Real, class Consts>
     __device__ static __forceinline__ Cell<Real> update(const Cell<Real> &U, const Cell<Real> &FL,
-                                                        const Cell<Real> &FR, const SweepConsts<Real> &K)
+                                                        const Cell<Real> &FR, const Consts &K)
     {
         const Real half = Real(0.5);
         // conserved vector of the cell: (rho, rho un, E, rho ut) as hi + lo

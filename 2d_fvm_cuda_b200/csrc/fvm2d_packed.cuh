@@ -31,32 +31,26 @@ __device__ __forceinline__ void two_sum2(float2 a, float2 b, float2 &s, float2 &
 
 struct PackedCompensated : HoistedCompensated {
     // Hoisted::interface_flux with the face states as two packed pairs
+    template <class Consts>
     __device__ static __forceinline__ Cell<float> interface_flux(const Cell<float> &UL, const Cell<float> &UR,
                                                                  const Cell<float> &sL, const Cell<float> &sR,
-                                                                 const SweepConsts<float> &K)
+                                                                 const Consts &K)
     {
-        const float2 hh = p2(K.h * 0.5f, K.h * 0.5f), mh = p2(-K.h * 0.5f, -K.h * 0.5f);
+        const float h2 = half_h(K);
+        const float2 hh = p2(h2, h2), mh = p2(-h2, -h2);
         const float2 l01 = fma2(p2(sL.rho, sL.p), hh, p2(UL.rho, UL.p));
         const float2 l23 = fma2(p2(sL.un, sL.ut), hh, p2(UL.un, UL.ut));
         const float2 r01 = fma2(p2(sR.rho, sR.p), mh, p2(UR.rho, UR.p));
         const float2 r23 = fma2(p2(sR.un, sR.ut), mh, p2(UR.un, UR.ut));
         const Cell<float> fL = {l01.x, l01.y, l23.x, l23.y}, fR = {r01.x, r01.y, r23.x, r23.y};
-        const Interface<float> w = grp(fL, fR, sL, sR, K);
-        const float hk = K.k * 0.5f;
-        const float m = w.rho * w.un, m_t = w.rho * w.un_t + w.un * w.rho_t;
-        const float es = w.e + 0.5f * (w.un * w.un + w.ut * w.ut);
-        Cell<float> F;
-        F.rho = m + hk * m_t;
-        F.p = m * w.un + w.p + hk * (m_t * w.un + m * w.un_t + w.p_t);
-        F.un = m * es + w.p * w.un + hk * (m_t * es + m * (w.e_t + w.un * w.un_t + w.ut * w.ut_t) + w.p_t * w.un + w.p * w.un_t);
-        F.ut = m * w.ut + hk * (m_t * w.ut + m * w.ut_t);
-        return F;
+        return flux_of(grp(fL, fR, sL, sR, K), K);
     }
 
     // HoistedCompensated::update with the conserved vector handled as the
     // pairs (rho, rho un), (E, rho ut) and the momenta as (rho un, rho ut)
+    template <class Consts>
     __device__ static __forceinline__ Cell<float> update(const Cell<float> &U, const Cell<float> &FL,
-                                                         const Cell<float> &FR, const SweepConsts<float> &K)
+                                                         const Cell<float> &FR, const Consts &K)
     {
         const float2 uv = p2(U.un, U.ut), rr = p2(U.rho, U.rho);
         // (m1, m3) = rho (un, ut) and their errors; (ka, kb) = (m1 un, m3 ut)
@@ -114,9 +108,10 @@ struct PackedCompensated : HoistedCompensated {
 // is otherwise idle in these sweeps.)
 struct PackedResidual : PackedCompensated {
     static constexpr bool kSplitStorage = true;
+    template <class Consts>
     __device__ static __forceinline__ Cell<double> update_split(const Cell<float> &U, const Cell<float> &L,
                                                                 const Cell<float> &FL, const Cell<float> &FR,
-                                                                const SweepConsts<float> &K)
+                                                                const Consts &K)
     {
         const double rho = double(U.rho) + double(L.rho), p = double(U.p) + double(L.p);
         const double un = double(U.un) + double(L.un), ut = double(U.ut) + double(L.ut);
