@@ -18,6 +18,7 @@
 
 #include "fvm2d_batch_control.h"
 #include "fvm2d_kernels.cuh"
+#include "fvm2d_tile.cuh"
 
 namespace fvm2d {
 namespace FVM2D_VARIANT {
@@ -32,6 +33,9 @@ struct BatchArgs {
     const int *rb0;            // [np + 1] first ghost block of each problem
     const int *ib0;            // [np + 1] first init block of each problem
     int np;
+    // steps in tiles: [np + 1] first tile of each problem (null: steps sweep by
+    // sweep); a problem's state is in its region b while its parity is odd
+    const long long *t0 = nullptr;
 };
 
 // Largest p with first[p] <= item (first[] ascending, first[0] = 0).
@@ -199,6 +203,67 @@ __global__ void __launch_bounds__(NT) batch_ghost_kernel(BatchArgs<Real> b)
     if (last_of_blocks(&ctl->ticket, unsigned(b.rb0[p + 1] - b.rb0[p]))) finish_step(ctl, P.plan);
 }
 
+#ifdef __CUDACC__
+// Problem p's arguments of a step in tiles, its state in src.
+template <typename Real>
+__device__ __forceinline__ TileArgs<Real> batch_tile_args(const BatchArgs<Real> &b, int p)
+{
+    const BatchProblem &P = b.prob[p];
+    TileArgs<Real> a;
+    a.ctl = b.ctl + p;
+    const int odd = a.ctl->parity;
+    a.src.base = b.base + (odd ? P.b : P.u);
+    a.dst.base = b.base + (odd ? P.u : P.b);
+    a.src.plane = a.dst.plane = P.plane;
+    a.src.pitch = a.dst.pitch = P.pitch;
+    a.nx = P.nx;
+    a.ny = P.ny;
+    a.hx = P.hx;
+    a.hy = P.hy;
+    a.rhx = P.rhx;
+    a.rhy = P.rhy;
+    a.alpha = P.alpha;
+    a.gamma = P.gamma;
+    a.strategy = P.strategy;
+    a.plan = P.plan;
+    return a;
+}
+
+// A step in tiles (fvm2d_tile.cuh): one block per tile of any problem.
+template <typename Real, class Phys, class T, int MINB>
+__global__ void __launch_bounds__(T::NT, MINB) batch_tile_kernel(BatchArgs<Real> b)
+{
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    pdl_launch();
+    const int p = find_problem(b.t0, b.np, (long long)blockIdx.x);
+    StepControl *ctl = b.ctl + p;
+    pdl_wait();
+    __shared__ StepControl c;
+    if (threadIdx.x == 0) c = *ctl;
+    __syncthreads();
+    if (!c.active) return;
+    const TileArgs<Real> a = batch_tile_args(b, p);
+    const int ntx = (a.nx - 4 + T::TX - 1) / T::TX, k = int(blockIdx.x - b.t0[p]);
+    double vmax = 0.0;
+    int bad = 0;
+    if (k == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
+    tile_step<Real, Phys, T>(a, c.dt, k % ntx, k / ntx, tile_smem, vmax, bad, c.ring_due, c.t);
+    end_tile<T::NT>(vmax, bad, ctl, c, a.plan, unsigned(b.t0[p + 1] - b.t0[p]));
+}
+
+// Stores the ghost rings after steps in tiles.
+template <typename Real, int NT>
+__global__ void __launch_bounds__(NT) batch_fill_ring_kernel(BatchArgs<Real> b)
+{
+    pdl_launch();
+    const int p = find_problem(b.rb0, b.np, int(blockIdx.x));
+    pdl_wait();
+    if (!b.ctl[p].ring_due) return;
+    const int k = (int(blockIdx.x) - b.rb0[p]) * NT + threadIdx.x;
+    if (k < b.prob[p].ring) ghost_cell(ring_args(batch_tile_args(b, p)), k, b.ctl[p].t);
+}
+#endif
+
 // Wave speed of every cell of each problem's initial state, then its first plan.
 template <typename Real, int NT>
 __global__ void __launch_bounds__(NT) batch_init_kernel(BatchArgs<Real> b)
@@ -207,7 +272,7 @@ __global__ void __launch_bounds__(NT) batch_init_kernel(BatchArgs<Real> b)
     const BatchProblem &P = b.prob[p];
     StepControl *ctl = b.ctl + p;
     Field<Real> U;
-    U.base = b.base + P.u;
+    U.base = b.base + (b.t0 && ctl->parity ? P.b : P.u);
     U.plane = P.plane;
     U.pitch = P.pitch;
     const long long n = (long long)P.nx * P.ny;

@@ -4,10 +4,12 @@
 // All problems of a batch share one allocation: problem p owns three
 // consecutive state-sized regions (U, A, B), each 4 planes of pitch_p x ny_p
 // doubles; FP32 planes start at the same byte addresses and fill the first
-// half of each region.  A step is five launches covering every problem (x-sweep, y-sweep,
-// y-sweep, final x-sweep, ghost ring); each problem carries its own dt, time
-// and end time in its control record, and its items are skipped once its loop
-// has ended.  The step is captured in CUDA graphs (16 steps and 1 step) that
+// half of each region.  A step is one launch covering every problem's tiles
+// (fvm2d_tile.cuh), going from a problem's U to its B and back by turns; each
+// problem carries its own dt, time and end time in its control record, and its
+// tiles are skipped once its loop has ended.  (Sweep by sweep, five launches:
+// x-sweep, y-sweep, y-sweep, final x-sweep, ghost ring, if the autotuner finds
+// that faster.)  The step is captured in CUDA graphs (16 steps and 1 step) that
 // are replayed until no problem has a step in flight; each replay reads the
 // control records back (64 bytes per problem).  fvm2d_batch_autotune times
 // candidate y-segment lengths and sweep grid sizes on the batch itself and
@@ -57,17 +59,23 @@ struct BatchVariant {
     cudaError_t (*init)(const BatchLaunch &, cudaStream_t);
     cudaError_t (*plan)(const BatchLaunch &, cudaStream_t);
     cudaError_t (*step)(const BatchLaunch &, cudaStream_t);
+    cudaError_t (*fill_ring)(const BatchLaunch &, cudaStream_t);
+    int (*tile_shape)(int, const int *, const int *);
+    long long (*tiles)(int, int, int);
 };
 
 const BatchVariant kBatchVariants[] = {
     {fvm2d::fp64::batch_prepare, fvm2d::fp64::batch_enqueue_init, fvm2d::fp64::batch_enqueue_plan,
-     fvm2d::fp64::batch_enqueue_step},
+     fvm2d::fp64::batch_enqueue_step, fvm2d::fp64::batch_enqueue_fill_ring, fvm2d::fp64::batch_tile_shape, fvm2d::fp64::batch_tiles},
     {fvm2d::fp64_strict::batch_prepare, fvm2d::fp64_strict::batch_enqueue_init, fvm2d::fp64_strict::batch_enqueue_plan,
-     fvm2d::fp64_strict::batch_enqueue_step},
+     fvm2d::fp64_strict::batch_enqueue_step,
+     fvm2d::fp64_strict::batch_enqueue_fill_ring, fvm2d::fp64_strict::batch_tile_shape, fvm2d::fp64_strict::batch_tiles},
     {fvm2d::fp64_reforder::batch_prepare, fvm2d::fp64_reforder::batch_enqueue_init,
-     fvm2d::fp64_reforder::batch_enqueue_plan, fvm2d::fp64_reforder::batch_enqueue_step},
+     fvm2d::fp64_reforder::batch_enqueue_plan, fvm2d::fp64_reforder::batch_enqueue_step,
+     fvm2d::fp64_reforder::batch_enqueue_fill_ring,
+     fvm2d::fp64_reforder::batch_tile_shape, fvm2d::fp64_reforder::batch_tiles},
     {fvm2d::fp32::batch_prepare, fvm2d::fp32::batch_enqueue_init, fvm2d::fp32::batch_enqueue_plan,
-     fvm2d::fp32::batch_enqueue_step},
+     fvm2d::fp32::batch_enqueue_step, fvm2d::fp32::batch_enqueue_fill_ring, fvm2d::fp32::batch_tile_shape, fvm2d::fp32::batch_tiles},
 };
 constexpr int kNumBatchVariants = sizeof(kBatchVariants) / sizeof(kBatchVariants[0]);
 
@@ -85,11 +93,12 @@ struct fvm2d_batch {
     std::vector<double> width, height, t_end, cfl, alpha, gamma;
     std::vector<long long> off;  // element offset of problem p's U region
     std::vector<char> have_state;
+    std::vector<int> flip;       // problem p's state is in its region U (0) or B (1): its record's parity after a run
     long long total_elems = 0;   // doubles in the allocation
     double *base = nullptr;
     BatchProblem *prob_d = nullptr;
     StepControl *ctl_d = nullptr, *ctl_h = nullptr;
-    long long *x0_d = nullptr, *y0_d = nullptr;
+    long long *x0_d = nullptr, *y0_d = nullptr, *t0_d = nullptr;
     int *rb0_d = nullptr, *ib0_d = nullptr;
     BatchLaunch L{};
     bool dirty = true;  // descriptors must be rebuilt and uploaded
@@ -98,6 +107,8 @@ struct fvm2d_batch {
     // step graphs re-captured) once they hold a sizeable share of the items,
     // so the static split of items over warps keeps every warp on live work
     std::vector<char> listed;
+    bool use_tiles = true;  // steps in tiles; fvm2d_batch_autotune may find the sweeps faster
+    int tile_shape = 0;
     int T = 32;         // y-sweep interfaces per segment
     int xchunks = 8;    // x-sweep chunks of 32 cells per item (set with the descriptors)
     int grid_x = 0, grid_y = 0;
@@ -118,6 +129,9 @@ struct fvm2d_batch {
     }
 
     long long plane(int p) const { return (long long)pitch[p] * ny[p]; }
+    // Problem p's state, and the two regions beside it (adjacent) as staging.
+    double *state(int p) { return base + off[p] + (flip[p] ? 8 * plane(p) : 0); }
+    double *staging(int p) { return base + off[p] + (flip[p] ? 0 : 4 * plane(p)); }
 
     // Host descriptors and prefix counts -> device.
     int upload_descriptors()
@@ -135,6 +149,7 @@ struct fvm2d_batch {
             xchunks /= 2;
         }
         if ((int)listed.size() != np) listed.assign(np, 1);
+        tile_shape = kBatchVariants[precision].tile_shape(np, nx.data(), ny.data());
         // offsets in elements of the storage type: FP32 planes start at the
         // same byte addresses as FP64 planes would (the layout is in doubles)
         const long long scale = (precision == FVM2D_FP32) ? 2 : 1;
@@ -193,20 +208,26 @@ struct fvm2d_batch {
     // Sweep items of one row or column group of problem p.
     long long x_items(int p) const { return (long long)fvm2d::x_items_per_row(nx[p], xchunks) * ny[p]; }
     long long y_items(int p) const { return (long long)((nx[p] + 31) / 32) * y_segments(ny[p], T); }
+    long long tiles(int p) const { return kBatchVariants[precision].tiles(tile_shape, nx[p], ny[p]); }
 
     // Item prefix counts of the listed problems (others get no items) -> device.
     int upload_items()
     {
-        std::vector<long long> x0(np + 1, 0), y0(np + 1, 0);
+        std::vector<long long> x0(np + 1, 0), y0(np + 1, 0), t0(np + 1, 0);
         for (int p = 0; p < np; ++p) {
             x0[p + 1] = x0[p] + (listed[p] ? x_items(p) : 0);
             y0[p + 1] = y0[p] + (listed[p] ? y_items(p) : 0);
+            t0[p + 1] = t0[p] + (listed[p] ? tiles(p) : 0);
         }
         CK(cudaMemcpyAsync(x0_d, x0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(y0_d, y0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(t0_d, t0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
         CK(cudaStreamSynchronize(stream));
         L.x_total = x0[np];
         L.y_total = y0[np];
+        L.t0 = use_tiles ? t0_d : nullptr;
+        L.tile_total = t0[np];
+        L.tile_shape = tile_shape;
         return FVM2D_OK;
     }
 
@@ -257,6 +278,13 @@ struct fvm2d_batch {
     int run(int limit)
     {
         if (int rc = upload_descriptors()) return rc;
+        if (!use_tiles)  // the sweeps step in place, in the first region
+            for (int p = 0; p < np; ++p)
+                if (flip[p]) {
+                    CK(cudaMemcpyAsync(base + off[p], state(p), 4 * plane(p) * sizeof(double), cudaMemcpyDeviceToDevice,
+                                       stream));
+                    flip[p] = 0;
+                }
         if (std::count(listed.begin(), listed.end(), 0)) {  // every problem's items back in the lists
             listed.assign(np, 1);
             if (int rc = upload_items()) return rc;
@@ -267,6 +295,7 @@ struct fvm2d_batch {
         for (int p = 0; p < np; ++p) {
             std::memset(&ctl_h[p], 0, sizeof(StepControl));
             ctl_h[p].step_limit = limit;
+            ctl_h[p].parity = flip[p];
         }
         CK(cudaMemcpyAsync(ctl_d, ctl_h, sizeof(StepControl) * np, cudaMemcpyHostToDevice, stream));
         auto t0 = std::chrono::high_resolution_clock::now();
@@ -278,13 +307,18 @@ struct fvm2d_batch {
             const int which = budget >= kGraphSteps[0] ? 0 : 1;
             CK(cudaGraphLaunch(graph[which], stream));
             budget -= kGraphSteps[which];
-            launches += (long long)kGraphSteps[which] * fvm2d::kStepKernels;
+            launches += (long long)kGraphSteps[which] * (use_tiles ? 1 : fvm2d::kStepKernels);
             CK(cudaMemcpyAsync(ctl_h, ctl_d, sizeof(StepControl) * np, cudaMemcpyDeviceToHost, stream));
             CK(cudaStreamSynchronize(stream));
             bool any = false;
             for (int p = 0; p < np && !any; ++p) any = ctl_h[p].active != 0;
             if (!any) break;
             if (int rc = compact_items()) return rc;
+        }
+        if (use_tiles) {
+            CK(kBatchVariants[precision].fill_ring(L, stream));
+            ++launches;
+            for (int p = 0; p < np; ++p) flip[p] = ctl_h[p].parity;
         }
         CK(cudaEventRecord(ev1, stream));
         CK(cudaEventSynchronize(ev1));
@@ -304,7 +338,7 @@ struct fvm2d_batch {
         for (int p = 0; p < np; ++p) {
             if (!have_state[p]) continue;
             const long long n = 4 * plane(p);
-            double *U = base + off[p], *S = base + off[p] + 4 * plane(p);
+            double *U = state(p), *S = staging(p);
             if (to == FVM2D_FP32)
                 fvm2d::convert_planes<<<148 * 4, 256, 0, stream>>>(fvm2d::Planes<double>{U},
                                                                     fvm2d::Planes<float>{reinterpret_cast<float *>(S)}, n);
@@ -372,6 +406,7 @@ int fvm2d_batch_create(fvm2d_batch **out, int nproblems, const int *nx, const in
             b->alpha.assign(nproblems, 1.9);
             b->gamma.assign(nproblems, 1.4);
             b->have_state.assign(nproblems, 0);
+            b->flip.assign(nproblems, 0);
         } catch (...) {
             rc = fail(FVM2D_ERR_INVALID, "out of host memory");
             break;
@@ -397,6 +432,7 @@ int fvm2d_batch_create(fvm2d_batch **out, int nproblems, const int *nx, const in
         if ((e = cudaMallocHost(&b->ctl_h, sizeof(StepControl) * nproblems))) { rc = cuda_fail(e, "cudaMallocHost"); break; }
         if ((e = cudaMalloc(&b->x0_d, sizeof(long long) * (nproblems + 1)))) { rc = cuda_fail(e, "cudaMalloc"); break; }
         if ((e = cudaMalloc(&b->y0_d, sizeof(long long) * (nproblems + 1)))) { rc = cuda_fail(e, "cudaMalloc"); break; }
+        if ((e = cudaMalloc(&b->t0_d, sizeof(long long) * (nproblems + 1)))) { rc = cuda_fail(e, "cudaMalloc"); break; }
         if ((e = cudaMalloc(&b->rb0_d, sizeof(int) * (nproblems + 1)))) { rc = cuda_fail(e, "cudaMalloc"); break; }
         if ((e = cudaMalloc(&b->ib0_d, sizeof(int) * (nproblems + 1)))) { rc = cuda_fail(e, "cudaMalloc"); break; }
         if ((e = cudaEventCreate(&b->ev0)) || (e = cudaEventCreate(&b->ev1))) { rc = cuda_fail(e, "cudaEventCreate"); break; }
@@ -425,6 +461,7 @@ int fvm2d_batch_destroy(fvm2d_batch *b)
     if (b->ctl_h) cudaFreeHost(b->ctl_h);
     cudaFree(b->x0_d);
     cudaFree(b->y0_d);
+    cudaFree(b->t0_d);
     cudaFree(b->rb0_d);
     cudaFree(b->ib0_d);
     if (b->ev0) cudaEventDestroy(b->ev0);
@@ -470,7 +507,7 @@ int fvm2d_batch_set_state(fvm2d_batch *b, int p, const double *cells, int stride
     if (int rc = check_problem(b, p)) return rc;
     if (!cells) return fail(FVM2D_ERR_INVALID, "null state pointer");
     if (stride != 4 && stride != 5) return fail(FVM2D_ERR_INVALID, "stride must be 4 or 5 doubles per cell");
-    double *U = b->base + b->off[p], *S = U + 4 * b->plane(p);  // staging: the problem's A and B regions
+    double *U = b->state(p), *S = b->staging(p);
     const size_t bytes = sizeof(double) * (size_t)b->nx[p] * b->ny[p] * stride;
     const cudaMemcpyKind kind = fvm2d::is_device_pointer(cells) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     CK(cudaMemcpyAsync(S, cells, bytes, kind, b->stream));
@@ -492,7 +529,7 @@ int fvm2d_batch_get_state(fvm2d_batch *b, int p, double *cells, int stride)
     if (!cells) return fail(FVM2D_ERR_INVALID, "null state pointer");
     if (stride != 4 && stride != 5) return fail(FVM2D_ERR_INVALID, "stride must be 4 or 5 doubles per cell");
     if (!b->have_state[p]) return fail(FVM2D_ERR_STATE, "no state has been set for this problem");
-    double *U = b->base + b->off[p], *S = U + 4 * b->plane(p);
+    double *U = b->state(p), *S = b->staging(p);
     if (b->precision == FVM2D_FP32)
         fvm2d::soa_to_aos<<<148 * 4, 256, 0, b->stream>>>(fvm2d::Planes<float>{reinterpret_cast<float *>(U)}, b->nx[p],
                                                            b->ny[p], b->pitch[p], b->plane(p), stride, S);
@@ -550,7 +587,7 @@ int fvm2d_batch_autotune(fvm2d_batch *b, int trial_steps, int *segment_interface
         size_t o = 0;
         for (int p = 0; p < b->np; ++p) {
             const size_t n = 4 * b->plane(p) * per_elem;
-            char *U = reinterpret_cast<char *>(b->base + b->off[p]);
+            char *U = reinterpret_cast<char *>(b->state(p));
             char *K = reinterpret_cast<char *>(saved) + o;
             cudaError_t e = cudaMemcpyAsync(save ? K : U, save ? U : K, n, cudaMemcpyDeviceToDevice, b->stream);
             if (e) return e;
@@ -564,6 +601,18 @@ int fvm2d_batch_autotune(fvm2d_batch *b, int trial_steps, int *segment_interface
     int rc = FVM2D_OK;
     const int Ts[] = {16, 32, 64};
     const int mults[] = {1, 2, 4};
+    bool best_tiles = false;
+    double sweeps = 1e300;
+    if (!e) {  // a step in tiles
+        b->use_tiles = true;
+        b->dirty = true;
+        if (!(rc = b->run(trial_steps))) {
+            best = b->last_device_ms;
+            best_tiles = true;
+            e = copy_states(false);
+        }
+        b->use_tiles = false;
+    }
     for (int ti = 0; ti < 3 && !e && !rc; ++ti)
         for (int mi = 0; mi < 3 && !e && !rc; ++mi) {
             b->T = Ts[ti];
@@ -572,10 +621,11 @@ int fvm2d_batch_autotune(fvm2d_batch *b, int trial_steps, int *segment_interface
             b->dirty = true;
             if ((rc = b->run(trial_steps))) break;
             const double ms = b->last_device_ms;
-            if (ms < best) best = ms, best_T = Ts[ti], best_g = mults[mi];
+            if (ms < sweeps) sweeps = ms, best_T = Ts[ti], best_g = mults[mi];
             e = copy_states(false);
         }
     cudaFree(saved);
+    b->use_tiles = best_tiles && best <= sweeps;
     if (rc) return rc;
     if (e) return cuda_fail(e, "state copy during tuning");
     b->T = best_T;

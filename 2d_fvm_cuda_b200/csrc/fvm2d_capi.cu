@@ -1,15 +1,19 @@
 // fvm2d_capi.cu -- host runtime behind include/fvm2d.h.
 //
 // A handle owns, on one device:
-//   U        the state: 4 planes (rho, p, u, v), rows padded to `pitch`
-//            elements (a multiple of 32) so every row starts 256-byte aligned;
-//   scratch  two more state-sized buffers (A, B) that the sweeps write, also
-//            used as the staging area for uploads and downloads;
+//   base     three state-sized buffers, each 4 planes (rho, p, u, v) with rows
+//            padded to `pitch` elements (a multiple of 32) so every row starts
+//            256-byte aligned.  U, the state, is the first or the last of
+//            them: a step in tiles reads one and writes the other, and the
+//            control record's parity says which holds the state; `flip` is
+//            the host's copy.  The two that are not U, adjacent either way,
+//            are `scratch`: the sweeps' A and B and the staging area for
+//            uploads and downloads;
 //   ctl      the device-resident StepControl of the time loop;
-//   CUDA graphs of 16 steps and of 1 step (5 kernels each) replayed until
-//   the control record says the loop has ended, so the only host round trip
-//   is one 64-byte read per graph replay (the reference reads the max wave
-//   speed back and synchronizes 17 times per step, src/wrappers.cuh:196-284);
+//   CUDA graphs of 16, 4 and 1 steps replayed until the control record says
+//   the loop has ended; the only host round trip is one 64-byte read per
+//   group of replays (the reference reads the max wave speed back and
+//   synchronizes 17 times per step, src/wrappers.cuh:196-284);
 //   and, allocated on first use, the differentiation workspaces (dual-number
 //   states of fvm2d_jvp; checkpoints, one segment's tape (or, for a
 //   full-tape forward, every step's) and the adjoint states of
@@ -80,13 +84,15 @@ struct Variant {
     cudaError_t (*prepare)();
     cudaError_t (*init)(const LaunchConfig &, cudaStream_t);
     cudaError_t (*plan)(const LaunchConfig &, cudaStream_t);
-    cudaError_t (*step)(const LaunchConfig &, cudaStream_t, cudaEvent_t *);
+    cudaError_t (*step)(const LaunchConfig &, cudaStream_t, cudaEvent_t *);       // in place, five kernels
+    cudaError_t (*tile_step)(const LaunchConfig &, cudaStream_t);                 // pair[parity] to the other
+    cudaError_t (*fill_ring)(const LaunchConfig &, cudaStream_t);                 // after steps in tiles
     cudaError_t (*plan_from)(const LaunchConfig &, cudaStream_t, const double *);
 };
 
 #define FVM2D_VARIANT_ENTRY(ns)                                                                        \
     {fvm2d::ns::prepare, fvm2d::ns::enqueue_init, fvm2d::ns::enqueue_plan, fvm2d::ns::enqueue_step,     \
-     fvm2d::ns::enqueue_plan_from}
+     fvm2d::ns::enqueue_tile_step, fvm2d::ns::enqueue_fill_ring, fvm2d::ns::enqueue_plan_from}
 const Variant kVariants[] = {FVM2D_VARIANT_ENTRY(fp64), FVM2D_VARIANT_ENTRY(fp64_strict),
                              FVM2D_VARIANT_ENTRY(fp64_reforder), FVM2D_VARIANT_ENTRY(fp32),
                              FVM2D_VARIANT_ENTRY(fp32r)};
@@ -153,14 +159,22 @@ struct fvm2d_solver {
     int strategy = FVM2D_OUTFLOW;
     int precision = FVM2D_FP64;
     cudaStream_t stream = nullptr;
-    double *U = nullptr;
-    double *scratch = nullptr;  // A then B
+    double *base = nullptr;     // three states
+    int flip = 0;               // U is the first (0) or the last (1) of them
+    double *U = nullptr;        // the state
+    double *scratch = nullptr;  // the other two: A then B
     StepControl *ctl = nullptr;
     StepControl *ctl_h = nullptr;  // pinned mirror
     // replayed graphs: kGraphSteps[g] steps each; built on first use for the
     // current precision and parameters, dropped by every setter
-    static constexpr int kGraphSteps[2] = {16, 1};
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    static constexpr int kGraphs = 3;
+    static constexpr int kGraphSteps[kGraphs] = {16, 4, 1};
+    // steps enqueued between two reads of the control record, at most: a run
+    // that ends early leaves up to that many empty steps
+    static constexpr int kStepsPerRead = 128;
+    cudaGraphExec_t graph[kGraphs] = {};
+    cudaGraphExec_t slab_graph = nullptr;  // one step in place, for fvm2d_slab_step
+    int slab_flip = 0;                     // the state's buffer it was captured with
     int graph_variant = -1;
     bool have_state = false;
     bool need_init = true;
@@ -202,6 +216,29 @@ struct fvm2d_solver {
     long long total_steps = 0;
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
 
+    // The state is the first (0) or the last (1) of the three buffers.
+    void set_flip(int f)
+    {
+        flip = f;
+        U = base + (f ? 8 * plane : 0);
+        scratch = base + (f ? 0 : 4 * plane);
+    }
+
+    // Whole problems step in tiles; a row slab steps in place, sweep by sweep
+    // (its halo rows pass through the sweeps, and its caller enqueues steps
+    // without knowing whether the loop has ended).
+    bool tiles() const { return ny_global == 0; }
+    cudaError_t enqueue_step(const LaunchConfig &c, cudaStream_t s) const;
+    // Stores the ghost ring that steps in tiles leave unfilled: after every
+    // group of steps whose state something else will read.
+    cudaError_t fill_ring(const LaunchConfig &c, cudaStream_t s) const;
+    int step_kernels() const { return tiles() ? 1 : fvm2d::kStepKernels; }
+    // m steps were enqueued, all of which run
+    void stepped(int m)
+    {
+        if (tiles() && (m & 1)) set_flip(flip ^ 1);
+    }
+
     LaunchConfig config() const
     {
         LaunchConfig c;
@@ -212,6 +249,8 @@ struct fvm2d_solver {
         c.U = U;
         c.A = scratch;
         c.B = scratch + 4 * plane;
+        c.pair[0] = base;
+        c.pair[1] = base + 8 * plane;
         c.ctl = ctl;
         c.hx = width / double(nx);
         c.hy = height / double(ny_global > 0 ? ny_global : ny);  // a slab keeps the problem's row spacing
@@ -237,6 +276,8 @@ struct fvm2d_solver {
             if (g) cudaGraphExecDestroy(g);
             g = nullptr;
         }
+        if (slab_graph) cudaGraphExecDestroy(slab_graph);
+        slab_graph = nullptr;
         graph_variant = -1;
         drop_vjp_graphs();
         last_taped = false;  // taped with the former parameters
@@ -280,54 +321,70 @@ struct fvm2d_solver {
 
     int build_graphs()
     {
-        if (graph_variant == precision && graph[0] && graph[1]) return FVM2D_OK;
+        if (graph_variant == precision && graph[0] && graph[1] && graph[2]) return FVM2D_OK;
         drop_graph();
         const LaunchConfig c = config();
-        for (int which = 0; which < 2; ++which) {
-            cudaGraph_t g = nullptr;
-            CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = cudaSuccess;
-            for (int k = 0; k < kGraphSteps[which] && e == cudaSuccess; ++k)
-                e = kVariants[precision].step(c, stream, nullptr);
-            cudaError_t e2 = cudaStreamEndCapture(stream, &g);
-            if (e != cudaSuccess) {
-                if (g) cudaGraphDestroy(g);
-                return cuda_fail(e, "capture of the step kernels");
-            }
-            if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamEndCapture");
-            e = cudaGraphInstantiate(&graph[which], g, 0);
-            cudaGraphDestroy(g);
-            if (e != cudaSuccess) {
-                graph[which] = nullptr;
-                return cuda_fail(e, "cudaGraphInstantiate");
-            }
-        }
+        for (int which = 0; which < kGraphs; ++which)
+            if (int rc = capture(&graph[which], [&] {
+                    for (int k = 0; k < kGraphSteps[which]; ++k) CK(enqueue_step(c, stream));
+                    return FVM2D_OK;
+                }))
+                return rc;
         graph_variant = precision;
+        return FVM2D_OK;
+    }
+
+    int build_slab_graph()
+    {
+        if (slab_graph && slab_flip == flip) return FVM2D_OK;
+        if (slab_graph) cudaGraphExecDestroy(slab_graph);
+        slab_graph = nullptr;
+        slab_flip = flip;
+        const LaunchConfig c = config();
+        return capture(&slab_graph, [&] {
+            CK(kVariants[precision].step(c, stream, nullptr));
+            return FVM2D_OK;
+        });
+    }
+
+    // Enqueues n steps as graph replays.
+    int replay(long long n)
+    {
+        for (int which = 0; which < kGraphs; ++which)
+            for (; n >= kGraphSteps[which]; n -= kGraphSteps[which]) CK(cudaGraphLaunch(graph[which], stream));
         return FVM2D_OK;
     }
 
     // Replays the step graphs until the control record says no step is in
     // flight.  The record on the device must already be planned; `first`
-    // kernels (init or plan) were enqueued just before.
-    // `budget` bounds the steps this loop may start; the long graph is
-    // replayed while at least its length remains, then the one-step graph.
+    // kernels (init or plan) were enqueued just before.  `budget` bounds the
+    // steps this loop may start.  The record is read after as many steps as
+    // the run is known to have left: the budget, or the remaining time over
+    // the last step size, and at most kStepsPerRead.
     int loop(int first, long long budget)
     {
         int rc = build_graphs();
         if (rc) return rc;
         auto t0 = std::chrono::high_resolution_clock::now();
         long long launches = first;
+        long long ahead = budget < LLONG_MAX ? kStepsPerRead : kGraphSteps[0];
         for (;;) {
-            const int which = budget >= kGraphSteps[0] ? 0 : 1;
-            CK(cudaGraphLaunch(graph[which], stream));
-            budget -= kGraphSteps[which];
-            launches += (long long)kGraphSteps[which] * fvm2d::kStepKernels;
+            const long long n = std::max(1ll, std::min(ahead, budget));
+            if ((rc = replay(n))) return rc;
+            CK(fill_ring(config(), stream));
+            budget -= n;
+            launches += n * step_kernels() + tiles();
+            CK(cudaEventRecord(ev_end, stream));
             CK(cudaMemcpyAsync(ctl_h, ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, stream));
             CK(cudaStreamSynchronize(stream));
             if (!ctl_h->active) break;
+            ahead = kStepsPerRead;
+            if (fixed_dt == 0.0) {
+                const double left = (t_end - ctl_h->t) / ctl_h->dt;  // NaN: a whole group
+                if (left < kStepsPerRead) ahead = (long long)left + 1;
+            }
         }
-        CK(cudaEventRecord(ev_end, stream));
-        CK(cudaEventSynchronize(ev_end));
+        if (tiles()) set_flip(ctl_h->parity);
         auto t1 = std::chrono::high_resolution_clock::now();
         last_ms = std::chrono::duration_cast<std::chrono::microseconds>(t1 - t0).count() / 1000.0;
         float dms = 0.f;
@@ -337,12 +394,26 @@ struct fvm2d_solver {
         return FVM2D_OK;
     }
 
-    int upload_control()
+    int upload_control() { return upload_control(flip); }
+    int upload_control(int parity)
     {
+        ctl_h->parity = parity;
+        ctl_h->ring_due = 0;
         CK(cudaMemcpyAsync(ctl, ctl_h, sizeof(StepControl), cudaMemcpyHostToDevice, stream));
         return FVM2D_OK;
     }
 };
+
+cudaError_t fvm2d_solver::enqueue_step(const LaunchConfig &c, cudaStream_t s) const
+{
+    const Variant &v = kVariants[precision];
+    return tiles() ? v.tile_step(c, s) : v.step(c, s, nullptr);
+}
+
+cudaError_t fvm2d_solver::fill_ring(const LaunchConfig &c, cudaStream_t s) const
+{
+    return tiles() ? kVariants[precision].fill_ring(c, s) : cudaSuccess;
+}
 
 namespace {
 
@@ -405,14 +476,13 @@ int fvm2d_create(fvm2d_solver **out, int nx, int ny)
             if ((e = kVariants[v].prepare()) != cudaSuccess) rc = cuda_fail(e, "kernel attributes");
         if (rc) break;
         if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking))) { rc = cuda_fail(e, "cudaStreamCreate"); break; }
-        if ((e = cudaMalloc(&s->U, state_bytes))) { rc = cuda_fail(e, "cudaMalloc(state)"); break; }
-        if ((e = cudaMalloc(&s->scratch, 2 * state_bytes))) { rc = cuda_fail(e, "cudaMalloc(scratch)"); break; }
+        if ((e = cudaMalloc(&s->base, 3 * state_bytes))) { rc = cuda_fail(e, "cudaMalloc(state)"); break; }
+        s->set_flip(0);
         if ((e = cudaMalloc(&s->ctl, sizeof(StepControl)))) { rc = cuda_fail(e, "cudaMalloc(control)"); break; }
         if ((e = cudaMallocHost(&s->ctl_h, sizeof(StepControl)))) { rc = cuda_fail(e, "cudaMallocHost"); break; }
         if ((e = cudaEventCreate(&s->ev_begin)) || (e = cudaEventCreate(&s->ev_end))) { rc = cuda_fail(e, "cudaEventCreate"); break; }
         std::memset(s->ctl_h, 0, sizeof(StepControl));
-        if ((e = cudaMemsetAsync(s->U, 0, state_bytes, s->stream))) { rc = cuda_fail(e, "cudaMemset"); break; }
-        if ((e = cudaMemsetAsync(s->scratch, 0, 2 * state_bytes, s->stream))) { rc = cuda_fail(e, "cudaMemset"); break; }
+        if ((e = cudaMemsetAsync(s->base, 0, 3 * state_bytes, s->stream))) { rc = cuda_fail(e, "cudaMemset"); break; }
         if ((e = cudaMemsetAsync(s->ctl, 0, sizeof(StepControl), s->stream))) { rc = cuda_fail(e, "cudaMemset"); break; }
         if ((e = cudaStreamSynchronize(s->stream))) { rc = cuda_fail(e, "cudaStreamSynchronize"); break; }
     } while (0);
@@ -430,8 +500,7 @@ int fvm2d_destroy(fvm2d_solver *s)
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     s->drop_graph();
-    if (s->U) cudaFree(s->U);
-    if (s->scratch) cudaFree(s->scratch);
+    if (s->base) cudaFree(s->base);
     if (s->ctl) cudaFree(s->ctl);
     if (s->ctl_h) cudaFreeHost(s->ctl_h);
     if (s->dual) cudaFree(s->dual);
@@ -707,14 +776,16 @@ int fvm2d_advance_dt(fvm2d_solver *s, double dt)
     c->step_limit = c->steps + 1;
     if (int rc = s->upload_control()) return rc;
     CK(cudaEventRecord(s->ev_begin, s->stream));
-    CK(cudaGraphLaunch(s->graph[1], s->stream));
+    if (int rc = s->replay(1)) return rc;
+    CK(s->fill_ring(cfg, s->stream));
     CK(cudaMemcpyAsync(c, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaEventRecord(s->ev_end, s->stream));
     CK(cudaEventSynchronize(s->ev_end));
+    s->stepped(1);
     float dms = 0.f;
     CK(cudaEventElapsedTime(&dms, s->ev_begin, s->ev_end));
     s->last_device_ms = dms;
-    s->last_launches = fvm2d::kStepKernels;
+    s->last_launches = s->step_kernels() + s->tiles();
     s->total_steps += 1;
     return FVM2D_OK;
 }
@@ -742,6 +813,11 @@ int fvm2d_set_row_frame(fvm2d_solver *s, int row0, int ny_global, int fill_top, 
         fill_top = fill_bottom = 1;
     } else if (row0 < 0 || ny_global < row0 + s->ny) {
         return fail(FVM2D_ERR_INVALID, "the slab must lie inside the global rows: 0 <= row0, row0 + ny <= ny_global");
+    }
+    if (ny_global != 0 && s->flip) {  // slabs step in place: the state goes to the first buffer for good
+        CK(cudaMemcpyAsync(s->base, s->U, state_bytes(s->precision, s->plane), cudaMemcpyDeviceToDevice, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        s->set_flip(0);
     }
     s->row0 = row0;
     s->ny_global = ny_global;
@@ -831,6 +907,7 @@ int fvm2d_slab_begin(fvm2d_solver *s, double *smax_out)
     c->step_limit = INT_MAX;
     if (int rc = s->upload_control()) return rc;
     if (int rc = s->build_graphs()) return rc;
+    if (int rc = s->build_slab_graph()) return rc;
     CK(kVariants[s->precision].init(s->config(), s->stream));
     s->need_init = false;
     CK(cudaMemcpyAsync(smax_out, &s->ctl->smax_last, sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
@@ -843,10 +920,11 @@ int fvm2d_slab_step(fvm2d_solver *s, const double *smax_in, double *smax_out)
     if (!s->have_state) return fail(FVM2D_ERR_STATE, "no state has been set");
     if (!smax_in || !smax_out || !is_device_pointer(smax_in) || !is_device_pointer(smax_out))
         return fail(FVM2D_ERR_INVALID, "smax_in and smax_out must be device memory");
-    if (s->graph_variant != s->precision || !s->graph[1])
+    if (s->graph_variant != s->precision || !s->slab_graph)
         return fail(FVM2D_ERR_STATE, "fvm2d_slab_begin must come first (and again after a setter)");
+    if (int rc = s->build_slab_graph()) return rc;  // again if steps since then left the state in the other buffer
     CK(kVariants[s->precision].plan_from(s->config(), s->stream, smax_in));
-    CK(cudaGraphLaunch(s->graph[1], s->stream));
+    CK(cudaGraphLaunch(s->slab_graph, s->stream));
     CK(cudaMemcpyAsync(smax_out, &s->ctl->smax_last, sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
     s->total_steps += 1;
     return FVM2D_OK;
@@ -1039,11 +1117,20 @@ int fvm2d_profile_kernels(fvm2d_solver *s, int nsteps, double *kernel_ms, int *s
         if ((rc = s->upload_control())) break;
         e = s->need_init ? kVariants[s->precision].init(cfg, s->stream) : kVariants[s->precision].plan(cfg, s->stream);
         s->need_init = false;
-        if (!e) e = kVariants[s->precision].step(cfg, s->stream, ev);
+        if (!e && s->tiles()) {
+            for (int q = 0; q < 4; ++q) cudaEventRecord(ev[q], s->stream);
+            e = s->enqueue_step(cfg, s->stream);
+            cudaEventRecord(ev[4], s->stream);
+            if (!e) e = s->fill_ring(cfg, s->stream);
+            cudaEventRecord(ev[5], s->stream);
+        } else if (!e) {
+            e = kVariants[s->precision].step(cfg, s->stream, ev);
+        }
         if (!e) e = cudaMemcpyAsync(c, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream);
         if (!e) e = cudaStreamSynchronize(s->stream);
         if (e) { rc = cuda_fail(e, "profiled step"); break; }
         if (c->steps == before) break;  // the loop has ended: nothing ran
+        s->stepped(1);
         ++done;
         for (int q = 0; q < fvm2d::kStepKernels; ++q) {
             float ms = 0.f;
@@ -1145,9 +1232,12 @@ int fvm2d_jvp(fvm2d_solver *s, int nsteps, const double *tangent_in, double *tan
     if (stride != 4 && stride != 5) return fail(FVM2D_ERR_INVALID, "stride must be 4 or 5 doubles per cell");
     if (nsteps < 0) return fail(FVM2D_ERR_INVALID, "nsteps must be non-negative");
     const long long n4 = 4 * s->plane;
-    if (!s->dual) CK(cudaMalloc(&s->dual, 3 * n4 * sizeof(Dual)));
+    if (!s->dual) {
+        CK(kJvp.prepare());
+        CK(cudaMalloc(&s->dual, 3 * n4 * sizeof(Dual)));
+    }
     Dual *dU = static_cast<Dual *>(s->dual), *dA = dU + n4, *dB = dA + n4;
-    double *T = reinterpret_cast<double *>(dB);  // tangent planes, before packing and after unpacking
+    double *T = reinterpret_cast<double *>(dA);  // tangent planes, before packing and after unpacking
     if (int rc = cells_to_planes(s, tangent_in, stride, T)) return rc;
     pack_dual<<<148 * 4, 256, 0, s->stream>>>(s->U, T, dU, n4);
     CK(cudaGetLastError());
@@ -1155,16 +1245,19 @@ int fvm2d_jvp(fvm2d_solver *s, int nsteps, const double *tangent_in, double *tan
     c.U = dU;
     c.A = dA;
     c.B = dB;
+    c.pair[0] = dU;
+    c.pair[1] = dB;
     StepControl *h = s->ctl_h;
     const int before = h->steps;
     h->step_limit = before + nsteps;
     h->done = 0;
     h->active = 0;
-    if (int rc = s->upload_control()) return rc;
+    if (int rc = s->upload_control(0)) return rc;
     CK(kJvp.init(c, s->stream));
-    for (int k = 0; k < nsteps; ++k) CK(kJvp.step(c, s->stream, nullptr));
+    for (int k = 0; k < nsteps; ++k) CK(s->tiles() ? kJvp.tile_step(c, s->stream) : kJvp.step(c, s->stream, nullptr));
+    if (s->tiles()) CK(kJvp.fill_ring(c, s->stream));
     CK(cudaMemcpyAsync(h, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream));
-    unpack_dual<<<148 * 4, 256, 0, s->stream>>>(dU, s->U, T, n4);
+    unpack_dual<<<148 * 4, 256, 0, s->stream>>>(s->tiles() && (nsteps & 1) ? dB : dU, s->U, T, n4);
     CK(cudaGetLastError());
     if (int rc = planes_to_cells(s, T, tangent_out, stride)) return rc;
     CK(cudaStreamSynchronize(s->stream));
@@ -1185,7 +1278,7 @@ static char *tape_at(const fvm2d_solver *s, int buf, int j, int q, size_t sb)
 // Enqueues on `st` m taped steps (control planned) from the state in slot 0
 // of tape buffer `buf`: step j reads slot j's input state, fills the rest of
 // slot j and writes its result as slot j+1's input state, the last step's
-// into U.
+// into the first state buffer.
 static int taped_steps(fvm2d_solver *s, const LaunchConfig &c, int m, int buf, cudaStream_t st)
 {
     const size_t sb = state_bytes_of(s);
@@ -1198,7 +1291,7 @@ static int taped_steps(fvm2d_solver *s, const LaunchConfig &c, int m, int buf, c
         void *const flux[4] = {tape_at(s, buf, j, 3, sb), tape_at(s, buf, j, 4, sb), tape_at(s, buf, j, 5, sb),
                                tape_at(s, buf, j, 6, sb)};
         void *const out =
-            j + 1 < m ? static_cast<void *>(tape_at(s, buf, j + 1, 0, sb)) : static_cast<void *>(s->U);
+            j + 1 < m ? static_cast<void *>(tape_at(s, buf, j + 1, 0, sb)) : static_cast<void *>(s->base);
         CK(taped_step(cj, st, flux, out));
     }
     return FVM2D_OK;
@@ -1222,6 +1315,8 @@ __global__ void segment_control(StepControl *c, double t, double dt)
         c->done = 0;
         c->ticket = 0u;
         c->first_bad = 0;
+        c->parity = 0;
+        c->ring_due = 0;
     }
 }
 
@@ -1256,6 +1351,7 @@ static int forward_full_tape(fvm2d_solver *s, int nsteps)
     s->need_init = false;
     CK(cudaMemcpyAsync(tape_at(s, 0, 0, 0, sb), s->U, sb, cudaMemcpyDeviceToDevice, s->stream));
     if (int rc = taped_steps(s, c, nsteps, 0, s->stream)) return rc;
+    s->set_flip(0);
     CK(cudaMemcpyAsync(h, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     s->ck_count = 1;
@@ -1379,7 +1475,7 @@ static int vjp_workspace(fvm2d_solver *s, int *bufs)
         const LaunchConfig c = s->config();
         const int len = s->ck_len;
         if (int rc = s->capture(&s->vjp_graph[6], [&] {
-                for (int j = 0; j < len; ++j) CK(kVariants[s->precision].step(c, s->stream, nullptr));
+                for (int j = 0; j < len; ++j) CK(s->enqueue_step(c, s->stream));
                 return FVM2D_OK;
             }))
             return rc;
@@ -1443,20 +1539,17 @@ int fvm2d_forward(fvm2d_solver *s, int nsteps, int checkpoints)
             } else if (int rc = taped_steps(s, c, m, b, s->stream)) {
                 return rc;
             }
-            for (int q = 0; q < m; ++q) t = t + s->fixed_dt;
-            continue;
+            s->set_flip(0);
+        } else {
+            if (count > 1 && m == s->vjp_len) {  // a full segment: one graph of its steps
+                CK(cudaGraphLaunch(s->vjp_graph[6], s->stream));
+            } else if (int rc = s->replay(m)) {
+                return rc;
+            }
+            CK(s->fill_ring(c, s->stream));
+            s->stepped(m);
         }
-        if (count > 1 && m == s->vjp_len) {  // a full segment: one graph of its steps
-            CK(cudaGraphLaunch(s->vjp_graph[6], s->stream));
-            for (int q = 0; q < m; ++q) t = t + s->fixed_dt;
-            continue;
-        }
-        for (int j = 0; j < m;) {
-            const int which = m - j >= fvm2d_solver::kGraphSteps[0] ? 0 : 1;
-            CK(cudaGraphLaunch(s->graph[which], s->stream));
-            for (int q = 0; q < fvm2d_solver::kGraphSteps[which]; ++q) t = t + s->fixed_dt;  // as the device adds
-            j += fvm2d_solver::kGraphSteps[which];
-        }
+        for (int q = 0; q < m; ++q) t = t + s->fixed_dt;  // as the device adds
     }
     CK(cudaMemcpyAsync(h, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));

@@ -20,6 +20,9 @@ struct StepControl {
     unsigned int ticket;           // last-block detection in grid reductions
     int first_bad;                 // 1-based step that first left an interior cell with NaN or
                                    // non-positive density or pressure; 0: none
+    int parity;                    // steps in tiles: which of the two state buffers holds the state
+    int ring_due;                  // 1: the state's ghost ring in memory is not filled yet (steps in
+                                   // tiles fill the ring cells they load; fill_ring stores them)
 };
 
 struct PlanParams {
@@ -34,6 +37,8 @@ struct LaunchConfig {
     int nx, ny, pitch;
     long long plane;       // elements between field planes
     void *U, *A, *B;       // state buffers: U holds the state, A and B are sweep scratch
+    void *pair[2] = {nullptr, nullptr};  // steps in tiles go from pair[parity] to pair[1 - parity]
+                                         // (parity: the control record's), so neither is swept in place
     StepControl *ctl;
     double hx, hy;         // width/nx, height/ny
     double rhx, rhy;       // 1.0/hx, 1.0/hy
@@ -49,6 +54,8 @@ struct LaunchConfig {
 };
 
 // Kernels per step: sweep X, sweep Y, sweep Y, sweep X + average, ghost ring.
+// A step in tiles is one kernel, and one more stores the ghost ring after a
+// group of them.
 constexpr int kStepKernels = 5;
 
 // x-sweep work items: a warp walks `chunks` chunks of 32 cells of one row and
@@ -78,6 +85,8 @@ inline int x_chunks_for(long long rows, int nx, long long resident_warps)
     cudaError_t enqueue_plan(const LaunchConfig &c, cudaStream_t s);           \
     cudaError_t enqueue_plan_from(const LaunchConfig &c, cudaStream_t s, const double *smax); \
     cudaError_t enqueue_step(const LaunchConfig &c, cudaStream_t s, cudaEvent_t *ev); \
+    cudaError_t enqueue_tile_step(const LaunchConfig &c, cudaStream_t s);      \
+    cudaError_t enqueue_fill_ring(const LaunchConfig &c, cudaStream_t s);      \
     }
 
 FVM2D_DECLARE_VARIANT(fp64)

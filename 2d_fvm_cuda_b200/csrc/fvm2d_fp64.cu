@@ -17,4 +17,13 @@
 #define FVM2D_X_MINB 5
 #define FVM2D_Y_MINB 5
 #endif
+// tiles of a step (fvm2d_tile.cuh): warps per block and resident blocks per SM
+#define FVM2D_TILE0_WARPS 10
+#define FVM2D_TILE0_MINB 2
+#define FVM2D_TILE1_WARPS 10
+#define FVM2D_TILE1_MINB 2
+#define FVM2D_TILE2_WARPS 9
+#define FVM2D_TILE2_MINB 2
+#define FVM2D_TILE3_WARPS 10
+#define FVM2D_TILE3_MINB 2
 #include "fvm2d_variant.inc"

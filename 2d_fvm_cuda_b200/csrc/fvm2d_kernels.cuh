@@ -79,6 +79,24 @@ __global__ void plan_from_kernel(StepControl *c, PlanParams p, const double *sma
     }
 }
 
+// Programmatic dependent launch: a kernel launched with it may start while
+// its predecessor on the stream is still running; pdl_wait returns once the
+// predecessor has completed and its writes are visible (at once in a kernel
+// launched without it).  Every thread of such a kernel calls it before it
+// touches global memory, so completion stays in stream order.
+__device__ __forceinline__ void pdl_wait()
+{
+#if defined(__CUDA_ARCH__)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void pdl_launch()
+{
+#if defined(__CUDA_ARCH__)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+
 // Block-wide max of a non-negative double, folded into *bits with one atomic
 // per block.  Values that are NaN never win (the running max ignores them).
 template <int NT>

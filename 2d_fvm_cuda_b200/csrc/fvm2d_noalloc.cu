@@ -71,6 +71,8 @@ __global__ void reset_control(fvm2d::StepControl *c, double t0, int nsteps)
     c->done = 0;
     c->ticket = 0u;
     c->first_bad = 0;
+    c->parity = 0;
+    c->ring_due = 0;
 }
 
 // Once per device, with that device current: the device address of
@@ -146,6 +148,8 @@ int fvm2d_advance_noalloc(const double *state_in, double *state_out, int nx, int
     c.U = state_out;
     c.A = scratch;
     c.B = scratch + 4 * plane;
+    c.pair[0] = c.U;  // steps in tiles go back and forth between the caller's buffer and the scratch
+    c.pair[1] = c.A;
     c.ctl = reinterpret_cast<fvm2d::StepControl *>(scratch + kScratchDoubles);
     c.hx = width / double(nx);
     c.hy = height / double(ny);
@@ -169,12 +173,18 @@ int fvm2d_advance_noalloc(const double *state_in, double *state_out, int nx, int
     do {
         const int n = (nsteps - queued < kStepsPerCheck) ? nsteps - queued : kStepsPerCheck;
         for (int k = 0; k < n; ++k)
-            if ((e = fvm2d::fp64::enqueue_step(c, s, nullptr))) return cuda_fail(e, "step kernels");
+            if ((e = fvm2d::fp64::enqueue_tile_step(c, s))) return cuda_fail(e, "step kernels");
         queued += n;
         if ((e = cudaMemcpyAsync(&out, c.ctl, sizeof(out), cudaMemcpyDeviceToHost, s)))
             return cuda_fail(e, "control read");
         if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "cudaStreamSynchronize");
     } while (out.active && queued < nsteps);
+    if ((e = fvm2d::fp64::enqueue_fill_ring(c, s))) return cuda_fail(e, "ghost ring");
+    if (out.parity) {  // an odd number of steps: the result is in the scratch
+        if ((e = cudaMemcpyAsync(state_out, c.A, sizeof(double) * 4 * plane, cudaMemcpyDeviceToDevice, s)))
+            return cuda_fail(e, "copy of the result");
+    }
+    if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "cudaStreamSynchronize");
     if (t_out) *t_out = out.t;
     if (steps_out) *steps_out = out.steps;
     return FVM2D_OK;

@@ -1,0 +1,402 @@
+// fvm2d_tile.cuh -- a whole split step of one tile of the array per block.
+//
+// A block takes a tile of TX x TY cells it will write, loads it with two
+// cells around it (the reach of a sweep) into shared memory, and runs both
+// split orders there:
+//
+//   phase 0   X(U) on the tile's columns of every loaded row -> A1, and
+//             Y(U) on the tile's rows of every loaded column -> B1
+//   phase 1   Y(A1) on the tile -> RA (over U, which is dead)
+//   phase 2   X(B1) on the tile, averaged with RA, wave-speed maximum and
+//             health test, result to global memory
+//
+// The last tile to finish commits the step and plans the next one.  The ghost
+// ring is not stored between steps: a tile that loads ring cells of a state
+// stepped to in tiles computes them from their interior sources
+// (ring_value); fill_ring_kernel stores the ring once after a group of
+// steps.  A ring cell's wave speed is its source's, which is in the maximum,
+// or an inflow constant's (ring_speed).
+//
+// So the four sweeps' intermediate states never leave the SM: 64 bytes per
+// FP64 cell and step in place of 288, one launch in place of five.  Work on
+// the two halo cells is done again by the neighbouring tiles (30 x 30: 128
+// warp tasks for 900 cells, 12% over four sweeps without overlap), which the
+// shorter instruction stream (no global addresses, clamps, carries or ring
+// copies per sweep: 476 slots per task against 430-640 per cell and sweep)
+// repays even where the array is large.  What bounds a tile is FP64 latency
+// and issue: FP64 pipe 59%, issue slots 60% busy at 20 warps per SM.
+//
+// Steps per second against the sweep kernels with the same arithmetic (FP64,
+// us per step of a varied four-quadrant flow): 400^2 58 -> 30, 131 x 517
+// 48 -> 18, 1003^2 164 -> 111, 4096^2 1830 -> 1640; FP32 4096^2 1240 -> 1070.
+//
+// A warp task is 32 interfaces, one per lane: a lane holds cell c of a line,
+// computes its limited slope, takes the slope of c-1 from its neighbour by
+// shuffle, computes the interface c-1/2, takes the flux of c-3/2 by shuffle
+// and updates c-1.  A line of T updated cells takes T + 2 lanes, so T is 30,
+// 14 or 6 (1, 2 or 4 lines per warp).  Lines along x and along y run the same
+// code with another stride between cells.
+//
+// Shared memory holds rows of four fields (RS elements apart, an odd number,
+// so that lanes along a column meet no bank conflict).
+#pragma once
+
+#include "fvm2d_kernels.cuh"
+
+namespace fvm2d {
+namespace FVM2D_VARIANT {
+
+// A direction's constants with the products its tasks use, in shared memory.
+template <typename Real>
+struct TileConsts : SweepConsts<Real> {
+    Real hh, hrh, rha, hk;
+};
+template <typename Real>
+__device__ __forceinline__ Real half_h(const TileConsts<Real> &K) { return K.hh; }
+template <typename Real>
+__device__ __forceinline__ Real half_rh(const TileConsts<Real> &K) { return K.hrh; }
+template <typename Real>
+__device__ __forceinline__ Real alpha_rh(const TileConsts<Real> &K) { return K.rha; }
+template <typename Real>
+__device__ __forceinline__ Real half_k(const TileConsts<Real> &K) { return K.hk; }
+
+template <typename Real>
+struct TileArgs {
+    Field<Real> src, dst;  // state read and state written (different buffers); the other way round
+                           // if the control record's parity is odd
+    int nx, ny;
+    double hx, hy, rhx, rhy;
+    double alpha, gamma;
+    StepControl *ctl;
+    int strategy;
+    PlanParams plan;
+};
+
+template <typename Real>
+__device__ __forceinline__ GhostArgs<Real> ring_args(const TileArgs<Real> &a)
+{
+    GhostArgs<Real> g;
+    g.U = a.src;
+    g.nx = a.nx;
+    g.ny = a.ny;
+    g.strategy = a.strategy;
+    g.gamma = a.gamma;
+    g.ctl = a.ctl;
+    g.plan = a.plan;
+    g.row0 = 0;
+    g.gny = a.ny;
+    g.fill_top = g.fill_bottom = 1;
+    return g;
+}
+
+// Ring cell (i, j) of a state at time t, from the state's interior.
+template <typename Real>
+__device__ __forceinline__ Cell<Real> ring_value(const GhostArgs<Real> &g, int i, int j, double t)
+{
+    return i < 2 || i >= g.nx - 2 ? col_rule(g, i, j, t) : row_rule(g, i, j, t);
+}
+
+// The largest wave speed of the ring cells that copy no interior cell: the
+// inflow states of the presets that have them, each of which is on the ring
+// of any array (the left columns' at least).
+template <typename Real>
+__device__ __forceinline__ double ring_speed(int strategy, double gamma)
+{
+    auto speed = [&](double r, double p, double u, double v) {
+        const Cell<Real> c = mk<Real>(r, p, u, v);
+        return wave_speed(c.rho, c.p, c.un, c.ut, gamma);
+    };
+    switch (strategy) {
+    case OUTFLOW:
+    case PERIODIC:
+    case REFLECTIVE_TB:
+        return 0.0;
+    case JET:
+        return fmax(speed(5.0, 0.4127, 800.0, 0.0), speed(0.5, 0.4127, 0.0, 0.0));
+    case JET800:
+        return fmax(speed(1.4, 1, 800, 0), speed(0.14, 1, 0, 0));
+    default:
+        return fmax(speed(8, 116.5, 4.125 * sqrt(3.0), -4.125), speed(1.4, 1, 0, 0));
+    }
+}
+
+// Geometry of a tile: TX x TY written cells, NW warps.
+template <int TX_, int TY_, int NW_>
+struct Tile {
+    static constexpr int TX = TX_, TY = TY_, NW = NW_, NT = 32 * NW_;
+    static constexpr int SX = TX + 2, SY = TY + 2;    // lanes per line
+    static constexpr int RX = 32 / SX, CY = 32 / SY;  // lines per warp task
+    static constexpr int NC = TX + 4, NR = TY + 4;    // loaded columns, rows
+    static constexpr int RS = 4 * NC + 1;             // elements between rows
+    static_assert(32 % SX == 0 && 32 % SY == 0, "a line takes 8, 16 or 32 lanes");
+    // U, A1: NR rows; B1: TY rows
+    static constexpr int kElems = (2 * NR + TY) * RS;
+    static constexpr int kLo = NC | 1;                // residual words per row
+    static constexpr int kLoWords = (2 * NR + TY) * kLo;
+    template <typename Real, class Phys>
+    static constexpr size_t bytes()
+    {
+        return 2 * sizeof(TileConsts<Real>) + (kElems + 1) / 2 * 2 * sizeof(Real) +
+               (split_storage<Phys>::value ? kLoWords * sizeof(unsigned long long) : 0);
+    }
+};
+
+template <typename Real>
+__device__ __forceinline__ void tile_copy(Real *dst_shared, const Real *src)
+{
+    if constexpr (sizeof(Real) == 4 || sizeof(Real) == 8)
+        async_copy(dst_shared, src);
+    else
+        *dst_shared = *src;
+}
+
+// One step of tile (bx, by), by the Tile::NT threads of a block; fill: the
+// state's ring cells are computed for time t, else read.
+template <typename Real, class Phys, class T>
+__device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, int bx, int by, unsigned char *smem,
+                                          double &vmax, int &bad, bool fill = false, double t = 0.0)
+{
+    constexpr bool kResidual = split_storage<Phys>::value;
+    using Word = unsigned long long;
+    constexpr int NC = T::NC, RS = T::RS;
+    TileConsts<Real> *const KK = reinterpret_cast<TileConsts<Real> *>(smem);
+    Real *const sU = reinterpret_cast<Real *>(KK + 2);
+    Real *const sA = sU + T::NR * RS;
+    Real *const sB = sA + (T::NR - 2) * RS;  // rows 2 .. TY+1 of B1 (rows 0, 1 are not kept)
+    Word *const lU = reinterpret_cast<Word *>(sU + (T::kElems + 1) / 2 * 2);
+    Word *const lA = lU + T::NR * T::kLo, *const lB = lA + (T::NR - 2) * T::kLo;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
+    const int x0 = 2 + bx * T::TX, y0 = 2 + by * T::TY;  // first written cell
+    const int ncol = min(NC, a.nx - x0 + 2), nrow = min(T::NR, a.ny - y0 + 2);  // loaded columns and rows in the array
+
+    // does the loaded tile reach the ring?
+    const bool edge = fill && (bx == 0 || by == 0 || x0 - 2 + NC > a.nx - 2 || y0 - 2 + T::NR > a.ny - 2);
+    for (int i = tid; i < T::NR * NC; i += T::NT) {
+        const int r = i / NC, c = i - r * NC;
+        if (r >= nrow) break;
+        const int x = min(x0 - 2 + c, a.nx - 1), y = y0 - 2 + r;
+        Real *const q = sU + r * RS + c;
+        if (edge && (x < 2 || x >= a.nx - 2 || y < 2 || y >= a.ny - 2)) {
+            const Cell<Real> v = ring_value(ring_args(a), x, y, t);
+            q[0] = v.rho;
+            q[NC] = v.p;
+            q[2 * NC] = v.un;
+            q[3 * NC] = v.ut;
+            if constexpr (kResidual) lU[r * T::kLo + c] = 0ull;  // a ring cell holds its FP32 value exactly
+            continue;
+        }
+        tile_copy(q, &a.src.at(0, x, y));
+        tile_copy(q + NC, &a.src.at(1, x, y));
+        tile_copy(q + 2 * NC, &a.src.at(2, x, y));
+        tile_copy(q + 3 * NC, &a.src.at(3, x, y));
+        if constexpr (kResidual) async_copy(lU + r * T::kLo + c, &lo_cell(a.src, x, y));
+    }
+    async_commit();
+    if (tid < 2) {
+        TileConsts<Real> K;
+        const double h = tid == 0 ? a.hx : a.hy;
+        K.h = Real(h);
+        K.rh = Real(tid == 0 ? a.rhx : a.rhy);
+        K.alpha = Real(a.alpha);
+        set_gamma_consts(K, a.gamma);
+        K.k = Real(dt);
+        K.lambda = Real(dt / h);
+        K.lambda_lo = Real(lo_part<Real>(dt / h));
+        K.hh = K.h * Real(0.5);
+        K.hrh = K.rh * Real(0.5);
+        K.rha = K.rh * K.alpha;
+        K.hk = K.k * Real(0.5);
+        KK[tid] = K;
+    }
+    async_wait<0>();
+    __syncthreads();
+
+    const int nx_rows0 = (nrow + T::RX - 1) / T::RX;  // phase 0: x tasks, then y tasks
+    for (int phase = 0; phase < 3; ++phase) {
+        const int ntask = phase == 0   ? nx_rows0 + (ncol + T::CY - 1) / T::CY
+                          : phase == 1 ? (ncol - 4 + T::CY - 1) / T::CY
+                                       : (nrow - 4 + T::RX - 1) / T::RX;
+        for (int t = warp; t < ntask; t += T::NW) {
+            const bool xdir = phase == 2 || (phase == 0 && t < nx_rows0);
+            // this lane's cell: row r, column c of the loaded tile; k its place on the line
+            int k, r, c, s;
+            bool mine;
+            if (xdir) {
+                k = lane & (T::SX - 1);
+                const int line = t * T::RX + lane / T::SX, n = phase == 0 ? nrow : nrow - 4;
+                mine = line < n;
+                r = min(line, n - 1) + (phase == 0 ? 0 : 2);
+                c = k + 1;
+                s = 1;
+            } else {
+                k = lane & (T::SY - 1);
+                const int line = (phase == 0 ? t - nx_rows0 : t) * T::CY + lane / T::SY, n = phase == 0 ? ncol : ncol - 4;
+                mine = line < n;
+                c = min(line, n - 1) + (phase == 0 ? 0 : 2);
+                r = T::TY + 2 - k;  // lines along y start at the bottom (u_n = v)
+                s = -RS;
+            }
+            const Real *const from = phase == 0 ? sU : phase == 1 ? sA : sB;
+            const Real *const q = from + r * RS + c;
+            const int on = xdir ? 2 * NC : 3 * NC, ot = 5 * NC - on;
+            auto get = [&](const Real *p) { return Cell<Real>{p[0], p[NC], p[on], p[ot]}; };
+            const TileConsts<Real> &K = KK[xdir ? 0 : 1];
+            Cell<Real> s0, F;
+            {
+                const Cell<Real> cm1 = get(q - s), c0 = get(q);
+                s0 = Phys::slope(cm1, c0, get(q + s), K);
+                F = Phys::interface_flux(cm1, c0, shfl_up(s0), s0, K);
+            }
+            const Cell<Real> FL = shfl_up(F);
+            // the updated cell: one back along the line
+            const int ru = xdir ? r : r + 1, cu = xdir ? c - 1 : c;
+            if (!mine || k < 2) continue;
+            if (phase < 2) {
+                Real *const d = (phase == 1 ? sU : xdir ? sA : sB) + ru * RS + cu;
+                if constexpr (kResidual) {
+                    const Word w = (phase == 0 ? lU : lA)[ru * T::kLo + cu];
+                    auto part = [&](int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
+                    const int fn = xdir ? 2 : 3;
+                    const Cell<Real> lo = {part(0), part(1), part(fn), part(5 - fn)};
+                    const Cell<double> v = Phys::update_split(get(q - s), lo, FL, F, K);
+                    float h[4];
+                    unsigned short l[4];
+                    split_value(v.rho, h[0], l[0]);
+                    split_value(v.p, h[1], l[1]);
+                    split_value(v.un, h[2], l[fn]);
+                    split_value(v.ut, h[3], l[5 - fn]);
+                    (phase == 1 ? lU : xdir ? lA : lB)[ru * T::kLo + cu] =
+                        (Word)l[0] | (Word)l[1] << 16 | (Word)l[2] << 32 | (Word)l[3] << 48;
+                    d[0] = h[0];
+                    d[NC] = h[1];
+                    d[on] = h[2];
+                    d[ot] = h[3];
+                } else {
+                    const Cell<Real> v = Phys::update(get(q - s), FL, F, K);
+                    d[0] = v.rho;
+                    d[NC] = v.p;
+                    d[on] = v.un;
+                    d[ot] = v.ut;
+                }
+            } else {
+                const int x = x0 - 2 + cu, y = y0 - 2 + ru;
+                const Real *const ra = sU + ru * RS + cu;
+                const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
+                if (x > a.nx - 3) continue;
+                if constexpr (kResidual) {
+                    auto part = [](Word w, int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
+                    auto parts = [&](Word w) { return Cell<Real>{part(w, 0), part(w, 1), part(w, 2), part(w, 3)}; };
+                    const Cell<double> v = Phys::update_split(get(q - s), parts(lB[ru * T::kLo + cu]), FL, F, K);
+                    const Cell<double> b = join_cell(A, parts(lU[ru * T::kLo + cu]));
+                    const Cell<double> o = {(b.rho + v.rho) * 0.5, (b.p + v.p) * 0.5, (b.un + v.un) * 0.5,
+                                            (b.ut + v.ut) * 0.5};
+                    const Cell<Real> h = store_split(a.dst, x, y, 2, 3, o);
+                    vmax = fmax(vmax, wave_speed(h.rho, h.p, h.un, h.ut, a.gamma));
+                    bad |= !(h.rho > Real(0) && h.p > Real(0));
+                } else {
+                    // primitive average with branch A (src/basicFuns.cuh:264-274)
+                    const Cell<Real> v = Phys::update(get(q - s), FL, F, K);
+                    Cell<Real> o;
+                    o.rho = (A.rho + v.rho) * Real(0.5);
+                    o.p = (A.p + v.p) * Real(0.5);
+                    o.un = (A.un + v.un) * Real(0.5);
+                    o.ut = (A.ut + v.ut) * Real(0.5);
+                    store_cell(a.dst, x, y, 2, 3, o);
+                    vmax = fmax(vmax, wave_speed(o.rho, o.p, o.un, o.ut, a.gamma));
+                    bad |= !(o.rho > Real(0) && o.p > Real(0));  // NaN fails both tests
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Ends a step in tiles (its last block): commits it as finish_step does, with
+// the state now in the other buffer and its ring unfilled.  `c` is the record
+// as the step began, of which a step changes nothing but smax_bits, ticket
+// and first_bad, so the only value waited for is the maximum.
+__device__ __forceinline__ void finish_tile_step(StepControl *ctl, StepControl c, const PlanParams &plan)
+{
+    c.smax_last = __longlong_as_double((long long)*(volatile unsigned long long *)&ctl->smax_bits);
+    ctl->smax_bits = 0ull;
+    c.t = c.t + c.dt;
+    c.steps += 1;
+    plan_step(&c, plan);
+    ctl->ticket = 0u;
+    ctl->t = c.t;
+    ctl->dt = c.dt;
+    ctl->smax_last = c.smax_last;
+    ctl->steps = c.steps;
+    ctl->active = c.active;
+    ctl->done = c.done;
+    ctl->parity = c.parity ^ 1;
+    ctl->ring_due = 1;
+}
+
+// Folds the block's maxima into the record and ends the step in the last of
+// the nblocks blocks of its problem.
+template <int NT>
+__device__ __forceinline__ void end_tile(double vmax, int bad, StepControl *ctl, const StepControl &c,
+                                         const PlanParams &plan, unsigned nblocks)
+{
+    __shared__ double red[NT / 32];
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicCAS(&ctl->first_bad, 0, c.steps + 1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x / 32] = vmax;
+        if (bad) __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+#pragma unroll
+    for (int w = 1; w < NT / 32; ++w) vmax = fmax(vmax, red[w]);
+    if (vmax > 0.0) atomicMax(&ctl->smax_bits, (unsigned long long)__double_as_longlong(vmax));
+    __threadfence();
+    if (atomicAdd(&ctl->ticket, 1u) == nblocks - 1) {
+        __threadfence();
+        finish_tile_step(ctl, c, plan);
+    }
+}
+
+#ifdef __CUDACC__  // (host builds of this file call tile_step)
+template <typename Real, class Phys, class T, int MINB>
+__global__ void __launch_bounds__(T::NT, MINB) step_tile_kernel(TileArgs<Real> a)
+{
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    pdl_launch();
+    pdl_wait();
+    __shared__ StepControl c;
+    if (threadIdx.x == 0) c = *a.ctl;
+    __syncthreads();
+    if (!c.active) return;
+    if (c.parity) {
+        const Field<Real> f = a.src;
+        a.src = a.dst;
+        a.dst = f;
+    }
+    double vmax = 0.0;
+    int bad = 0;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
+    tile_step<Real, Phys, T>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, c.ring_due, c.t);
+    end_tile<T::NT>(vmax, bad, a.ctl, c, a.plan, gridDim.x * gridDim.y);
+}
+
+// Stores the ghost ring after steps in tiles (src: the state if the parity
+// is even, dst: if odd).  One thread per ring cell.
+template <typename Real, int NT>
+__global__ void __launch_bounds__(NT) fill_ring_kernel(TileArgs<Real> a, int residual)
+{
+    pdl_launch();
+    pdl_wait();
+    if (!a.ctl->ring_due) return;
+    if (a.ctl->parity) a.src = a.dst;
+    GhostArgs<Real> g = ring_args(a);
+    g.residual = residual;
+    const int k = blockIdx.x * NT + threadIdx.x;
+    if (k < 4 * a.nx + 4 * (a.ny - 4)) ghost_cell(g, k, a.ctl->t);
+}
+#endif
+
+} // namespace FVM2D_VARIANT
+} // namespace fvm2d

@@ -262,9 +262,11 @@ int fvm2d_get_time(fvm2d_solver *s, double *t, int *steps, double *last_dt);
 int fvm2d_get_run_stats(fvm2d_solver *s, double *device_ms, long long *kernel_launches);
 
 /* Runs up to nsteps steps one at a time outside the graph, with CUDA events
- * between the five kernels of a step (sweep X, sweep Y, sweep Y, final sweep X
- * + average, ghost ring); kernel_ms[0..4] receive their mean durations in
- * milliseconds and *steps_done the steps taken.  Advances the state like
+ * between the kernels of a step; kernel_ms[0..4] receive their mean durations
+ * in milliseconds and *steps_done the steps taken.  A whole problem steps in
+ * tiles, all four sweeps and the average in one kernel: [3] is that kernel,
+ * [4] the ghost ring's, [0..2] next to nothing.  A row slab's step has five:
+ * sweep X, sweep Y, sweep Y, final sweep X + average, ghost ring.  Advances the state like
  * fvm2d_advance.  No reference counterpart (diagnostics). */
 int fvm2d_profile_kernels(fvm2d_solver *s, int nsteps, double *kernel_ms, int *steps_done);
 
@@ -367,10 +369,11 @@ int fvm2d_batch_get_time(fvm2d_batch *b, int p, double *t, int *steps);
 int fvm2d_batch_get_run_stats(fvm2d_batch *b, double *device_ms, long long *kernel_launches,
                               long long *cell_updates);
 
-/* Times trial_steps steps of the batch for each candidate y-sweep segment
- * length (16, 32, 64 interfaces) and sweep grid size (1, 2, 4 times the
- * resident blocks), keeps the fastest and restores the states; reports the
- * choice. */
+/* Times trial_steps steps of the batch in tiles and for each candidate
+ * y-sweep segment length (16, 32, 64 interfaces) and sweep grid size (1, 2, 4
+ * times the resident blocks), keeps the fastest and restores the states;
+ * reports the best segment length and grid (in use unless the tiles were
+ * faster). */
 int fvm2d_batch_autotune(fvm2d_batch *b, int trial_steps, int *segment_interfaces, int *grid_blocks);
 
 /* Largest nx * ny that fvm2d_advance_noalloc accepts. */
