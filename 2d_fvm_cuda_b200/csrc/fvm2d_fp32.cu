@@ -20,14 +20,15 @@
 #define FVM2D_X_MINB 6
 #define FVM2D_Y_MINB 6
 #endif
-// tiles of a step (fvm2d_tile.cuh): warps per block and resident blocks per SM
+// tiles of a step (fvm2d_tile.cuh): warps per block and resident blocks per SM,
+// and the rule on sizes (best_tile_shape); measured best of several for this build
 #define FVM2D_TILE0_WARPS 8
 #define FVM2D_TILE0_MINB 4
-#define FVM2D_TILE1_WARPS 8
-#define FVM2D_TILE1_MINB 4
+#define FVM2D_TILE1_WARPS 10
+#define FVM2D_TILE1_MINB 3
 #define FVM2D_TILE2_WARPS 9
 #define FVM2D_TILE2_MINB 3
 #define FVM2D_TILE3_WARPS 10
-#define FVM2D_TILE3_MINB 3
+#define FVM2D_TILE3_MINB 2
 #include "fvm2d_packed.cuh"
 #include "fvm2d_variant.inc"

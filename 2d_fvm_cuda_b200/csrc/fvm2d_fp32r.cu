@@ -20,8 +20,9 @@
 #define FVM2D_X_MINB 6
 #define FVM2D_Y_MINB 6
 #endif
-// tiles of a step (fvm2d_tile.cuh): warps per block and resident blocks per SM
-#define FVM2D_TILE0_WARPS 10
+// tiles of a step (fvm2d_tile.cuh): warps per block and resident blocks per SM,
+// and the rule on sizes (best_tile_shape); measured best of several for this build
+#define FVM2D_TILE0_WARPS 12
 #define FVM2D_TILE0_MINB 2
 #define FVM2D_TILE1_WARPS 8
 #define FVM2D_TILE1_MINB 3

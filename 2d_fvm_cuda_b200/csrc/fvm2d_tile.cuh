@@ -10,6 +10,11 @@
 //   phase 2   X(B1) on the tile, averaged with RA, wave-speed maximum and
 //             health test, result to global memory
 //
+// The smaller shapes, which serve arrays whose steps are a chain of latencies,
+// take the tasks of phases 1 and 2 together (X(B1) -> RB) and average after
+// one more barrier: 14 x 6 tiles then run two rounds of tasks instead of
+// three.
+//
 // The last tile to finish commits the step and plans the next one.  The ghost
 // ring is not stored between steps: a tile that loads ring cells of a state
 // stepped to in tiles computes them from their interior sources
@@ -26,7 +31,7 @@
 // repays even where the array is large.  What bounds a tile is FP64 latency
 // and issue: FP64 pipe 59%, issue slots 60% busy at 20 warps per SM.
 //
-// Steps per second against the sweep kernels with the same arithmetic (FP64,
+// Against the sweep kernels with the same arithmetic (FP64,
 // us per step of a varied four-quadrant flow): 400^2 58 -> 30, 131 x 517
 // 48 -> 18, 1003^2 164 -> 111, 4096^2 1830 -> 1640; FP32 4096^2 1240 -> 1070.
 //
@@ -129,8 +134,11 @@ struct Tile {
     static constexpr int NC = TX + 4, NR = TY + 4;    // loaded columns, rows
     static constexpr int RS = 4 * NC + 1;             // elements between rows
     static_assert(32 % SX == 0 && 32 % SY == 0, "a line takes 8, 16 or 32 lanes");
-    // U, A1: NR rows; B1: TY rows
-    static constexpr int kElems = (2 * NR + TY) * RS;
+    // phases 1 and 2 together (30 x 30 has no shared memory left for RB)
+    static constexpr bool kMerge = TX * TY < 900;
+    // U, A1: NR rows; B1, RB: TY rows
+    static constexpr int kRows = 2 * NR + TY + (kMerge ? TY : 0);
+    static constexpr int kElems = kRows * RS;
     static constexpr int kLo = NC | 1;                // residual words per row
     static constexpr int kLoWords = (2 * NR + TY) * kLo;
     template <typename Real, class Phys>
@@ -159,10 +167,13 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
     constexpr bool kResidual = split_storage<Phys>::value;
     using Word = unsigned long long;
     constexpr int NC = T::NC, RS = T::RS;
+    // (a residual build's branch B is averaged before it is split)
+    constexpr bool MERGE = T::kMerge && !kResidual;
     TileConsts<Real> *const KK = reinterpret_cast<TileConsts<Real> *>(smem);
     Real *const sU = reinterpret_cast<Real *>(KK + 2);
     Real *const sA = sU + T::NR * RS;
     Real *const sB = sA + (T::NR - 2) * RS;  // rows 2 .. TY+1 of B1 (rows 0, 1 are not kept)
+    Real *const sR = sB + T::TY * RS;        // the same rows of RB
     Word *const lU = reinterpret_cast<Word *>(sU + (T::kElems + 1) / 2 * 2);
     Word *const lA = lU + T::NR * T::kLo, *const lB = lA + (T::NR - 2) * T::kLo;
     const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
@@ -211,32 +222,61 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
     async_wait<0>();
     __syncthreads();
 
-    const int nx_rows0 = (nrow + T::RX - 1) / T::RX;  // phase 0: x tasks, then y tasks
-    for (int phase = 0; phase < 3; ++phase) {
-        const int ntask = phase == 0   ? nx_rows0 + (ncol + T::CY - 1) / T::CY
-                          : phase == 1 ? (ncol - 4 + T::CY - 1) / T::CY
-                                       : (nrow - 4 + T::RX - 1) / T::RX;
+    // residual word -> the residuals of fields 0, 1, f2, f3
+    auto parts = [](Word w, int f2, int f3) {
+        auto part = [&](int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
+        return Cell<Real>{part(0), part(1), part(f2), part(f3)};
+    };
+    // the step's result at tile cell (r, c): branch A (ra, la) averaged with
+    // branch B in primitive variables (src/basicFuns.cuh:264-274)
+    auto finish = [&](int r, int c, auto b) {
+        const int x = x0 - 2 + c, y = y0 - 2 + r;
+        const Real *const ra = sU + r * RS + c;
+        const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
+        Cell<Real> o;
+        if constexpr (kResidual) {
+            const Cell<double> d = join_cell(A, parts(lU[r * T::kLo + c], 2, 3));
+            o = store_split(a.dst, x, y, 2, 3,
+                            Cell<double>{(d.rho + b.rho) * 0.5, (d.p + b.p) * 0.5, (d.un + b.un) * 0.5,
+                                         (d.ut + b.ut) * 0.5});
+        } else {
+            o.rho = (A.rho + b.rho) * Real(0.5);
+            o.p = (A.p + b.p) * Real(0.5);
+            o.un = (A.un + b.un) * Real(0.5);
+            o.ut = (A.ut + b.ut) * Real(0.5);
+            store_cell(a.dst, x, y, 2, 3, o);
+        }
+        vmax = fmax(vmax, wave_speed(o.rho, o.p, o.un, o.ut, a.gamma));
+        bad |= !(o.rho > Real(0) && o.p > Real(0));  // NaN fails both tests
+    };
+
+    // tasks along x and along y of the two sweeps of each branch
+    const int nx0 = (nrow + T::RX - 1) / T::RX, ny0 = (ncol + T::CY - 1) / T::CY;
+    const int ny1 = (ncol - 4 + T::CY - 1) / T::CY, nx1 = (nrow - 4 + T::RX - 1) / T::RX;
+    for (int phase = 0; phase < (MERGE ? 2 : 3); ++phase) {
+        const int ntask = phase == 0 ? nx0 + ny0 : MERGE ? ny1 + nx1 : phase == 1 ? ny1 : nx1;
         for (int t = warp; t < ntask; t += T::NW) {
-            const bool xdir = phase == 2 || (phase == 0 && t < nx_rows0);
+            const bool xdir = phase == 0 ? t < nx0 : MERGE ? t >= ny1 : phase == 2;
             // this lane's cell: row r, column c of the loaded tile; k its place on the line
             int k, r, c, s;
             bool mine;
             if (xdir) {
                 k = lane & (T::SX - 1);
-                const int line = t * T::RX + lane / T::SX, n = phase == 0 ? nrow : nrow - 4;
+                const int line = (MERGE && phase ? t - ny1 : t) * T::RX + lane / T::SX;
+                const int n = phase == 0 ? nrow : nrow - 4;
                 mine = line < n;
                 r = min(line, n - 1) + (phase == 0 ? 0 : 2);
                 c = k + 1;
                 s = 1;
             } else {
                 k = lane & (T::SY - 1);
-                const int line = (phase == 0 ? t - nx_rows0 : t) * T::CY + lane / T::SY, n = phase == 0 ? ncol : ncol - 4;
+                const int line = (phase == 0 ? t - nx0 : t) * T::CY + lane / T::SY, n = phase == 0 ? ncol : ncol - 4;
                 mine = line < n;
                 c = min(line, n - 1) + (phase == 0 ? 0 : 2);
                 r = T::TY + 2 - k;  // lines along y start at the bottom (u_n = v)
                 s = -RS;
             }
-            const Real *const from = phase == 0 ? sU : phase == 1 ? sA : sB;
+            const Real *const from = phase == 0 ? sU : xdir ? sB : sA;
             const Real *const q = from + r * RS + c;
             const int on = xdir ? 2 * NC : 3 * NC, ot = 5 * NC - on;
             auto get = [&](const Real *p) { return Cell<Real>{p[0], p[NC], p[on], p[ot]}; };
@@ -251,63 +291,52 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
             // the updated cell: one back along the line
             const int ru = xdir ? r : r + 1, cu = xdir ? c - 1 : c;
             if (!mine || k < 2) continue;
-            if (phase < 2) {
-                Real *const d = (phase == 1 ? sU : xdir ? sA : sB) + ru * RS + cu;
-                if constexpr (kResidual) {
-                    const Word w = (phase == 0 ? lU : lA)[ru * T::kLo + cu];
-                    auto part = [&](int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
-                    const int fn = xdir ? 2 : 3;
-                    const Cell<Real> lo = {part(0), part(1), part(fn), part(5 - fn)};
-                    const Cell<double> v = Phys::update_split(get(q - s), lo, FL, F, K);
-                    float h[4];
-                    unsigned short l[4];
-                    split_value(v.rho, h[0], l[0]);
-                    split_value(v.p, h[1], l[1]);
-                    split_value(v.un, h[2], l[fn]);
-                    split_value(v.ut, h[3], l[5 - fn]);
-                    (phase == 1 ? lU : xdir ? lA : lB)[ru * T::kLo + cu] =
-                        (Word)l[0] | (Word)l[1] << 16 | (Word)l[2] << 32 | (Word)l[3] << 48;
-                    d[0] = h[0];
-                    d[NC] = h[1];
-                    d[on] = h[2];
-                    d[ot] = h[3];
-                } else {
-                    const Cell<Real> v = Phys::update(get(q - s), FL, F, K);
-                    d[0] = v.rho;
-                    d[NC] = v.p;
-                    d[on] = v.un;
-                    d[ot] = v.ut;
-                }
+            const int fn = xdir ? 2 : 3;
+            auto updated = [&] {
+                if constexpr (kResidual)
+                    return Phys::update_split(get(q - s),
+                                              parts((phase == 0 ? lU : xdir ? lB : lA)[ru * T::kLo + cu], fn, 5 - fn),
+                                              FL, F, K);
+                else
+                    return Phys::update(get(q - s), FL, F, K);
+            };
+            if (!MERGE && phase == 2) {
+                if (x0 - 2 + cu <= a.nx - 3) finish(ru, cu, updated());
+                continue;
+            }
+            Real *const d = (phase == 0 ? (xdir ? sA : sB) : xdir ? sR : sU) + ru * RS + cu;
+            const auto v = updated();
+            if constexpr (kResidual) {
+                float h[4];
+                unsigned short l[4];
+                split_value(v.rho, h[0], l[0]);
+                split_value(v.p, h[1], l[1]);
+                split_value(v.un, h[2], l[fn]);
+                split_value(v.ut, h[3], l[5 - fn]);
+                (phase == 0 ? (xdir ? lA : lB) : lU)[ru * T::kLo + cu] =
+                    (Word)l[0] | (Word)l[1] << 16 | (Word)l[2] << 32 | (Word)l[3] << 48;
+                d[0] = h[0];
+                d[NC] = h[1];
+                d[on] = h[2];
+                d[ot] = h[3];
             } else {
-                const int x = x0 - 2 + cu, y = y0 - 2 + ru;
-                const Real *const ra = sU + ru * RS + cu;
-                const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
-                if (x > a.nx - 3) continue;
-                if constexpr (kResidual) {
-                    auto part = [](Word w, int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
-                    auto parts = [&](Word w) { return Cell<Real>{part(w, 0), part(w, 1), part(w, 2), part(w, 3)}; };
-                    const Cell<double> v = Phys::update_split(get(q - s), parts(lB[ru * T::kLo + cu]), FL, F, K);
-                    const Cell<double> b = join_cell(A, parts(lU[ru * T::kLo + cu]));
-                    const Cell<double> o = {(b.rho + v.rho) * 0.5, (b.p + v.p) * 0.5, (b.un + v.un) * 0.5,
-                                            (b.ut + v.ut) * 0.5};
-                    const Cell<Real> h = store_split(a.dst, x, y, 2, 3, o);
-                    vmax = fmax(vmax, wave_speed(h.rho, h.p, h.un, h.ut, a.gamma));
-                    bad |= !(h.rho > Real(0) && h.p > Real(0));
-                } else {
-                    // primitive average with branch A (src/basicFuns.cuh:264-274)
-                    const Cell<Real> v = Phys::update(get(q - s), FL, F, K);
-                    Cell<Real> o;
-                    o.rho = (A.rho + v.rho) * Real(0.5);
-                    o.p = (A.p + v.p) * Real(0.5);
-                    o.un = (A.un + v.un) * Real(0.5);
-                    o.ut = (A.ut + v.ut) * Real(0.5);
-                    store_cell(a.dst, x, y, 2, 3, o);
-                    vmax = fmax(vmax, wave_speed(o.rho, o.p, o.un, o.ut, a.gamma));
-                    bad |= !(o.rho > Real(0) && o.p > Real(0));  // NaN fails both tests
-                }
+                d[0] = v.rho;
+                d[NC] = v.p;
+                d[on] = v.un;
+                d[ot] = v.ut;
             }
         }
         __syncthreads();
+    }
+    if constexpr (MERGE) {
+        const int w = ncol - 4;
+        for (int i = tid; i < T::TY * T::TX; i += T::NT) {
+            const int r = 2 + i / T::TX, c = 2 + i % T::TX;
+            if (c - 2 >= w || r - 2 >= nrow - 4) continue;
+            const Real *const rb = sR + r * RS + c;
+            const Cell<Real> b = {rb[0], rb[NC], rb[2 * NC], rb[3 * NC]};
+            finish(r, c, b);
+        }
     }
 }
 
