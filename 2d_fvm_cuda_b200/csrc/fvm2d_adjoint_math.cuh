@@ -33,6 +33,18 @@ __device__ __forceinline__ int slope_choice(A m, A c, A p, A rh, A alpha)
     return (a2 < a1) ? 3 : 2;
 }
 
+// The slope itself (Hoisted's limiter) with its choice.
+__device__ __forceinline__ A slope_with_choice(A m, A c, A p, A hrh, A rha, int &choice)
+{
+    const A d1 = c - m, d2 = p - c, dc = p - m;
+    const A a1 = fabs(d1), a2 = fabs(d2);
+    const bool forward = a2 < a1;
+    const A inner = rha * (forward ? a2 : a1), outer = fabs(dc) * hrh;
+    const bool one_sided = inner < outer, sloped = d1 * d2 > A(0);
+    choice = !sloped ? 0 : !one_sided ? 1 : forward ? 3 : 2;
+    return sloped ? copysign(one_sided ? inner : outer, dc) : A(0);
+}
+
 // Adds the adjoint of one slope component (sbar) to its three cells.
 __device__ __forceinline__ void slope_adjoint(int choice, A sbar, A rh, A alpha, A &mbar, A &cbar, A &pbar)
 {
@@ -86,493 +98,303 @@ __device__ __forceinline__ Cell<A> update_adjoint(const Cell<A> &U, const Cell<A
 }
 
 // ---- interface: face states, relaxation GRP, midpoint flux -------------------
+// One side of an interface in Hoisted::grp's terms: the face state and its
+// slopes, i = 1/(rho a), the relaxation speed c with ic = 1/c and s = c/rho,
+// the sound-speed slope cx = (gamma/2) Y i with Y = p rho_x + rho p_x.
+struct Side {
+    A r, p, u, v, rx, px, ux, vx;
+    A gp, i, Y, cx, c, ic, s;
+};
+// The adjoints of a side's quantities.
+struct SideAdjoint {
+    A r = 0, p = 0, u = 0, v = 0, rx = 0, px = 0, ux = 0, vx = 0, i = 0, cx = 0, c = 0, ic = 0, s = 0;
+};
+
+// Adjoint of Hoisted::flux_of at the interface state W and its derivative Wt.
+__device__ __forceinline__ void flux_adjoint(const Cell5 &W, const Cell5 &Wt, A hk, const Cell<A> &Fb, Cell5 &Wb,
+                                             Cell5 &Wtb)
+{
+    const A half = A(0.5);
+    const A m = W.rho * W.un, M = fma(hk, fma(W.rho, Wt.un, W.un * Wt.rho), m), Q = fma(hk, Wt.p, W.p), hm = hk * m;
+    const A es = fma(half, fma(W.un, W.un, W.ut * W.ut), W.e), et = fma(W.un, Wt.un, fma(W.ut, Wt.ut, Wt.e));
+    // F = (M, M un + hm un_t + Q, es M + hm et + un Q + hk p un_t, M ut + hm ut_t)
+    const A Mb = fma(W.un, Fb.p, fma(es, Fb.un, fma(W.ut, Fb.ut, Fb.rho))), Qb = fma(W.un, Fb.un, Fb.p);
+    const A hmb = fma(Wt.un, Fb.p, fma(et, Fb.un, Wt.ut * Fb.ut));
+    const A esb = M * Fb.un, etb = hm * Fb.un, he = hk * Fb.un;
+    const A mb = fma(hk, hmb, Mb), mtb = hk * Mb;
+    Wb.rho = fma(Wt.un, mtb, W.un * mb);
+    Wb.p = fma(he, Wt.un, Qb);
+    Wb.un = fma(M, Fb.p, fma(Q, Fb.un, fma(Wt.un, etb, fma(W.un, esb, fma(Wt.rho, mtb, W.rho * mb)))));
+    Wb.ut = fma(M, Fb.ut, fma(Wt.ut, etb, W.ut * esb));
+    Wb.e = esb;
+    Wtb.rho = W.un * mtb;
+    Wtb.p = hk * Qb;
+    Wtb.un = fma(hm, Fb.p, fma(W.p, he, fma(W.un, etb, W.rho * mtb)));
+    Wtb.ut = fma(hm, Fb.ut, W.ut * etb);
+    Wtb.e = etb;
+}
+
+// Reverse of a fan that lies on one side: the interface state is the face
+// state of side S.
+__device__ __forceinline__ void one_sided_adjoint(const Side &S, SideAdjoint &b, A igm1, A hk, const Cell<A> &Fb)
+{
+    const A ir = rrcp(S.r), iri = ir * igm1, tp = S.p * ir, X = fma(-tp, S.rx, S.px), ex = X * iri, cs = S.c * S.s;
+    const Cell5 W = {S.r, S.p, S.u, S.v, S.p * iri};
+    const Cell5 Wt = {-fma(S.r, S.ux, S.u * S.rx), -fma(S.u, S.px, cs * S.ux), -fma(S.u, S.ux, S.px * ir),
+                      -(S.u * S.vx), -fma(S.u, ex, tp * S.ux)};
+    Cell5 Wb, Wtb;
+    flux_adjoint(W, Wt, hk, Fb, Wb, Wtb);
+    const A tr = -Wtb.rho, tn = -Wtb.un, te = -Wtb.e, tv = -Wtb.ut, tq = -Wtb.p;
+    const A exb = S.u * te, Xb = iri * exb, tpb = fma(S.ux, te, -(S.rx * Xb)), irib = fma(S.p, Wb.e, X * exb);
+    const A irb = fma(S.px, tn, fma(S.p, tpb, igm1 * irib));
+    b.r = fma(S.ux, tr, Wb.rho) - ir * ir * irb;
+    b.p = fma(iri, Wb.e, fma(ir, tpb, Wb.p));
+    b.u = fma(S.rx, tr, fma(S.ux, tn, fma(ex, te, fma(S.vx, tv, fma(S.px, tq, Wb.un)))));
+    b.v = Wb.ut;
+    b.rx = fma(S.u, tr, -(tp * Xb));
+    b.px = fma(ir, tn, fma(S.u, tq, Xb));
+    b.ux = fma(S.r, tr, fma(S.u, tn, fma(tp, te, cs * tq)));
+    b.vx = S.u * tv;
+    const A uq = S.ux * tq;
+    b.c = S.s * uq;
+    b.s = S.c * uq;
+}
+
+// Reverse of the star region, on the contact's side S (SG = 1: right, -1:
+// left; O the other side).  Forward, as Hoisted::grp has it:
+//   z = 1 / (SG (u_s - u) + s_s), rho = c_s z, w = u z, h = 1 + SG w, q = rho / rho_s,
+//   Sx = s_s^2 rho_sx - SG c_s u_sx + 3/2 (u - u_s) c_sx, rho_t = -z (z h nD + w q Sx),
+//   P = b_o h, N = c_o - SG u rho, p_t = -isum (c_s P + b_s N),
+//   H = 1 - SG w c_o ic_s, un_t = SG isum (b_s H - P),
+//   E2 = (pm^2 - p_s^2) ic_s^2, e = p_s iri + E2 / 2, iri = igm1 / rho_s,
+//   G = (p_sx - p_s rho_sx / rho_s) iri - ic_s (E2 c_sx + ic_s p_s p_sx),
+//   e_t = pm ic_s^2 p_t - u q G, ut_t = -u q v_sx.
+// Adds the adjoints of the sides' quantities; ub, pmb, nDb, bsb and bob
+// receive those of u, pm, nD, b_s and b_o, and xb un_t un_tb + p_t p_tb,
+// their part of isum's.
+template <int SG>
+__device__ __forceinline__ void star_adjoint(const Side &S, const Side &O, SideAdjoint &Sb, SideAdjoint &Ob, A u, A pm,
+                                             A nD, A b_s, A b_o, A isum, A igm1, A hk, const Cell<A> &Fb, A &ub,
+                                             A &pmb, A &nDb, A &bsb, A &bob, A &xb)
+{
+    const A one = A(1), half = A(0.5), sg = A(SG);
+    const A z = rrcp(SG > 0 ? (S.u - u) + S.s : (u - S.u) + S.s);
+    const A rho = S.c * z, w = u * z, h = fma(sg, w, one), irs = rrcp(S.r), q = rho * irs;
+    const A du15 = A(1.5) * (u - S.u), ss = S.s * S.s;
+    const A Sx = fma(ss, S.rx, fma(-sg * S.c, S.ux, du15 * S.cx));
+    const A zh = z * h, wq = w * q, Kz = fma(zh, nD, wq * Sx);
+    const A P = b_o * h, N = fma(-sg * u, rho, O.c), wc = w * O.c, H = fma(-sg * wc, S.ic, one);
+    const A ic2 = S.ic * S.ic, dE = (pm - S.p) * (pm + S.p), E2 = dE * ic2;
+    const A iri = irs * igm1, tp = S.p * irs, X = fma(-tp, S.rx, S.px), ppx = S.p * S.px;
+    const A Y = fma(E2, S.cx, S.ic * ppx), G = fma(-S.ic, Y, X * iri), uq = u * q, pmi = pm * ic2;
+    Cell5 W = {rho, pm, u, S.v, fma(half, E2, S.p * iri)}, Wt;
+    Wt.rho = -(z * Kz);
+    Wt.p = -(isum * fma(S.c, P, b_s * N));
+    Wt.un = sg * isum * fma(b_s, H, -P);
+    Wt.e = fma(pmi, Wt.p, -(uq * G));
+    Wt.ut = -(uq * S.vx);
+    Cell5 Wb, Wtb;
+    flux_adjoint(W, Wt, hk, Fb, Wb, Wtb);
+    // ut_t, e_t, e
+    Sb.v = Wb.ut;
+    Sb.vx = -(uq * Wtb.ut);
+    const A uqb = -fma(S.vx, Wtb.ut, G * Wtb.e), Gb = -(uq * Wtb.e), pe = Wt.p * Wtb.e;
+    pmb = fma(ic2, pe, Wb.p);
+    const A ptb = fma(pmi, Wtb.e, Wtb.p);
+    // G: X, Y
+    const A Xb = iri * Gb, Yb = -(S.ic * Gb), m = S.ic * Yb, tpb = -(S.rx * Xb);
+    const A E2b = fma(S.cx, Yb, half * Wb.e), f = (ic2 + ic2) * E2b;
+    pmb = fma(pm, f, pmb);
+    Sb.p = fma(iri, Wb.e, fma(S.px, m, fma(irs, tpb, -(S.p * f))));
+    Sb.px = fma(S.p, m, Xb);
+    Sb.cx = E2 * Yb;
+    A icb = fma(ppx, Yb, -(Y * Gb));
+    icb = fma(S.ic + S.ic, fma(dE, E2b, pm * pe), icb);  // ic2 = ic^2
+    A irb = fma(S.p, tpb, igm1 * fma(S.p, Wb.e, X * Gb));
+    // un_t
+    const A j1 = sg * isum * Wtb.un, t1 = -(sg * b_s) * j1;
+    A wb = O.c * S.ic * t1;
+    icb = fma(wc, t1, icb);
+    // p_t
+    const A j2 = -(isum * ptb), Nb = b_s * j2, Pb = fma(S.c, j2, -j1);
+    bsb = fma(H, j1, N * j2);
+    Ob.c = fma(w * S.ic, t1, Nb);
+    xb = fma(Wt.un, Wtb.un, Wt.p * ptb);
+    bob = h * Pb;
+    A rhob = fma(-sg * u, Nb, Wb.rho);
+    // rho_t
+    const A j3 = -(z * Wtb.rho), zhb = nD * j3, wqb = Sx * j3, Sxb = wq * j3;
+    nDb = zh * j3;
+    const A hb = fma(z, zhb, b_o * Pb), qb = fma(w, wqb, u * uqb);
+    wb = fma(q, wqb, fma(sg, hb, wb));
+    Sb.rx = fma(ss, Sxb, -(tp * Xb));
+    Sb.ux = -(sg * S.c) * Sxb;
+    Sb.cx = fma(du15, Sxb, Sb.cx);
+    const A m5 = A(1.5) * S.cx * Sxb;
+    rhob = fma(irs, qb, rhob);
+    irb = fma(rho, qb, irb);
+    // z, and through it rho, w, h
+    const A zb = fma(h, zhb, fma(u, wb, fma(S.c, rhob, -(Kz * Wtb.rho)))), d = -(z * z) * zb;
+    ub = fma(-sg * rho, Nb, fma(q, uqb, fma(z, wb, fma(-sg, d, Wb.un + m5))));
+    Sb.u = fma(sg, d, -m5);
+    Sb.s = fma(A(2) * S.s * S.rx, Sxb, d);
+    Sb.c = fma(P, j2, fma(-sg * S.ux, Sxb, z * rhob));
+    Sb.r = -(irs * irs) * irb;
+    Sb.ic = icb;
+}
+
+// Reverse of the relaxation speeds: of the two sides the one computed first
+// (from the other's i) and second (from the first's 1/c), e = the pressure
+// rise from first to second.  zf, zs: the arguments of max(0, .).
+__device__ __forceinline__ void speeds_adjoint(const Side &f, const Side &s, SideAdjoint &fb, SideAdjoint &sb, A e,
+                                               A kappa, A zf, A zs, A &eb, A &dub)
+{
+    sb.c = fma(-(s.ic * s.ic), sb.ic, sb.c);
+    sb.r = fma(s.s, sb.c, sb.r);
+    sb.s = fma(s.r, sb.c, sb.s);
+    const A ts = zs > A(0) ? kappa * sb.s : A(0);
+    fb.ic = fma(-e, ts, fb.ic);
+    fb.c = fma(-(f.ic * f.ic), fb.ic, fb.c);
+    fb.r = fma(f.s, fb.c, fb.r);
+    fb.s = fma(f.r, fb.c, fb.s);
+    const A tf = zf > A(0) ? kappa * fb.s : A(0);
+    sb.i = e * tf;
+    fb.i = A(0);
+    eb = fma(s.i, tf, -(f.ic * ts));
+    dub += ts + tf;
+}
+
+// Reverse of a side's sound speed a = gp i (adjoint s), of cx and of
+// i = 1/sqrt(gp rho), gp = gamma p.
+__device__ __forceinline__ void sound_adjoint(const Side &S, SideAdjoint &b, A g)
+{
+    const A hg = A(0.5) * g, t = hg * S.i * b.cx;
+    const A ib = fma(hg * S.Y, b.cx, fma(S.gp, b.s, b.i));
+    const A yb = A(-0.5) * (S.i * S.i) * (S.i * ib);
+    b.p = fma(S.rx, t, fma(g, fma(S.i, b.s, S.r * yb), b.p));
+    b.r = fma(S.px, t, fma(S.gp, yb, b.r));
+    b.rx = fma(S.p, t, b.rx);
+    b.px = fma(S.r, t, b.px);
+}
+
 // Adjoint of Hoisted::interface_flux(UL, UR, sL, sR): given the flux adjoint
 // Fb (slots mass, normal momentum, energy, tangential momentum), adds the
-// adjoints of the two cells and the two slopes.
+// adjoints of the two cells and the two slopes.  The forward is recomputed
+// with Hoisted::grp's grouping, and the reverse follows it.
 __device__ __forceinline__ void interface_flux_adjoint(const Cell<A> &UL, const Cell<A> &UR, const Cell<A> &sL,
                                                        const Cell<A> &sR, const SweepConsts<A> &K, const Cell<A> &Fb,
                                                        Cell<A> &ULb, Cell<A> &URb, Cell<A> &sLb, Cell<A> &sRb)
 {
-    const A one = A(1), half = A(0.5), zero = A(0), two = A(2), onehalf = A(1.5);
-    const A g = K.g, igm1 = K.igm1, kappa = K.kappa, hk = K.k * half, hh = K.h * half;
-    // ---- forward: face states ----
-    const A rho_l = fma(sL.rho, hh, UL.rho), pi_l = fma(sL.p, hh, UL.p);
-    const A u_l = fma(sL.un, hh, UL.un), v_l = fma(sL.ut, hh, UL.ut);
-    const A rho_r = fma(-sR.rho, hh, UR.rho), pi_r = fma(-sR.p, hh, UR.p);
-    const A u_r = fma(-sR.un, hh, UR.un), v_r = fma(-sR.ut, hh, UR.ut);
-    const A rho_lx = sL.rho, pi_lx = sL.p, u_lx = sL.un, v_lx = sL.ut;
-    const A rho_rx = sR.rho, pi_rx = sR.p, u_rx = sR.un, v_rx = sR.ut;
-    // ---- forward: Hoisted::grp, its reciprocals formed as it forms them
-    // (the reverse below uses only what they are: irl = 1/rho_l,
-    // il = 1/(rho_l a_l), a_l = sqrt(g pi_l / rho_l), icl = 1/c_l,
-    // isum = 1/(c_l + c_r), and the same on the right) ----
-    const A irlr = rrcp(rho_l * rho_r);
-    const A irl = rho_r * irlr, irr = rho_l * irlr;
-    const A e_l = pi_l * irl * igm1, e_r = pi_r * irr * igm1;
-    const A X_l = pi_lx - pi_l * rho_lx * irl, X_r = pi_rx - pi_r * rho_rx * irr;
-    const A e_lx = X_l * irl * igm1, e_rx = X_r * irr * igm1;
-    const A il = rrsqrt(g * pi_l * rho_l), ir = rrsqrt(g * pi_r * rho_r);
-    const A a_l = g * pi_l * il, a_r = g * pi_r * ir;
-    const A Y_l = pi_l * rho_lx + rho_l * pi_lx, Y_r = pi_r * rho_rx + rho_r * pi_rx;
-    const A c_lx = half * g * Y_l * il, c_rx = half * g * Y_r * ir;
-    const A du = u_l - u_r;
-    const bool right_first = pi_r >= pi_l;
-    A zl_arg, zr_arg, c_l, c_r, icl, icr, isum;
-    if (right_first) {
-        zl_arg = (pi_r - pi_l) * ir + du;
-        c_l = rho_l * (a_l + kappa * rmax(zero, zl_arg));
-        icl = rrcp(c_l);
-        zr_arg = (pi_l - pi_r) * icl + du;
-        c_r = rho_r * (a_r + kappa * rmax(zero, zr_arg));
-        const A sc = c_l + c_r, q = rrcp(c_r * sc);
-        icr = sc * q;
-        isum = c_r * q;
+    const A half = A(0.5), zero = A(0);
+    const A g = K.g, igm1 = K.igm1, kappa = K.kappa, hk = K.k * half, hh = K.h * half, hg = half * g;
+    Side l, r;
+    l.r = fma(sL.rho, hh, UL.rho), l.p = fma(sL.p, hh, UL.p), l.u = fma(sL.un, hh, UL.un), l.v = fma(sL.ut, hh, UL.ut);
+    r.r = fma(-sR.rho, hh, UR.rho), r.p = fma(-sR.p, hh, UR.p), r.u = fma(-sR.un, hh, UR.un);
+    r.v = fma(-sR.ut, hh, UR.ut);
+    l.rx = sL.rho, l.px = sL.p, l.ux = sL.un, l.vx = sL.ut;
+    r.rx = sR.rho, r.px = sR.p, r.ux = sR.un, r.vx = sR.ut;
+    l.gp = g * l.p, r.gp = g * r.p;
+    l.i = rrsqrt(l.gp * l.r), r.i = rrsqrt(r.gp * r.r);
+    l.Y = fma(l.p, l.rx, l.r * l.px), r.Y = fma(r.p, r.rx, r.r * r.px);
+    l.cx = l.Y * (hg * l.i), r.cx = r.Y * (hg * r.i);
+    const A du = l.u - r.u, dp = r.p - l.p;
+    const bool left_first = r.p >= l.p;
+    A zl, zr, isum;
+    if (left_first) {
+        zl = fma(dp, r.i, du);
+        l.s = fma(kappa, rmax(zero, zl), l.gp * l.i);
+        l.c = l.r * l.s;
+        l.ic = rrcp(l.c);
+        zr = fma(-dp, l.ic, du);
+        r.s = fma(kappa, rmax(zero, zr), r.gp * r.i);
+        r.c = r.r * r.s;
+        const A sc = l.c + r.c, q = rrcp(r.c * sc);
+        r.ic = sc * q;
+        isum = r.c * q;
     } else {
-        zr_arg = (pi_l - pi_r) * il + du;
-        c_r = rho_r * (a_r + kappa * rmax(zero, zr_arg));
-        icr = rrcp(c_r);
-        zl_arg = (pi_r - pi_l) * icr + du;
-        c_l = rho_l * (a_l + kappa * rmax(zero, zl_arg));
-        const A sc = c_l + c_r, q = rrcp(c_l * sc);
-        icl = sc * q;
-        isum = c_l * q;
+        zr = fma(-dp, l.i, du);
+        r.s = fma(kappa, rmax(zero, zr), r.gp * r.i);
+        r.c = r.r * r.s;
+        r.ic = rrcp(r.c);
+        zl = fma(dp, r.ic, du);
+        l.s = fma(kappa, rmax(zero, zl), l.gp * l.i);
+        l.c = l.r * l.s;
+        const A sc = l.c + r.c, q = rrcp(l.c * sc);
+        l.ic = sc * q;
+        isum = l.c * q;
     }
-    const A zl = rmax(zero, zl_arg), zr = rmax(zero, zr_arg);
-    const A sl = c_l * irl, sr = c_r * irr;
-    const int wave = (u_l - sl >= zero) ? 0 : ((u_r + sr <= zero) ? 1 : 2);  // left, right, star
-    Cell5 W, Wt;
-    // star-region intermediates (used only when wave == 2)
-    A u = 0, pm = 0, k_l = 0, k_r = 0, H = 0, G = 0, d_l = 0, d_r = 0, Dp = 0;
-    A irho = 0, rho = 0, ic2 = 0, rho3 = 0, urho = 0, A1 = 0, B1 = 0, C1 = 0, P = 0, V = 0, Q = 0, T1 = 0, T2 = 0;
-    bool star_right = false;
-    if (wave == 0) {
-        W = {rho_l, pi_l, u_l, v_l, e_l};
-        Wt.rho = -rho_l * u_lx - u_l * rho_lx;
-        Wt.un = -u_l * u_lx - pi_lx * irl;
-        Wt.e = -u_l * e_lx - pi_l * irl * u_lx;
-        Wt.ut = -u_l * v_lx;
-        Wt.p = -u_l * pi_lx - c_l * sl * u_lx;
-    } else if (wave == 1) {
-        W = {rho_r, pi_r, u_r, v_r, e_r};
-        Wt.rho = -rho_r * u_rx - u_r * rho_rx;
-        Wt.un = -u_r * u_rx - pi_rx * irr;
-        Wt.e = -u_r * e_rx - pi_r * irr * u_rx;
-        Wt.ut = -u_r * v_rx;
-        Wt.p = -u_r * pi_rx - c_r * sr * u_rx;
+    SideAdjoint lb, rb;
+    A dub = zero, dpb = zero;
+    if (l.u - l.s >= zero) {
+        one_sided_adjoint(l, lb, igm1, hk, Fb);
+    } else if (r.u + r.s <= zero) {
+        one_sided_adjoint(r, rb, igm1, hk, Fb);
     } else {
-        u = (u_l * c_l + u_r * c_r + pi_l - pi_r) * isum;
-        pm = (du * c_l * c_r + c_l * pi_r + c_r * pi_l) * isum;
-        k_l = -pi_lx - c_l * u_lx - half * u_l * c_lx;
-        k_r = -pi_rx + c_r * u_rx + half * u_r * c_rx;
-        H = A(-2) * (c_l * u_lx + pi_lx) - u_l * c_lx;
-        G = two * (c_r * u_rx - pi_rx) + u_r * c_rx;
-        d_l = sl * H;
-        d_r = sr * G;
-        Dp = (c_r * d_l - c_l * d_r) * half * isum;
-        star_right = u <= zero;
-        if (star_right) {
-            irho = (u_r - u + sr) * icr;
-            rho = rrcp(irho);
-            ic2 = icr * icr;
-            const A e = e_r + (pm - pi_r) * (pm + pi_r) * half * ic2;
-            rho3 = rho * rho * rho;
-            urho = u * rho;
-            P = sr * sr * rho_rx - c_r * u_rx + onehalf * (u - u_r) * c_rx;
-            V = u + c_r * irho;
-            T1 = rho3 * irr * ic2;
-            T2 = rho3 * ic2 * icr;
-            A1 = one + urho * icr;
-            B1 = one - urho * c_l * ic2;
-            C1 = one - urho * icl;
-            Q = e_rx - pi_r * pi_rx * ic2 + two * (e_r - e) * c_rx * icr;
-            W = {rho, pm, u, v_r, e};
-            Wt.rho = -u * T1 * P + T2 * V * Dp;
-            Wt.p = isum * (c_r * sl * A1 * k_l - c_l * sr * C1 * k_r);
-            Wt.un = isum * (sl * A1 * k_l + sr * B1 * k_r);
-            Wt.e = -urho * irr * Q + pm * ic2 * Wt.p;
-            Wt.ut = -urho * irr * v_rx;
-        } else {
-            irho = (u - u_l + sl) * icl;
-            rho = rrcp(irho);
-            ic2 = icl * icl;
-            const A e = e_l + (pm - pi_l) * (pm + pi_l) * half * ic2;
-            rho3 = rho * rho * rho;
-            urho = u * rho;
-            P = sl * sl * rho_lx + c_l * u_lx + onehalf * (u - u_l) * c_lx;
-            V = u - c_l * irho;
-            T1 = rho3 * irl * ic2;
-            T2 = rho3 * ic2 * icl;
-            A1 = one + urho * icr;
-            B1 = one + urho * c_r * ic2;  // the left case's factor of k_l in un_t
-            C1 = one - urho * icl;
-            Q = e_lx - pi_l * pi_lx * ic2 + two * (e_l - e) * c_lx * icl;
-            W = {rho, pm, u, v_l, e};
-            Wt.rho = -u * T1 * P - T2 * V * Dp;
-            Wt.p = isum * (c_r * sl * A1 * k_l - c_l * sr * C1 * k_r);
-            Wt.un = isum * (sl * B1 * k_l + sr * C1 * k_r);
-            Wt.e = -urho * irl * Q + pm * ic2 * Wt.p;
-            Wt.ut = -urho * irl * v_lx;
-        }
+        const A u = (fma(l.u, l.c, r.u * r.c) - dp) * isum;
+        const A pm = fma(du * l.c, r.c, fma(l.c, r.p, r.c * l.p)) * isum;
+        const A Bl = fma(half * l.u, l.cx, fma(l.c, l.ux, l.px)), Br = fma(half * r.u, r.cx, fma(r.c, r.ux, -r.px));
+        const A b_l = l.s * Bl, b_r = r.s * Br, nD = fma(r.c, b_l, l.c * b_r) * isum;
+        A ub, pmb, nDb, blb, brb, xb;
+        if (u <= zero)
+            star_adjoint<1>(r, l, rb, lb, u, pm, nD, b_r, b_l, isum, igm1, hk, Fb, ub, pmb, nDb, brb, blb, xb);
+        else
+            star_adjoint<-1>(l, r, lb, rb, u, pm, nD, b_l, b_r, isum, igm1, hk, Fb, ub, pmb, nDb, blb, brb, xb);
+        // nD, u and pm are brackets times isum = 1/(c_l + c_r), whose adjoint
+        // reaches c_l and c_r as -isum sum(X Xb)
+        const A jD = isum * nDb, ju = isum * ub, jp = isum * pmb;
+        const A jc = -(isum * fma(u, ub, fma(pm, pmb, fma(nD, nDb, xb))));
+        blb = fma(r.c, jD, blb);
+        brb = fma(l.c, jD, brb);
+        const A tl = l.s * blb, tr = r.s * brb;
+        lb.c += fma(b_r, jD, fma(l.u, ju, fma(fma(du, r.c, r.p), jp, fma(l.ux, tl, jc))));
+        rb.c += fma(b_l, jD, fma(r.u, ju, fma(fma(du, l.c, l.p), jp, fma(r.ux, tr, jc))));
+        lb.p += r.c * jp;
+        rb.p += l.c * jp;
+        dub = l.c * r.c * jp;
+        dpb = -ju;
+        // b = s B
+        lb.s = fma(Bl, blb, lb.s);
+        rb.s = fma(Br, brb, rb.s);
+        lb.u += fma(l.c, ju, half * l.cx * tl);
+        rb.u += fma(r.c, ju, half * r.cx * tr);
+        lb.cx = fma(half * l.u, tl, lb.cx);
+        rb.cx = fma(half * r.u, tr, rb.cx);
+        lb.ux = fma(l.c, tl, lb.ux);
+        rb.ux = fma(r.c, tr, rb.ux);
+        lb.px += tl;
+        rb.px -= tr;
     }
-    // ---- reverse: midpoint flux ----
-    // F.rho = m + hk mt; F.p = m un + p + hk (mt un + m un_t + p_t);
-    // F.un (energy) = m es + p un + hk (mt es + m q + p_t un + p un_t);
-    // F.ut = m ut + hk (mt ut + m ut_t), with m = rho un, mt = rho un_t + un rho_t,
-    // es = e + (un^2 + ut^2)/2, q = e_t + un un_t + ut ut_t
-    Cell5 Wb, Wtb;
-    {
-        const A m = W.rho * W.un, mt = W.rho * Wt.un + W.un * Wt.rho;
-        const A es = W.e + half * (W.un * W.un + W.ut * W.ut);
-        const A q = Wt.e + W.un * Wt.un + W.ut * Wt.ut;
-        const A hr = hk * Fb.rho, hp = hk * Fb.p, he = hk * Fb.un, hu = hk * Fb.ut;
-        const A mb = Fb.rho + W.un * Fb.p + Wt.un * hp + es * Fb.un + q * he + W.ut * Fb.ut + Wt.ut * hu;
-        const A mtb = hr + W.un * hp + es * he + W.ut * hu;
-        const A esb = m * Fb.un + mt * he, qb = m * he;
-        Wb.rho = Wt.un * mtb + W.un * mb;
-        Wb.p = Fb.p + W.un * Fb.un + Wt.un * he;
-        Wb.un = m * Fb.p + mt * hp + W.p * Fb.un + Wt.p * he + Wt.un * qb + W.un * esb + Wt.rho * mtb + W.rho * mb;
-        Wb.ut = m * Fb.ut + mt * hu + Wt.ut * qb + W.ut * esb;
-        Wb.e = esb;
-        Wtb.rho = W.un * mtb;
-        Wtb.p = hp + W.un * he;
-        Wtb.un = m * hp + W.p * he + W.un * qb + W.rho * mtb;
-        Wtb.ut = m * hu + W.ut * qb;
-        Wtb.e = qb;
-    }
-    // ---- reverse: Hoisted::grp ----
-    A rho_lb = 0, pi_lb = 0, u_lb = 0, v_lb = 0, rho_rb = 0, pi_rb = 0, u_rb = 0, v_rb = 0;
-    A rho_lxb = 0, pi_lxb = 0, u_lxb = 0, v_lxb = 0, rho_rxb = 0, pi_rxb = 0, u_rxb = 0, v_rxb = 0;
-    A irlb = 0, irrb = 0, e_lb = 0, e_rb = 0, e_lxb = 0, e_rxb = 0, c_lxb = 0, c_rxb = 0;
-    A c_lb = 0, c_rb = 0, iclb = 0, icrb = 0, slb = 0, srb = 0, dub = 0;
-    if (wave == 0) {
-        // W = left face state; Wt: rho_t = -rho_l u_lx - u_l rho_lx, un_t = -u_l u_lx - pi_lx irl,
-        // e_t = -u_l e_lx - pi_l irl u_lx, ut_t = -u_l v_lx, p_t = -u_l pi_lx - c_l sl u_lx
-        const A tp = -Wtb.p, te = -Wtb.e, tn = -Wtb.un, tr = -Wtb.rho;
-        rho_lb += Wb.rho + u_lx * tr;
-        pi_lb += Wb.p + irl * u_lx * te;
-        u_lb += Wb.un + pi_lx * tp - v_lx * Wtb.ut + e_lx * te + u_lx * tn + rho_lx * tr;
-        v_lb += Wb.ut;
-        e_lb += Wb.e;
-        pi_lxb += u_l * tp + irl * tn;
-        c_lb += sl * u_lx * tp;
-        slb += c_l * u_lx * tp;
-        u_lxb += c_l * sl * tp + pi_l * irl * te + u_l * tn + rho_l * tr;
-        v_lxb += -u_l * Wtb.ut;
-        e_lxb += u_l * te;
-        irlb += pi_l * u_lx * te + pi_lx * tn;
-        rho_lxb += u_l * tr;
-    } else if (wave == 1) {
-        const A tp = -Wtb.p, te = -Wtb.e, tn = -Wtb.un, tr = -Wtb.rho;
-        rho_rb += Wb.rho + u_rx * tr;
-        pi_rb += Wb.p + irr * u_rx * te;
-        u_rb += Wb.un + pi_rx * tp - v_rx * Wtb.ut + e_rx * te + u_rx * tn + rho_rx * tr;
-        v_rb += Wb.ut;
-        e_rb += Wb.e;
-        pi_rxb += u_r * tp + irr * tn;
-        c_rb += sr * u_rx * tp;
-        srb += c_r * u_rx * tp;
-        u_rxb += c_r * sr * tp + pi_r * irr * te + u_r * tn + rho_r * tr;
-        v_rxb += -u_r * Wtb.ut;
-        e_rxb += u_r * te;
-        irrb += pi_r * u_rx * te + pi_rx * tn;
-        rho_rxb += u_r * tr;
+    A eb;
+    if (left_first) {
+        speeds_adjoint(l, r, lb, rb, dp, kappa, zl, zr, eb, dub);
+        dpb += eb;
     } else {
-        // The star state's side s (right if u <= 0, else left), written once for
-        // both sides with sg = +1 (right) or -1 (left):
-        //   irho = (sg (u_s - u) + s_s) ic_s, rho = 1/irho, ic2 = ic_s^2,
-        //   e = e_s + (pm^2 - pi_s^2)/2 ic2, rho3 = rho^3, urho = u rho,
-        //   P = s_s^2 rho_sx - sg c_s u_sx + 1.5 (u - u_s) c_sx, V = u + sg c_s irho,
-        //   T1 = rho3 ir_s ic2, T2 = rho3 ic2 ic_s, Q = e_sx - pi_s pi_sx ic2 + 2 (e_s - e) c_sx ic_s,
-        //   rho_t = -u T1 P + sg T2 V Dp, e_t = -urho ir_s Q + pm ic2 p_t, ut_t = -urho ir_s v_sx,
-        //   p_t = isum (c_r sl A1 k_l - c_l sr C1 k_r), A1 = 1 + urho icr, C1 = 1 - urho icl,
-        //   un_t = isum (sl a k_l + sr b k_r), with (a, b) = (A1, B1) on the right and (B1, C1)
-        //   on the left, B1 = 1 - sg urho c_o ic2 (c_o the other side's c).
-        const bool R = star_right;
-        const A sg = R ? one : -one;
-        const A u_s = R ? u_r : u_l, s_s = R ? sr : sl, ic_s = R ? icr : icl, ir_s = R ? irr : irl;
-        const A c_s = R ? c_r : c_l, c_o = R ? c_l : c_r, pi_s = R ? pi_r : pi_l, pi_sx = R ? pi_rx : pi_lx;
-        const A e_s = R ? e_r : e_l, c_sx = R ? c_rx : c_lx, rho_sx = R ? rho_rx : rho_lx;
-        const A u_sx = R ? u_rx : u_lx, v_sx = R ? v_rx : v_lx;
-        A ub = Wb.un, pmb = Wb.p, rhob = Wb.rho, eb = Wb.e, p_tb = Wtb.p, Dpb = 0;
-        A k_lb = 0, k_rb = 0, urhob = 0, ic2b = 0, ir_sb = 0, ic_sb = 0, c_sb = 0, c_ob = 0;
-        A u_sb = 0, s_sb = 0, pi_sb = 0, pi_sxb = 0, e_sb = 0, e_sxb = 0, c_sxb = 0, rho_sxb = 0, u_sxb = 0;
-        const A v_sxb = -urho * ir_s * Wtb.ut;
-        // ut_t and e_t
-        const A tt = -(v_sx * Wtb.ut + Q * Wtb.e);
-        urhob += ir_s * tt;
-        ir_sb += urho * tt;
-        const A Qb = -urho * ir_s * Wtb.e;
-        const A cpe = Wt.p * Wtb.e;
-        pmb += ic2 * cpe;
-        ic2b += pm * cpe;
-        p_tb += pm * ic2 * Wtb.e;
-        // Q
-        e_sxb += Qb;
-        const A dq = -ic2 * Qb;
-        pi_sb += pi_sx * dq;
-        pi_sxb += pi_s * dq;
-        ic2b += -pi_s * pi_sx * Qb;
-        const A fq = two * c_sx * ic_s * Qb;
-        e_sb += fq;
-        eb -= fq;
-        const A gq = two * (e_s - W.e) * Qb;
-        c_sxb += ic_s * gq;
-        ic_sb += c_sx * gq;
-        // un_t
-        const A iu = isum * Wtb.un;
-        const A a = R ? A1 : B1, b = R ? B1 : C1;
-        slb += a * k_l * iu;
-        k_lb += sl * a * iu;
-        srb += b * k_r * iu;
-        k_rb += sr * b * iu;
-        const A ab = sl * k_l * iu, bb = sr * k_r * iu;
-        A A1b = R ? ab : A(0), C1b = R ? A(0) : bb;
-        const A B1b = R ? bb : ab;
-        const A hb = -sg * B1b;  // B1 = 1 - sg urho c_o ic2
-        urhob += c_o * ic2 * hb;
-        c_ob += urho * ic2 * hb;
-        ic2b += urho * c_o * hb;
-        // p_t
-        const A ip = isum * p_tb;
-        const A LL = c_r * sl, L2 = A1 * k_l, RR = c_l * sr, R2 = C1 * k_r;
-        const A x1 = ip * L2, x2 = ip * LL, x3 = -ip * R2, x4 = -ip * RR;
-        c_rb += sl * x1;
-        slb += c_r * x1;
-        A1b += k_l * x2;
-        k_lb += A1 * x2;
-        c_lb += sr * x3;
-        srb += c_l * x3;
-        C1b += k_r * x4;
-        k_rb += C1 * x4;
-        urhob += icr * A1b - icl * C1b;
-        icrb += urho * A1b;
-        iclb -= urho * C1b;
-        // rho_t
-        const A y1 = -Wtb.rho * T1, y2 = sg * Wtb.rho * T2;
-        ub += P * y1;
-        const A Pb = u * y1, Vb = Dp * y2;
-        Dpb += V * y2;
-        const A T1b = -u * P * Wtb.rho, T2b = sg * V * Dp * Wtb.rho;
-        const A zt = ir_s * T1b + ic_s * T2b, w = rho3 * ic2;
-        A rho3b = ic2 * zt;
-        ic2b += rho3 * zt;
-        ir_sb += w * T1b;
-        ic_sb += w * T2b;
-        // P
-        s_sb += two * s_s * rho_sx * Pb;
-        rho_sxb += s_s * s_s * Pb;
-        c_sb += -sg * u_sx * Pb;
-        u_sxb += -sg * c_s * Pb;
-        const A kp = onehalf * c_sx * Pb;
-        ub += kp;
-        u_sb -= kp;
-        c_sxb += onehalf * (u - u_s) * Pb;
-        // V
-        ub += Vb;
-        c_sb += sg * irho * Vb;
-        A irhob = sg * c_s * Vb;
-        // urho, rho3
-        ub += rho * urhob;
-        rhob += u * urhob + A(3) * rho * rho * rho3b;
-        // e, ic2
-        e_sb += eb;
-        pmb += pm * ic2 * eb;
-        pi_sb -= pi_s * ic2 * eb;
-        ic2b += half * (pm * pm - pi_s * pi_s) * eb;
-        ic_sb += two * ic_s * ic2b;
-        // rho = 1/irho, irho = (sg (u_s - u) + s_s) ic_s
-        irhob -= rho * rho * rhob;
-        const A vi = ic_s * irhob;
-        u_sb += sg * vi;
-        ub -= sg * vi;
-        s_sb += vi;
-        ic_sb += (sg * (u_s - u) + s_s) * irhob;
-        // back to the two sides
-        if (R) {
-            v_rb += Wb.ut; v_rxb += v_sxb; u_rb += u_sb; srb += s_sb; icrb += ic_sb; irrb += ir_sb;
-            c_rb += c_sb; c_lb += c_ob; pi_rb += pi_sb; pi_rxb += pi_sxb; e_rb += e_sb; e_rxb += e_sxb;
-            c_rxb += c_sxb; rho_rxb += rho_sxb; u_rxb += u_sxb;
-        } else {
-            v_lb += Wb.ut; v_lxb += v_sxb; u_lb += u_sb; slb += s_sb; iclb += ic_sb; irlb += ir_sb;
-            c_lb += c_sb; c_rb += c_ob; pi_lb += pi_sb; pi_lxb += pi_sxb; e_lb += e_sb; e_lxb += e_sxb;
-            c_lxb += c_sxb; rho_lxb += rho_sxb; u_lxb += u_sxb;
-        }
-        // Dp = (c_r d_l - c_l d_r) isum / 2
-        const A hD = half * isum * Dpb;
-        c_rb += d_l * hD;
-        c_lb -= d_r * hD;
-        const A d_lb = c_r * hD, d_rb = -c_l * hD;
-        // d_r = sr G ; G = 2 (c_r u_rx - pi_rx) + u_r c_rx
-        srb += G * d_rb;
-        const A Gb = sr * d_rb;
-        c_rb += two * u_rx * Gb;
-        u_rxb += two * c_r * Gb;
-        pi_rxb -= two * Gb;
-        u_rb += c_rx * Gb;
-        c_rxb += u_r * Gb;
-        // d_l = sl H ; H = -2 (c_l u_lx + pi_lx) - u_l c_lx
-        slb += H * d_lb;
-        const A Hb = sl * d_lb;
-        c_lb -= two * u_lx * Hb;
-        u_lxb -= two * c_l * Hb;
-        pi_lxb -= two * Hb;
-        u_lb -= c_lx * Hb;
-        c_lxb -= u_l * Hb;
-        // k_r = -pi_rx + c_r u_rx + u_r c_rx / 2 ; k_l = -pi_lx - c_l u_lx - u_l c_lx / 2
-        pi_rxb -= k_rb;
-        c_rb += u_rx * k_rb;
-        u_rxb += c_r * k_rb;
-        u_rb += half * c_rx * k_rb;
-        c_rxb += half * u_r * k_rb;
-        pi_lxb -= k_lb;
-        c_lb -= u_lx * k_lb;
-        u_lxb -= c_l * k_lb;
-        u_lb -= half * c_lx * k_lb;
-        c_lxb -= half * u_l * k_lb;
-        // pm = (du c_l c_r + c_l pi_r + c_r pi_l) isum
-        const A ipm = isum * pmb;
-        dub += c_l * c_r * ipm;
-        c_lb += (du * c_r + pi_r) * ipm;
-        c_rb += (du * c_l + pi_l) * ipm;
-        pi_rb += c_l * ipm;
-        pi_lb += c_r * ipm;
-        // u = (u_l c_l + u_r c_r + pi_l - pi_r) isum
-        const A iub = isum * ub;
-        u_lb += c_l * iub;
-        c_lb += u_l * iub;
-        u_rb += c_r * iub;
-        c_rb += u_r * iub;
-        pi_lb += iub;
-        pi_rb -= iub;
-        // isum = 1/(c_l + c_r): each quantity X = bracket isum above gives
-        // bracket * Xb = X (c_l + c_r) Xb to isum's adjoint, and
-        // d isum / d c = -isum^2, so c_l and c_r receive -isum sum(X Xb)
-        const A sb = -isum * (u * ub + pm * pmb + Wt.p * p_tb + Wt.un * Wtb.un + Dp * Dpb);
-        c_lb += sb;
-        c_rb += sb;
+        speeds_adjoint(r, l, rb, lb, -dp, kappa, zr, zl, eb, dub);
+        dpb -= eb;
     }
-    // sl = c_l irl ; sr = c_r irr
-    c_lb += irl * slb;
-    irlb += c_l * slb;
-    c_rb += irr * srb;
-    irrb += c_r * srb;
-    // relaxation speeds (the order of the forward branch, reversed)
-    A a_lb = 0, a_rb = 0, ilb = 0, irb = 0;
-    if (right_first) {
-        c_rb += -icr * icr * icrb;
-        rho_rb += (a_r + kappa * zr) * c_rb;
-        a_rb += rho_r * c_rb;
-        if (zr_arg > zero) {
-            const A zb = rho_r * kappa * c_rb;
-            pi_lb += icl * zb;
-            pi_rb -= icl * zb;
-            iclb += (pi_l - pi_r) * zb;
-            dub += zb;
-        }
-        c_lb += -icl * icl * iclb;
-        rho_lb += (a_l + kappa * zl) * c_lb;
-        a_lb += rho_l * c_lb;
-        if (zl_arg > zero) {
-            const A zb = rho_l * kappa * c_lb;
-            pi_rb += ir * zb;
-            pi_lb -= ir * zb;
-            irb += (pi_r - pi_l) * zb;
-            dub += zb;
-        }
-    } else {
-        c_lb += -icl * icl * iclb;
-        rho_lb += (a_l + kappa * zl) * c_lb;
-        a_lb += rho_l * c_lb;
-        if (zl_arg > zero) {
-            const A zb = rho_l * kappa * c_lb;
-            pi_rb += icr * zb;
-            pi_lb -= icr * zb;
-            icrb += (pi_r - pi_l) * zb;
-            dub += zb;
-        }
-        c_rb += -icr * icr * icrb;
-        rho_rb += (a_r + kappa * zr) * c_rb;
-        a_rb += rho_r * c_rb;
-        if (zr_arg > zero) {
-            const A zb = rho_r * kappa * c_rb;
-            pi_lb += il * zb;
-            pi_rb -= il * zb;
-            ilb += (pi_l - pi_r) * zb;
-            dub += zb;
-        }
-    }
-    // du = u_l - u_r
-    u_lb += dub;
-    u_rb -= dub;
-    // c_lx = g Y_l il / 2 ; Y_l = pi_l rho_lx + rho_l pi_lx  (and the right side)
-    {
-        const A Ylb = half * g * il * c_lxb, Yrb = half * g * ir * c_rxb;
-        ilb += half * g * Y_l * c_lxb;
-        irb += half * g * Y_r * c_rxb;
-        pi_lb += rho_lx * Ylb;
-        rho_lxb += pi_l * Ylb;
-        rho_lb += pi_lx * Ylb;
-        pi_lxb += rho_l * Ylb;
-        pi_rb += rho_rx * Yrb;
-        rho_rxb += pi_r * Yrb;
-        rho_rb += pi_rx * Yrb;
-        pi_rxb += rho_r * Yrb;
-    }
-    // il = 1/(rho_l a_l) ; ir = 1/(rho_r a_r)
-    {
-        const A Dl = -il * il * ilb, Dr = -ir * ir * irb;
-        rho_lb += a_l * Dl;
-        a_lb += rho_l * Dl;
-        rho_rb += a_r * Dr;
-        a_rb += rho_r * Dr;
-    }
-    // a = sqrt(g pi irho); 1/a = rho il
-    {
-        const A al = half * a_lb * rho_l * il, ar = half * a_rb * rho_r * ir;
-        pi_lb += g * irl * al;
-        irlb += g * pi_l * al;
-        pi_rb += g * irr * ar;
-        irrb += g * pi_r * ar;
-    }
-    // e_x = X irho igm1 ; X = pi_x - pi rho_x irho
-    {
-        const A Xlb = irl * igm1 * e_lxb, Xrb = irr * igm1 * e_rxb;
-        irlb += X_l * igm1 * e_lxb;
-        irrb += X_r * igm1 * e_rxb;
-        pi_lxb += Xlb;
-        pi_lb += -rho_lx * irl * Xlb;
-        rho_lxb += -pi_l * irl * Xlb;
-        irlb += -pi_l * rho_lx * Xlb;
-        pi_rxb += Xrb;
-        pi_rb += -rho_rx * irr * Xrb;
-        rho_rxb += -pi_r * irr * Xrb;
-        irrb += -pi_r * rho_rx * Xrb;
-    }
-    // e = pi irho igm1
-    pi_lb += irl * igm1 * e_lb;
-    irlb += pi_l * igm1 * e_lb;
-    pi_rb += irr * igm1 * e_rb;
-    irrb += pi_r * igm1 * e_rb;
-    // irho = 1/rho
-    rho_lb += -irl * irl * irlb;
-    rho_rb += -irr * irr * irrb;
-    // ---- reverse: face states ----
-    ULb.rho += rho_lb;
-    ULb.p += pi_lb;
-    ULb.un += u_lb;
-    ULb.ut += v_lb;
-    URb.rho += rho_rb;
-    URb.p += pi_rb;
-    URb.un += u_rb;
-    URb.ut += v_rb;
-    sLb.rho += rho_lxb + hh * rho_lb;
-    sLb.p += pi_lxb + hh * pi_lb;
-    sLb.un += u_lxb + hh * u_lb;
-    sLb.ut += v_lxb + hh * v_lb;
-    sRb.rho += rho_rxb - hh * rho_rb;
-    sRb.p += pi_rxb - hh * pi_rb;
-    sRb.un += u_rxb - hh * u_rb;
-    sRb.ut += v_rxb - hh * v_rb;
+    sound_adjoint(l, lb, g);
+    sound_adjoint(r, rb, g);
+    lb.u += dub;
+    rb.u -= dub;
+    lb.p -= dpb;
+    rb.p += dpb;
+    // face states
+    ULb.rho += lb.r;
+    ULb.p += lb.p;
+    ULb.un += lb.u;
+    ULb.ut += lb.v;
+    URb.rho += rb.r;
+    URb.p += rb.p;
+    URb.un += rb.u;
+    URb.ut += rb.v;
+    sLb.rho += fma(hh, lb.r, lb.rx);
+    sLb.p += fma(hh, lb.p, lb.px);
+    sLb.un += fma(hh, lb.u, lb.ux);
+    sLb.ut += fma(hh, lb.v, lb.vx);
+    sRb.rho += fma(-hh, rb.r, rb.rx);
+    sRb.p += fma(-hh, rb.p, rb.px);
+    sRb.un += fma(-hh, rb.u, rb.ux);
+    sRb.ut += fma(-hh, rb.v, rb.vx);
 }
 
 } // namespace FVM2D_VARIANT
