@@ -16,23 +16,16 @@ struct AdjointLaunch {
     const void *U;         // input state of the step
     const void *A1, *B1;   // X(U) and Y(U)
     const void *flux[4];   // interface fluxes of the sweeps X(U), Y(U), Y(A1), X(B1)
-    const void *lb_out;    // adjoint of the step's output state
-    void *lb_in;           // result: adjoint of the input state (may not alias lb_out)
-    void *work[4];         // work states (the fourth used with a fork stream)
-    // optional: a second stream and two events of the caller's; branch B's
-    // first sweep transpose then runs on `fork` beside branch A's two, so
-    // the transposes fill each other's tail waves (also inside a graph
-    // capture, as parallel branches)
-    cudaStream_t fork = nullptr;
-    cudaEvent_t fork_ev[2] = {nullptr, nullptr};
+    void *lb[2];           // in: the adjoint of the step's output state, the sum of the two;
+                           // out: the adjoint of its input state, likewise (branch A's and branch B's)
+    void *work[3];         // work states
 };
 
 #define FVM2D_DECLARE_ADJOINT(ns)                                                 \
     namespace ns {                                                                \
-    /* Queries the device once (SM count, occupancy); call before capturing    \
-       adjoint steps into a graph.  adjoint_step calls it too. */               \
-    cudaError_t adjoint_prepare();                                                \
     cudaError_t adjoint_step(const AdjointLaunch &L, cudaStream_t s);            \
+    /* lb[0] += lb[1]: the adjoint as one state, after the last step */          \
+    cudaError_t adjoint_sum(const AdjointLaunch &L, cudaStream_t s);             \
     }
 
 FVM2D_DECLARE_ADJOINT(adj)    // FP64

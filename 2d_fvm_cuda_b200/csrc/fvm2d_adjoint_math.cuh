@@ -45,6 +45,15 @@ __device__ __forceinline__ A slope_with_choice(A m, A c, A p, A hrh, A rha, int 
     return sloped ? copysign(one_sided ? inner : outer, dc) : A(0);
 }
 
+// The adjoints a slope component passes to its right cell (the return value)
+// and left cell (mbar); its own cell gets minus their sum.
+__device__ __forceinline__ A slope_parts(int choice, A sbar, A hrh, A rha, A &mbar)
+{
+    const A x = (choice == 1 ? hrh : rha) * sbar;
+    mbar = choice == 1 || choice == 2 ? -x : A(0);
+    return choice & 1 ? x : A(0);
+}
+
 // Adds the adjoint of one slope component (sbar) to its three cells.
 __device__ __forceinline__ void slope_adjoint(int choice, A sbar, A rh, A alpha, A &mbar, A &cbar, A &pbar)
 {

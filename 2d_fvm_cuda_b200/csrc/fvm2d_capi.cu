@@ -194,10 +194,10 @@ struct fvm2d_solver {
     int ck_count = 0, ck_len = 0, fwd_steps = -1, fwd_precision = -1;
     bool full_tape = false;       // the last fvm2d_forward kept every step's tape
     // the graphs of a full checkpoint segment: its taped recompute into tape
-    // buffer b ([b]), its reverse from tape buffer b starting from adjoint
-    // buffer a ([2 + 2b + a]), and its untaped forward steps ([6], for
-    // fvm2d_forward); built for vjp_len steps and vjp_bufs tape buffers
-    cudaGraphExec_t vjp_graph[7] = {};
+    // buffer b ([b]), its reverse from tape buffer b ([2 + b]), and its untaped
+    // forward steps ([4], for fvm2d_forward); built for vjp_len steps and
+    // vjp_bufs tape buffers
+    cudaGraphExec_t vjp_graph[5] = {};
     int vjp_len = 0, vjp_bufs = 0;
     bool last_taped = false;      // the checkpointed forward taped its last segment (fvm2d_vjp skips its recompute)
     bool vjp_overlap = true;      // fvm2d_set_vjp_overlap: two tape buffers where they fit
@@ -206,9 +206,6 @@ struct fvm2d_solver {
     // buffer b filled, vjp_ev[2 + b] free again, vjp_ev[4] the start
     cudaStream_t aux = nullptr;
     cudaEvent_t vjp_ev[5] = {};
-    // the adjoint step's fork stream and events (AdjointLaunch::fork)
-    cudaStream_t fork = nullptr;
-    cudaEvent_t fork_ev[2] = {};
     std::vector<double> ck_t;     // time at each checkpoint
     double last_ms = 0.0;         // wall time of the last loop (the reference's timer)
     double last_device_ms = 0.0;  // CUDA-event time of the last loop on the stream
@@ -511,12 +508,6 @@ int fvm2d_destroy(fvm2d_solver *s)
     if (s->ev_end) cudaEventDestroy(s->ev_end);
     for (auto &e : s->vjp_ev)
         if (e) cudaEventDestroy(e);
-    for (auto &e : s->fork_ev)
-        if (e) cudaEventDestroy(e);
-    if (s->fork) {
-        cudaStreamSynchronize(s->fork);
-        cudaStreamDestroy(s->fork);
-    }
     if (s->aux) {
         cudaStreamSynchronize(s->aux);
         cudaStreamDestroy(s->aux);
@@ -1282,7 +1273,9 @@ static char *tape_at(const fvm2d_solver *s, int buf, int j, int q, size_t sb)
 static int taped_steps(fvm2d_solver *s, const LaunchConfig &c, int m, int buf, cudaStream_t st)
 {
     const size_t sb = state_bytes_of(s);
-    auto taped_step = is_fp32(s->precision) ? fvm2d::fp32::enqueue_step_taped : fvm2d::fp64::enqueue_step_taped;
+    const bool f32 = is_fp32(s->precision);
+    auto tile_step = f32 ? fvm2d::fp32::enqueue_tile_step_taped : fvm2d::fp64::enqueue_tile_step_taped;
+    auto sweep_step = f32 ? fvm2d::fp32::enqueue_step_taped : fvm2d::fp64::enqueue_step_taped;
     for (int j = 0; j < m; ++j) {
         LaunchConfig cj = c;
         cj.U = tape_at(s, buf, j, 0, sb);
@@ -1292,8 +1285,14 @@ static int taped_steps(fvm2d_solver *s, const LaunchConfig &c, int m, int buf, c
                                tape_at(s, buf, j, 6, sb)};
         void *const out =
             j + 1 < m ? static_cast<void *>(tape_at(s, buf, j + 1, 0, sb)) : static_cast<void *>(s->base);
-        CK(taped_step(cj, st, flux, out));
+        if (s->tiles())
+            CK(tile_step(cj, st, flux, out, j > 0));
+        else
+            CK(sweep_step(cj, st, flux, out));
     }
+    LaunchConfig last = c;
+    last.pair[0] = last.pair[1] = s->base;
+    CK(s->fill_ring(last, st));
     return FVM2D_OK;
 }
 
@@ -1372,9 +1371,9 @@ static int segment_steps(int nsteps, int len, int count, int k)
     return k == 0 ? nsteps - (count - 1) * len : len;
 }
 
-// adjoint workspace: two adjoints, three work states, the saved final state,
-// the fourth work state of the fork stream's branch
-constexpr int kAdjStates = 7;
+// adjoint workspace: the adjoint as two states (its sum is meant), three work
+// states, the saved final state
+constexpr int kAdjStates = 6;
 
 // The adjoint step's launch parameters for this handle; the tape and
 // adjoint pointers are filled per step.
@@ -1394,41 +1393,23 @@ static fvm2d::AdjointLaunch adjoint_launch_of(const fvm2d_solver *s, size_t sb)
     L.alpha = s->alpha;
     L.gamma = s->gamma;
     L.dt = s->fixed_dt;
+    for (int k = 0; k < 2; ++k) L.lb[k] = s->adj + k * sb;
     for (int k = 0; k < 3; ++k) L.work[k] = s->adj + (2 + k) * sb;
-    L.work[3] = s->adj + 6 * sb;
-    L.fork = s->fork;
-    L.fork_ev[0] = s->fork_ev[0];
-    L.fork_ev[1] = s->fork_ev[1];
     return L;
 }
 
-// The adjoint step's fork stream and its events (created once per handle).
-static int ensure_fork(fvm2d_solver *s)
-{
-    if (s->fork) return FVM2D_OK;
-    CK(cudaStreamCreateWithFlags(&s->fork, cudaStreamNonBlocking));
-    for (auto &e : s->fork_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    return FVM2D_OK;
-}
-
-// Enqueues on `st` the reverse of m steps taped in buffer `buf`, starting
-// from adjoint buffer `from` (0 or 1 of the workspace); the result lands in
-// `from` for even m, in the other buffer for odd m.
-static int reverse_steps(fvm2d_solver *s, int m, int buf, int from, cudaStream_t st)
+// Enqueues on `st` the reverse of m steps taped in buffer `buf`.
+static int reverse_steps(fvm2d_solver *s, int m, int buf, cudaStream_t st)
 {
     const size_t sb = state_bytes_of(s);
     auto adjoint_step = is_fp32(s->precision) ? fvm2d::adj32::adjoint_step : fvm2d::adj::adjoint_step;
     fvm2d::AdjointLaunch L = adjoint_launch_of(s, sb);
-    char *a = s->adj + from * sb, *b = s->adj + (1 - from) * sb;
     for (int j = m - 1; j >= 0; --j) {
         L.U = tape_at(s, buf, j, 0, sb);
         L.A1 = tape_at(s, buf, j, 1, sb);
         L.B1 = tape_at(s, buf, j, 2, sb);
         for (int q = 0; q < 4; ++q) L.flux[q] = tape_at(s, buf, j, 3 + q, sb);
-        L.lb_out = a;
-        L.lb_in = b;
         CK(adjoint_step(L, st));
-        std::swap(a, b);
     }
     return FVM2D_OK;
 }
@@ -1459,7 +1440,6 @@ static int vjp_workspace(fvm2d_solver *s, int *bufs)
     if (int rc = ensure(s->adj, s->adj_bytes, kAdjStates * sb, grew_adj)) return rc;
     if (grew_tape || grew_adj) s->drop_vjp_graphs();
     if (grew_tape) s->last_taped = false;
-    if (int rc = ensure_fork(s)) return rc;
     if (*bufs == 2 && !s->aux) {
         // default priority: the recompute fills the SM room the reverse's
         // blocks leave (measured: at the device's higher priority the VJP
@@ -1471,10 +1451,9 @@ static int vjp_workspace(fvm2d_solver *s, int *bufs)
     // buffers stay the same
     if (s->ck_count > 1 && (s->vjp_len != s->ck_len || s->vjp_bufs != *bufs)) {
         s->drop_vjp_graphs();
-        CK(is_fp32(s->precision) ? fvm2d::adj32::adjoint_prepare() : fvm2d::adj::adjoint_prepare());
         const LaunchConfig c = s->config();
         const int len = s->ck_len;
-        if (int rc = s->capture(&s->vjp_graph[6], [&] {
+        if (int rc = s->capture(&s->vjp_graph[4], [&] {
                 for (int j = 0; j < len; ++j) CK(s->enqueue_step(c, s->stream));
                 return FVM2D_OK;
             }))
@@ -1482,9 +1461,7 @@ static int vjp_workspace(fvm2d_solver *s, int *bufs)
         for (int b = 0; b < *bufs; ++b) {
             if (int rc = s->capture(&s->vjp_graph[b], [&] { return taped_steps(s, c, len, b, s->stream); }))
                 return rc;
-            for (int a = 0; a < 2; ++a)
-                if (int rc = s->capture(&s->vjp_graph[2 + 2 * b + a], [&] { return reverse_steps(s, len, b, a, s->stream); }))
-                    return rc;
+            if (int rc = s->capture(&s->vjp_graph[2 + b], [&] { return reverse_steps(s, len, b, s->stream); })) return rc;
         }
         s->vjp_len = len;
         s->vjp_bufs = *bufs;
@@ -1542,7 +1519,7 @@ int fvm2d_forward(fvm2d_solver *s, int nsteps, int checkpoints)
             s->set_flip(0);
         } else {
             if (count > 1 && m == s->vjp_len) {  // a full segment: one graph of its steps
-                CK(cudaGraphLaunch(s->vjp_graph[6], s->stream));
+                CK(cudaGraphLaunch(s->vjp_graph[4], s->stream));
             } else if (int rc = s->replay(m)) {
                 return rc;
             }
@@ -1575,20 +1552,18 @@ int fvm2d_vjp(fvm2d_solver *s, const double *cotangent_in, double *cotangent_out
         bool grew_adj;
         if (int rc = ensure(s->adj, s->adj_bytes, kAdjStates * sb, grew_adj)) return rc;
         if (grew_adj) s->drop_vjp_graphs();
-        if (int rc = ensure_fork(s)) return rc;
     } else if (int rc = vjp_workspace(s, &bufs)) {
         return rc;
     }
     char *const saved = s->adj + 5 * sb;
-    int lam = 0;  // adjoint buffer holding the current adjoint
     const StepControl after = *s->ctl_h;
     CK(cudaMemcpyAsync(saved, s->U, sb, cudaMemcpyDeviceToDevice, s->stream));
     if (int rc = cells_to_planes(s, cotangent_in, stride, s->adj)) return rc;
+    CK(cudaMemsetAsync(s->adj + sb, 0, sb, s->stream));  // the adjoint's second part
     const int count = s->ck_count;
     auto seg_len = [&](int k) { return segment_steps(s->fwd_steps, s->ck_len, count, k); };
     if (s->full_tape) {  // the forward taped every step: reverse only
-        if (int rc = reverse_steps(s, s->fwd_steps, 0, lam, s->stream)) return rc;
-        lam ^= s->fwd_steps & 1;
+        if (int rc = reverse_steps(s, s->fwd_steps, 0, s->stream)) return rc;
     } else {
         // segment k is taped in buffer k % bufs
         auto recompute_segment = [&](int k, cudaStream_t st) -> int {
@@ -1607,11 +1582,10 @@ int fvm2d_vjp(fvm2d_solver *s, const double *cotangent_in, double *cotangent_out
         auto reverse_segment = [&](int k, cudaStream_t st) -> int {
             const int m = seg_len(k), b = k % bufs;
             if (m == s->vjp_len) {
-                CK(cudaGraphLaunch(s->vjp_graph[2 + 2 * b + lam], st));
-            } else if (int rc = reverse_steps(s, m, b, lam, st)) {
+                CK(cudaGraphLaunch(s->vjp_graph[2 + b], st));
+            } else if (int rc = reverse_steps(s, m, b, st)) {
                 return rc;
             }
-            lam ^= m & 1;
             return FVM2D_OK;
         };
         if (bufs == 1) {
@@ -1643,7 +1617,11 @@ int fvm2d_vjp(fvm2d_solver *s, const double *cotangent_in, double *cotangent_out
         }
         s->last_taped = false;  // its buffer has been reused (or will be by the next call)
     }
-    if (int rc = planes_to_cells(s, s->adj + lam * sb, cotangent_out, stride)) return rc;
+    {
+        const fvm2d::AdjointLaunch L = adjoint_launch_of(s, sb);
+        CK(is_fp32(s->precision) ? fvm2d::adj32::adjoint_sum(L, s->stream) : fvm2d::adj::adjoint_sum(L, s->stream));
+    }
+    if (int rc = planes_to_cells(s, s->adj, cotangent_out, stride)) return rc;
     CK(cudaMemcpyAsync(s->U, saved, sb, cudaMemcpyDeviceToDevice, s->stream));
     *s->ctl_h = after;
     if (int rc = s->upload_control()) return rc;

@@ -100,13 +100,18 @@ FVM2D_DECLARE_VARIANT(jvp)
 // in c.B and the interface fluxes of the four sweeps (X of U, Y of U, Y of A,
 // X of B), each stored at the interface's right cell in planes mass, normal
 // momentum, energy, tangential momentum.  The step reads c.U and writes its
-// result to `out` (c.U when null).
-namespace fp64 {
-cudaError_t enqueue_step_taped(const LaunchConfig &c, cudaStream_t s, void *const flux[4], void *out);
-}
-namespace fp32 {
-cudaError_t enqueue_step_taped(const LaunchConfig &c, cudaStream_t s, void *const flux[4], void *out);
-}
+// result to `out`.  In tiles (whole problems) the result's ghost ring is left
+// to the next taped step, which fills it (`fill`) as it loads it, or to
+// enqueue_fill_ring; the step sweep by sweep is for row slabs.
+#define FVM2D_DECLARE_TAPED(ns)                                                                             \
+    namespace ns {                                                                                          \
+    cudaError_t enqueue_step_taped(const LaunchConfig &c, cudaStream_t s, void *const flux[4], void *out);  \
+    cudaError_t enqueue_tile_step_taped(const LaunchConfig &c, cudaStream_t s, void *const flux[4], void *out, \
+                                        bool fill);                                                         \
+    }
+
+FVM2D_DECLARE_TAPED(fp64)
+FVM2D_DECLARE_TAPED(fp32)
 
 // Records `msg` as the calling thread's fvm2d_last_error() text; returns code.
 int report_error(int code, const char *msg);

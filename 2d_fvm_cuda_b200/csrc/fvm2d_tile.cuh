@@ -77,6 +77,16 @@ struct TileArgs {
     PlanParams plan;
 };
 
+// What a taped step keeps for its adjoint besides its input state: X(U), Y(U)
+// and the interface fluxes of X(U), Y(U), Y(A1) and X(B1), each at the
+// interface's right cell in planes mass, normal momentum, energy, tangential
+// momentum.  The second sweeps' fluxes on the ring, where nothing is updated,
+// are stored as 0.
+template <typename Real>
+struct TapeArgs {
+    Field<Real> A1, B1, F[4];
+};
+
 template <typename Real>
 __device__ __forceinline__ GhostArgs<Real> ring_args(const TileArgs<Real> &a)
 {
@@ -159,10 +169,12 @@ __device__ __forceinline__ void tile_copy(Real *dst_shared, const Real *src)
 }
 
 // One step of tile (bx, by), by the Tile::NT threads of a block; fill: the
-// state's ring cells are computed for time t, else read.
-template <typename Real, class Phys, class T>
+// state's ring cells are computed for time t, else read.  TAPE: the step also
+// writes its tape (and the ring it fills, into the state it reads).
+template <typename Real, class Phys, class T, bool TAPE = false>
 __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, int bx, int by, unsigned char *smem,
-                                          double &vmax, int &bad, bool fill = false, double t = 0.0)
+                                          double &vmax, int &bad, bool fill = false, double t = 0.0,
+                                          const TapeArgs<Real> *tape = nullptr)
 {
     constexpr bool kResidual = split_storage<Phys>::value;
     using Word = unsigned long long;
@@ -180,6 +192,12 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
     const int x0 = 2 + bx * T::TX, y0 = 2 + by * T::TY;  // first written cell
     const int ncol = min(NC, a.nx - x0 + 2), nrow = min(T::NR, a.ny - y0 + 2);  // loaded columns and rows in the array
 
+    // TAPE: the cells whose tape this tile writes -- its own and, at an edge of
+    // the array, the ring's beside them
+    const bool last_x = x0 + T::TX > a.nx - 3, last_y = y0 + T::TY > a.ny - 3;
+    auto owns_x = [&](int x) { return (x >= x0 || bx == 0) && (x < x0 + T::TX || last_x); };
+    auto owns_y = [&](int y) { return (y >= y0 || by == 0) && (y < y0 + T::TY || last_y); };
+    const Cell<Real> none = {Real(0), Real(0), Real(0), Real(0)};
     // does the loaded tile reach the ring?
     const bool edge = fill && (bx == 0 || by == 0 || x0 - 2 + NC > a.nx - 2 || y0 - 2 + T::NR > a.ny - 2);
     for (int i = tid; i < T::NR * NC; i += T::NT) {
@@ -194,6 +212,7 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
             q[2 * NC] = v.un;
             q[3 * NC] = v.ut;
             if constexpr (kResidual) lU[r * T::kLo + c] = 0ull;  // a ring cell holds its FP32 value exactly
+            if (TAPE && x0 - 2 + c < a.nx && owns_x(x) && owns_y(y)) store_cell(a.src, x, y, 2, 3, v);
             continue;
         }
         tile_copy(q, &a.src.at(0, x, y));
@@ -221,6 +240,23 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
     }
     async_wait<0>();
     __syncthreads();
+    if constexpr (TAPE) {  // the ring's part: sweeps across it pass its cells through
+        for (int i = tid; i < T::NR * NC; i += T::NT) {
+            const int r = i / NC, c = i - r * NC, x = x0 - 2 + c, y = y0 - 2 + r;
+            const bool col = x < 2 || x >= a.nx - 2, row = y < 2 || y >= a.ny - 2;
+            if (!(col || row) || x >= a.nx || y >= a.ny || !owns_x(x) || !owns_y(y)) continue;
+            const Real *const q = sU + r * RS + c;
+            const Cell<Real> v = {q[0], q[NC], q[2 * NC], q[3 * NC]};
+            if (col) {
+                store_cell(tape->A1, x, y, 2, 3, v);
+                store_cell(tape->F[2], x, y, 2, 3, none);
+            }
+            if (row) {
+                store_cell(tape->B1, x, y, 2, 3, v);
+                store_cell(tape->F[3], x, y, 2, 3, none);
+            }
+        }
+    }
 
     // residual word -> the residuals of fields 0, 1, f2, f3
     auto parts = [](Word w, int f2, int f3) {
@@ -290,6 +326,14 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
             const Cell<Real> FL = shfl_up(F);
             // the updated cell: one back along the line
             const int ru = xdir ? r : r + 1, cu = xdir ? c - 1 : c;
+            if constexpr (TAPE) {
+                // the interface before this lane's cell, kept at the cell:
+                // cells 2 .. n-2 along x, rows n-3 .. 1 along y
+                const int x = x0 - 2 + c, y = y0 - 2 + r;
+                const bool in = xdir ? x <= a.nx - 2 && (x < x0 + T::TX || x == a.nx - 2) && (phase || owns_y(y))
+                                     : y <= a.ny - 3 && (y >= y0 || by == 0) && (phase || owns_x(x));
+                if (mine && k >= 1 && in) store_cell(tape->F[phase == 0 ? (xdir ? 0 : 1) : xdir ? 3 : 2], x, y, 2, 3, F);
+            }
             if (!mine || k < 2) continue;
             const int fn = xdir ? 2 : 3;
             auto updated = [&] {
@@ -324,6 +368,11 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
                 d[NC] = v.p;
                 d[on] = v.un;
                 d[ot] = v.ut;
+                if constexpr (TAPE) {
+                    const int x = x0 - 2 + cu, y = y0 - 2 + ru;
+                    if (phase == 0 && xdir && x <= a.nx - 3 && owns_y(y)) store_cell(tape->A1, x, y, 2, 3, v);
+                    if (phase == 0 && !xdir && y <= a.ny - 3 && owns_x(x)) store_cell(tape->B1, x, y, 3, 2, v);
+                }
             }
         }
         __syncthreads();
@@ -408,6 +457,25 @@ __global__ void __launch_bounds__(T::NT, MINB) step_tile_kernel(TileArgs<Real> a
     int bad = 0;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
     tile_step<Real, Phys, T>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, c.ring_due, c.t);
+    end_tile<T::NT>(vmax, bad, a.ctl, c, a.plan, gridDim.x * gridDim.y);
+}
+
+// A taped step, from src to dst whatever the parity; fill: the ring of src is
+// not filled yet (the steps of a tape but its first).
+template <typename Real, class Phys, class T, int MINB>
+__global__ void __launch_bounds__(T::NT, MINB) step_tape_kernel(TileArgs<Real> a, TapeArgs<Real> tape, int fill)
+{
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    pdl_launch();
+    pdl_wait();
+    __shared__ StepControl c;
+    if (threadIdx.x == 0) c = *a.ctl;
+    __syncthreads();
+    if (!c.active) return;
+    double vmax = 0.0;
+    int bad = 0;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
+    tile_step<Real, Phys, T, true>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, fill != 0, c.t, &tape);
     end_tile<T::NT>(vmax, bad, a.ctl, c, a.plan, gridDim.x * gridDim.y);
 }
 

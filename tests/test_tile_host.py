@@ -18,6 +18,8 @@ def th(tmp_path_factory):
     lib = build_host(tmp_path_factory, "tile_host.cpp")
     lib.th_step.argtypes = ([ctypes.c_int] * 2 + [ctypes.c_void_p] * 2 + [ctypes.c_int] * 2 + [ctypes.c_double] * 5 +
                             [ctypes.c_void_p] * 2)
+    lib.th_tape.argtypes = [ctypes.c_int, ctypes.c_void_p] + [ctypes.c_int] * 3 + [ctypes.c_double] * 4 + [ctypes.c_int]
+    lib.th_tape.restype = ctypes.c_long
     return lib
 
 
@@ -50,3 +52,18 @@ def test_interior_of_a_step_equals_the_oracle(th, oracle, pkg, shape):
             else:
                 # two sweeps of relative rounding, as the walkers' items (1e-13 each)
                 assert np.abs(A - B).max() <= 2e-13 * np.abs(B).max(), (nx, ny)
+
+
+@pytest.mark.parametrize("strategy", range(7))
+@pytest.mark.parametrize("shape", range(4))
+def test_tape_equals_the_sweeps(th, oracle, pkg, shape, strategy):
+    """What a taped step in tiles keeps (X(U), Y(U), the sweeps' fluxes, and
+    the ring it fills in its input) against the taped sweeps, bit for bit."""
+    tx, ty = SHAPES[shape]
+    for k, (nx, ny) in enumerate([(6, 6), (tx + 4, ty + 4), (tx + 5, 2 * ty + 3)]):
+        U, width, height, _ = sweep_case(pkg, oracle, nx, ny, 60 + k)
+        t = 0.01 * k
+        U = np.ascontiguousarray(oracle.ghost(U, strategy, t=t, width=width, height=height))
+        dt = 0.3 * min(width / nx, height / ny) / oracle.max_speed(U)  # the presets' inflows are in the ring
+        for fill in (0, 1):
+            assert th.th_tape(shape, U.ctypes.data, nx, ny, strategy, t, dt, width, height, fill) == 0, (nx, ny, fill)
