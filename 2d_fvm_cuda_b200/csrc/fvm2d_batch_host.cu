@@ -9,9 +9,10 @@
 // problem carries its own dt, time and end time in its control record, and its
 // tiles are skipped once its loop has ended.  (Sweep by sweep, five launches:
 // x-sweep, y-sweep, y-sweep, final x-sweep, ghost ring, if the autotuner finds
-// that faster.)  The step is captured in CUDA graphs (16 steps and 1 step) that
-// are replayed until no problem has a step in flight; each replay reads the
-// control records back (64 bytes per problem).  fvm2d_batch_autotune times
+// that faster.)  Steps in tiles are enqueued up to 16 at a time (a launch costs
+// the host less than any step the device), sweeps as CUDA graphs of 16 steps
+// and 1 step, until no problem has a step in flight; after each group the
+// control records are read back (64 bytes per problem).  fvm2d_batch_autotune times
 // candidate y-segment lengths and sweep grid sizes on the batch itself and
 // keeps the fastest.
 //
@@ -210,32 +211,49 @@ struct fvm2d_batch {
     long long y_items(int p) const { return (long long)((nx[p] + 31) / 32) * y_segments(ny[p], T); }
     long long tiles(int p) const { return kBatchVariants[precision].tiles(tile_shape, nx[p], ny[p]); }
 
+    // Tile prefix counts of the listed problems -> device.
+    int upload_tiles()
+    {
+        std::vector<long long> t0(np + 1, 0);
+        for (int p = 0; p < np; ++p) t0[p + 1] = t0[p] + (listed[p] ? tiles(p) : 0);
+        CK(cudaMemcpyAsync(t0_d, t0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
+        L.tile_total = t0[np];
+        return FVM2D_OK;
+    }
+
     // Item prefix counts of the listed problems (others get no items) -> device.
     int upload_items()
     {
-        std::vector<long long> x0(np + 1, 0), y0(np + 1, 0), t0(np + 1, 0);
+        std::vector<long long> x0(np + 1, 0), y0(np + 1, 0);
         for (int p = 0; p < np; ++p) {
             x0[p + 1] = x0[p] + (listed[p] ? x_items(p) : 0);
             y0[p + 1] = y0[p] + (listed[p] ? y_items(p) : 0);
-            t0[p + 1] = t0[p] + (listed[p] ? tiles(p) : 0);
         }
         CK(cudaMemcpyAsync(x0_d, x0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
         CK(cudaMemcpyAsync(y0_d, y0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
-        CK(cudaMemcpyAsync(t0_d, t0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
+        if (int rc = upload_tiles()) return rc;
         CK(cudaStreamSynchronize(stream));
         L.x_total = x0[np];
         L.y_total = y0[np];
         L.t0 = use_tiles ? t0_d : nullptr;
-        L.tile_total = t0[np];
         L.tile_shape = tile_shape;
         return FVM2D_OK;
     }
 
-    // After a graph replay: drops the problems whose loop has ended from the
-    // item lists once they hold at least a quarter of the listed x items.
+    // After a group of steps: drops the problems whose loop has ended from the
+    // lists once they hold at least an eighth of the listed tiles, or a
+    // quarter of the listed x items (whose lists the graphs hold).
     int compact_items()
     {
         long long ended = 0;
+        if (use_tiles) {
+            for (int p = 0; p < np; ++p)
+                if (listed[p] && !ctl_h[p].active) ended += tiles(p);
+            if (ended == 0 || 8 * ended < L.tile_total) return FVM2D_OK;
+            for (int p = 0; p < np; ++p)
+                if (!ctl_h[p].active) listed[p] = 0;
+            return upload_tiles();
+        }
         for (int p = 0; p < np; ++p)
             if (listed[p] && !ctl_h[p].active) ended += x_items(p);
         if (ended == 0 || 4 * ended < L.x_total) return FVM2D_OK;
@@ -290,8 +308,8 @@ struct fvm2d_batch {
             if (int rc = upload_items()) return rc;
             drop_graphs();
         }
-        if (int rc = build_graphs()) return rc;
-        std::vector<int> before(np);
+        if (!use_tiles)
+            if (int rc = build_graphs()) return rc;
         for (int p = 0; p < np; ++p) {
             std::memset(&ctl_h[p], 0, sizeof(StepControl));
             ctl_h[p].step_limit = limit;
@@ -302,18 +320,30 @@ struct fvm2d_batch {
         CK(cudaEventRecord(ev0, stream));
         CK(kBatchVariants[precision].init(L, stream));
         long long launches = 1;
-        long long budget = limit;
+        long long budget = limit, ahead = kGraphSteps[0];
         for (;;) {
-            const int which = budget >= kGraphSteps[0] ? 0 : 1;
-            CK(cudaGraphLaunch(graph[which], stream));
-            budget -= kGraphSteps[which];
-            launches += (long long)kGraphSteps[which] * (use_tiles ? 1 : fvm2d::kStepKernels);
+            if (use_tiles) {
+                const int n = (int)std::max(1ll, std::min(ahead, budget));
+                for (int k = 0; k < n; ++k) CK(kBatchVariants[precision].step(L, stream));
+                budget -= n;
+                launches += n;
+            } else {
+                const int which = budget >= kGraphSteps[0] ? 0 : 1;
+                CK(cudaGraphLaunch(graph[which], stream));
+                budget -= kGraphSteps[which];
+                launches += (long long)kGraphSteps[which] * fvm2d::kStepKernels;
+            }
             CK(cudaMemcpyAsync(ctl_h, ctl_d, sizeof(StepControl) * np, cudaMemcpyDeviceToHost, stream));
             CK(cudaStreamSynchronize(stream));
             bool any = false;
             for (int p = 0; p < np && !any; ++p) any = ctl_h[p].active != 0;
             if (!any) break;
             if (int rc = compact_items()) return rc;
+            // the steps the longest run has left at its last step size
+            double left = 0.0;
+            for (int p = 0; p < np; ++p)
+                if (ctl_h[p].active) left = std::max(left, (t_end[p] - ctl_h[p].t) / ctl_h[p].dt);
+            ahead = left < kGraphSteps[0] ? (long long)left + 1 : kGraphSteps[0];
         }
         if (use_tiles) {
             CK(kBatchVariants[precision].fill_ring(L, stream));

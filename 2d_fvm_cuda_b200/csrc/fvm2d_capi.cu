@@ -267,6 +267,16 @@ struct fvm2d_solver {
         return c;
     }
 
+    // A parameter was set: a taped forward no longer counts, whatever the value.
+    void discard_tape()
+    {
+        last_taped = false;  // taped with the former parameters
+        if (full_tape) {     // the tape no longer belongs to this solver's step
+            full_tape = false;
+            fwd_steps = -1;
+        }
+    }
+
     void drop_graph()
     {
         for (auto &g : graph) {
@@ -277,11 +287,7 @@ struct fvm2d_solver {
         slab_graph = nullptr;
         graph_variant = -1;
         drop_vjp_graphs();
-        last_taped = false;  // taped with the former parameters
-        if (full_tape) {  // a parameter changed: the tape no longer belongs to this solver's step
-            full_tape = false;
-            fwd_steps = -1;
-        }
+        discard_tape();
     }
 
     void drop_vjp_graphs()
@@ -522,6 +528,10 @@ int fvm2d_destroy(fvm2d_solver *s)
     {                                                                          \
         if (int rc = check(s)) return rc;                                      \
         if (!(cond)) return fail(FVM2D_ERR_INVALID, msg);                      \
+        if (s->field == v) { /* the graphs hold this value already */          \
+            s->discard_tape();                                                 \
+            return FVM2D_OK;                                                   \
+        }                                                                      \
         s->field = v;                                                          \
         s->drop_graph();                                                       \
         return FVM2D_OK;                                                       \
@@ -537,6 +547,10 @@ int fvm2d_set_precision(fvm2d_solver *s, int v)
 {
     if (int rc = check(s)) return rc;
     if (!(v >= 0 && v < kNumVariants)) return fail(FVM2D_ERR_INVALID, "unknown precision");
+    if (v == s->precision) {
+        s->discard_tape();
+        return FVM2D_OK;
+    }
     if (s->have_state && storage_of(v) != storage_of(s->precision)) {
         // keep the current state: convert its planes to the new storage type
         const long long n = 4 * s->plane;
@@ -558,6 +572,10 @@ int fvm2d_set_spatial_layout(fvm2d_solver *s, double width, double height)
 {
     if (int rc = check(s)) return rc;
     if (!(width > 0.0 && height > 0.0)) return fail(FVM2D_ERR_INVALID, "width and height must be positive");
+    if (width == s->width && height == s->height) {
+        s->discard_tape();
+        return FVM2D_OK;
+    }
     s->width = width;
     s->height = height;
     s->drop_graph();
