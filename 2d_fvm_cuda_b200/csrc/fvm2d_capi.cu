@@ -45,6 +45,9 @@ using fvm2d::conserved_partials;
 using fvm2d::conserved_sum;
 using fvm2d::convert_planes;
 using fvm2d::is_device_pointer;
+using fvm2d::is_memory_of;
+using fvm2d::kRowThreads;
+using fvm2d::rows_grid;
 using fvm2d::rows_in;
 using fvm2d::rows_out;
 using fvm2d::soa_to_aos;
@@ -430,11 +433,15 @@ int check(fvm2d_solver *s)
 
 int upload(fvm2d_solver *s, const double *cells, int stride)
 {
-    const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
-    const cudaMemcpyKind kind = is_device_pointer(cells) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    CK(cudaMemcpyAsync(s->scratch, cells, bytes, kind, s->stream));
+    const double *src = cells;
+    if (!is_memory_of(cells, s->device)) {
+        const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
+        const cudaMemcpyKind kind = is_device_pointer(cells) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        CK(cudaMemcpyAsync(s->scratch, cells, bytes, kind, s->stream));
+        src = s->scratch;
+    }
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
-        aos_to_soa<<<148 * 4, 256, 0, s->stream>>>(s->scratch, stride, st, s->nx, s->ny, s->pitch, s->plane);
+        aos_to_soa<<<148 * 4, 256, 0, s->stream>>>(src, stride, st, s->nx, s->ny, s->pitch, s->plane);
     });
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s->stream));
@@ -601,9 +608,13 @@ int fvm2d_set_state_planes(fvm2d_solver *s, const double *planes)
 {
     if (int rc = check(s)) return rc;
     if (!planes) return fail(FVM2D_ERR_INVALID, "null state pointer");
-    CK(cudaMemcpyAsync(s->scratch, planes, sizeof(double) * 4 * (size_t)s->nx * s->ny, cudaMemcpyDefault, s->stream));
+    const double *src = planes;
+    if (!is_memory_of(planes, s->device)) {
+        CK(cudaMemcpyAsync(s->scratch, planes, sizeof(double) * 4 * (size_t)s->nx * s->ny, cudaMemcpyDefault, s->stream));
+        src = s->scratch;
+    }
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
-        rows_in<<<148 * 4, 256, 0, s->stream>>>(st, s->plane, s->pitch, 0, s->ny, s->nx, s->scratch);
+        rows_in<<<rows_grid(s->ny, s->nx), kRowThreads, 0, s->stream>>>(st, s->plane, s->pitch, 0, s->ny, s->nx, src);
     });
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s->stream));
@@ -648,13 +659,17 @@ int fvm2d_get_state(fvm2d_solver *s, double *cells, int stride)
     if (!cells) return fail(FVM2D_ERR_INVALID, "null state pointer");
     if (stride != 4 && stride != 5) return fail(FVM2D_ERR_INVALID, "stride must be 4 or 5 doubles per cell");
     if (!s->have_state) return fail(FVM2D_ERR_STATE, "no state has been set");
+    const bool direct = is_memory_of(cells, s->device);
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
-        soa_to_aos<<<148 * 4, 256, 0, s->stream>>>(st, s->nx, s->ny, s->pitch, s->plane, stride, s->scratch);
+        soa_to_aos<<<148 * 4, 256, 0, s->stream>>>(st, s->nx, s->ny, s->pitch, s->plane, stride,
+                                                   direct ? cells : s->scratch);
     });
     CK(cudaGetLastError());
-    const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
-    const cudaMemcpyKind kind = is_device_pointer(cells) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    CK(cudaMemcpyAsync(cells, s->scratch, bytes, kind, s->stream));
+    if (!direct) {
+        const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
+        const cudaMemcpyKind kind = is_device_pointer(cells) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+        CK(cudaMemcpyAsync(cells, s->scratch, bytes, kind, s->stream));
+    }
     CK(cudaStreamSynchronize(s->stream));
     return FVM2D_OK;
 }
@@ -848,11 +863,14 @@ static int rows_check(fvm2d_solver *s, int j0, int nrows, const void *buf)
 int fvm2d_get_rows(fvm2d_solver *s, int j0, int nrows, double *rows)
 {
     if (int rc = rows_check(s, j0, nrows, rows)) return rc;
+    const bool direct = is_memory_of(rows, s->device);
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
-        rows_out<<<148 * 4, 256, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx, s->scratch);
+        rows_out<<<rows_grid(nrows, s->nx), kRowThreads, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx,
+                                                                         direct ? rows : s->scratch);
     });
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(rows, s->scratch, sizeof(double) * 4 * (size_t)nrows * s->nx, cudaMemcpyDefault, s->stream));
+    if (!direct)
+        CK(cudaMemcpyAsync(rows, s->scratch, sizeof(double) * 4 * (size_t)nrows * s->nx, cudaMemcpyDefault, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return FVM2D_OK;
 }
@@ -860,9 +878,13 @@ int fvm2d_get_rows(fvm2d_solver *s, int j0, int nrows, double *rows)
 int fvm2d_set_rows(fvm2d_solver *s, int j0, int nrows, const double *rows)
 {
     if (int rc = rows_check(s, j0, nrows, rows)) return rc;
-    CK(cudaMemcpyAsync(s->scratch, rows, sizeof(double) * 4 * (size_t)nrows * s->nx, cudaMemcpyDefault, s->stream));
+    const double *src = rows;
+    if (!is_memory_of(rows, s->device)) {
+        CK(cudaMemcpyAsync(s->scratch, rows, sizeof(double) * 4 * (size_t)nrows * s->nx, cudaMemcpyDefault, s->stream));
+        src = s->scratch;
+    }
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
-        rows_in<<<148 * 4, 256, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx, s->scratch);
+        rows_in<<<rows_grid(nrows, s->nx), kRowThreads, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx, src);
     });
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s->stream));
@@ -888,7 +910,7 @@ int fvm2d_get_rows_async(fvm2d_solver *s, int j0, int nrows, double *rows)
     if (int rc = rows_check(s, j0, nrows, rows)) return rc;
     if (!is_device_pointer(rows)) return fail(FVM2D_ERR_INVALID, "the row buffer must be device memory");
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
-        rows_out<<<148 * 4, 256, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx, rows);
+        rows_out<<<rows_grid(nrows, s->nx), kRowThreads, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx, rows);
     });
     CK(cudaGetLastError());
     return FVM2D_OK;
@@ -899,7 +921,7 @@ int fvm2d_set_rows_async(fvm2d_solver *s, int j0, int nrows, const double *rows)
     if (int rc = rows_check(s, j0, nrows, rows)) return rc;
     if (!is_device_pointer(rows)) return fail(FVM2D_ERR_INVALID, "the row buffer must be device memory");
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
-        rows_in<<<148 * 4, 256, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx, rows);
+        rows_in<<<rows_grid(nrows, s->nx), kRowThreads, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx, rows);
     });
     CK(cudaGetLastError());
     return FVM2D_OK;

@@ -7,6 +7,8 @@
 
 #include <cuda_runtime.h>
 
+#include <stdint.h>
+
 #include "fvm2d_split.cuh"
 
 namespace fvm2d {
@@ -16,23 +18,23 @@ template <class S>
 static __global__ void aos_to_soa(const double *__restrict__ in, int stride, S U, int nx, int ny, int pitch,
                                   long long plane)
 {
-    const long long n = (long long)nx * ny;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int y = int(k / nx), x = int(k % nx);
+    const unsigned n = (unsigned)nx * (unsigned)ny;  // below 2^31
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const unsigned y = k / (unsigned)nx, x = k - y * (unsigned)nx;
         const long long o = (long long)y * pitch + x;
-        for (int f = 0; f < 4; ++f) U.put(f * plane + o, in[k * stride + f]);
+        for (int f = 0; f < 4; ++f) U.put(f * plane + o, in[(size_t)k * stride + f]);
     }
 }
 
 template <class S>
 static __global__ void soa_to_aos(S U, int nx, int ny, int pitch, long long plane, int stride, double *__restrict__ out)
 {
-    const long long n = (long long)nx * ny;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int y = int(k / nx), x = int(k % nx);
+    const unsigned n = (unsigned)nx * (unsigned)ny;  // below 2^31
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const unsigned y = k / (unsigned)nx, x = k - y * (unsigned)nx;
         const long long o = (long long)y * pitch + x;
-        for (int f = 0; f < 4; ++f) out[k * stride + f] = U.get(f * plane + o);
-        for (int f = 4; f < stride; ++f) out[k * stride + f] = 0.0;
+        for (int f = 0; f < 4; ++f) out[(size_t)k * stride + f] = U.get(f * plane + o);
+        for (int f = 4; f < stride; ++f) out[(size_t)k * stride + f] = 0.0;
     }
 }
 
@@ -46,25 +48,44 @@ static __global__ void convert_planes(S in, D out, long long n)
 }
 
 // Rows j0 .. j0+nrows-1 of the four planes, packed as [4][nrows][nx] doubles
-// (rows_out) and back (rows_in).
-template <class S>
-static __global__ void rows_out(S U, long long plane, int pitch, int j0, int nrows, int nx, double *__restrict__ out)
+// (rows_out) and back (rows_in).  A block takes 4 * NT columns of a row at a
+// time (grid of rows_grid), so no element is located by a division; bound by
+// memory.
+constexpr int kRowThreads = 256, kRowCols = 4 * kRowThreads;
+inline dim3 rows_grid(int nrows, int nx)
 {
-    const long long per = (long long)nrows * nx, n = 4 * per;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int f = int(k / per), r = int(k % per / nx), x = int(k % nx);
-        out[k] = U.get(f * plane + (long long)(j0 + r) * pitch + x);
+    const long long rows = 4ll * nrows;
+    return dim3((nx + kRowCols - 1) / kRowCols, rows < 65535 ? (unsigned)rows : 65535u);
+}
+
+template <class F>
+static __device__ __forceinline__ void for_rows(int nrows, int nx, F f)
+{
+    const int x0 = blockIdx.x * kRowCols + threadIdx.x;
+    for (long long q = blockIdx.y; q < 4ll * nrows; q += gridDim.y) {
+        const int field = int(q / nrows), r = int(q % nrows);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (x0 + u * kRowThreads < nx) f(field, r, q, x0 + u * kRowThreads);
     }
 }
 
 template <class S>
-static __global__ void rows_in(S U, long long plane, int pitch, int j0, int nrows, int nx, const double *__restrict__ in)
+static __global__ void __launch_bounds__(kRowThreads) rows_out(S U, long long plane, int pitch, int j0, int nrows, int nx,
+                                                               double *__restrict__ out)
 {
-    const long long per = (long long)nrows * nx, n = 4 * per;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int f = int(k / per), r = int(k % per / nx), x = int(k % nx);
-        U.put(f * plane + (long long)(j0 + r) * pitch + x, in[k]);
-    }
+    for_rows(nrows, nx, [&](int f, int r, long long q, int x) {
+        out[q * nx + x] = U.get(f * plane + (long long)(j0 + r) * pitch + x);
+    });
+}
+
+template <class S>
+static __global__ void __launch_bounds__(kRowThreads) rows_in(S U, long long plane, int pitch, int j0, int nrows, int nx,
+                                                              const double *__restrict__ in)
+{
+    for_rows(nrows, nx, [&](int f, int r, long long q, int x) {
+        U.put(f * plane + (long long)(j0 + r) * pitch + x, in[q * nx + x]);
+    });
 }
 
 // Conserved totals of the interior cells (rows and columns 2 .. n-3, the
@@ -125,6 +146,19 @@ inline bool is_device_pointer(const void *p)
         return false;
     }
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+}
+
+// True for memory allocated on `device` itself: what a kernel there may read
+// and write in place.  (Memory of another device, managed memory or an odd
+// address goes through a copy.)
+inline bool is_memory_of(const void *p, int device)
+{
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == device && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0;
 }
 
 } // namespace fvm2d
