@@ -30,7 +30,10 @@ struct Dual {
 __host__ __device__ __forceinline__ Dual operator+(Dual a, Dual b) { return Dual(a.v + b.v, a.d + b.d); }
 __host__ __device__ __forceinline__ Dual operator-(Dual a, Dual b) { return Dual(a.v - b.v, a.d - b.d); }
 __host__ __device__ __forceinline__ Dual operator-(Dual a) { return Dual(-a.v, -a.d); }
-__host__ __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
+__host__ __device__ __forceinline__ Dual operator*(Dual a, Dual b)
+{
+    return Dual(a.v * b.v, ::fma(a.d, b.v, a.v * b.d));
+}
 __host__ __device__ __forceinline__ Dual operator/(Dual a, Dual b)
 {
     const double q = a.v / b.v;
@@ -49,13 +52,18 @@ __device__ __forceinline__ Dual sqrt(Dual a)
     const double r = ::sqrt(a.v);
     return Dual(r, a.d / (2.0 * r));
 }
+#ifndef FVM2D_DUAL_RECIPROCALS  // the tangent-linear build brings its own (fvm2d_jvp.cu)
 __device__ __forceinline__ Dual rrsqrt(Dual a)
 {
     const double r = ::rsqrt(a.v);
     return Dual(r, -0.5 * r * r * r * a.d);
 }
+#endif
 __device__ __forceinline__ Dual fabs(Dual a) { return a.v < 0.0 ? -a : a; }
-__device__ __forceinline__ Dual fma(Dual a, Dual b, Dual c) { return a * b + c; }
+__device__ __forceinline__ Dual fma(Dual a, Dual b, Dual c)
+{
+    return Dual(::fma(a.v, b.v, c.v), ::fma(a.d, b.v, ::fma(a.v, b.d, c.d)));
+}
 
 // Warp shuffles of a dual move both parts.
 __device__ __forceinline__ Dual lane_down(Dual a)
