@@ -32,13 +32,17 @@ __device__ __forceinline__ Dual rrsqrt(Dual a)
 #define FVM2D_PHYS Hoisted
 #define FVM2D_X_MINB 2
 #define FVM2D_Y_MINB 2
-// tiles of a step (fvm2d_tile.cuh): warps per block and resident blocks per SM
-#define FVM2D_TILE0_WARPS 8
+// tiles of a step (fvm2d_tile.cuh): warps per block and resident blocks per SM,
+// and the rule on sizes (best_tile_shape); measured best of several: 256 x 300
+// 47 -> 40 us per step, 100^2 13.9 -> 10.3
+#define FVM2D_TILE0_WARPS 10
 #define FVM2D_TILE0_MINB 1
-#define FVM2D_TILE1_WARPS 8
+#define FVM2D_TILE1_WARPS 10
 #define FVM2D_TILE1_MINB 1
-#define FVM2D_TILE2_WARPS 8
-#define FVM2D_TILE2_MINB 1
-#define FVM2D_TILE3_WARPS 5
+#define FVM2D_TILE2_WARPS 5
+#define FVM2D_TILE2_MINB 2
+#define FVM2D_TILE3_WARPS 10
 #define FVM2D_TILE3_MINB 1
+#define FVM2D_TILE0_NEED 2
+#define FVM2D_TILE1_NEED 1e9
 #include "fvm2d_variant.inc"
