@@ -247,8 +247,10 @@ __global__ void __launch_bounds__(T::NT, MINB) batch_tile_kernel(BatchArgs<Real>
     double vmax = 0.0;
     int bad = 0;
     if (k == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
-    tile_step<Real, Phys, T>(a, c.dt, k % ntx, k / ntx, tile_smem, vmax, bad, c.ring_due, c.t);
+    TileResults<Real, T> res;
+    tile_step<Real, Phys, T>(a, c.dt, k % ntx, k / ntx, tile_smem, vmax, bad, res, c.ring_due, c.t);
     end_tile<T::NT>(vmax, bad, ctl, c, a.plan, unsigned(b.t0[p + 1] - b.t0[p]));
+    tile_store<Real, Phys, T>(a, k % ntx, k / ntx, res);
 }
 
 // Stores the ghost rings after steps in tiles.

@@ -168,13 +168,20 @@ __device__ __forceinline__ void tile_copy(Real *dst_shared, const Real *src)
         *dst_shared = *src;
 }
 
+// Results of a merged tile a thread holds until it stores them (tile_store).
+template <typename Real, class T>
+struct TileResults {
+    static constexpr int N = (T::TX * T::TY + T::NT - 1) / T::NT;
+    Cell<Real> v[N];
+};
+
 // One step of tile (bx, by), by the Tile::NT threads of a block; fill: the
 // state's ring cells are computed for time t, else read.  TAPE: the step also
 // writes its tape (and the ring it fills, into the state it reads).
 template <typename Real, class Phys, class T, bool TAPE = false>
 __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, int bx, int by, unsigned char *smem,
-                                          double &vmax, int &bad, bool fill = false, double t = 0.0,
-                                          const TapeArgs<Real> *tape = nullptr)
+                                          double &vmax, int &bad, TileResults<Real, T> &res, bool fill = false,
+                                          double t = 0.0, const TapeArgs<Real> *tape = nullptr)
 {
     constexpr bool kResidual = split_storage<Phys>::value;
     using Word = unsigned long long;
@@ -263,27 +270,32 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
         auto part = [&](int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
         return Cell<Real>{part(0), part(1), part(f2), part(f3)};
     };
-    // the step's result at tile cell (r, c): branch A (ra, la) averaged with
+    // the step's result at tile cell (r, c): branch A (sU, lU) averaged with
     // branch B in primitive variables (src/basicFuns.cuh:264-274)
-    auto finish = [&](int r, int c, auto b) {
-        const int x = x0 - 2 + c, y = y0 - 2 + r;
+    auto average = [&](int r, int c, const Cell<Real> &b) {
         const Real *const ra = sU + r * RS + c;
         const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
-        Cell<Real> o;
-        if constexpr (kResidual) {
-            const Cell<double> d = join_cell(A, parts(lU[r * T::kLo + c], 2, 3));
-            o = store_split(a.dst, x, y, 2, 3,
-                            Cell<double>{(d.rho + b.rho) * 0.5, (d.p + b.p) * 0.5, (d.un + b.un) * 0.5,
-                                         (d.ut + b.ut) * 0.5});
-        } else {
-            o.rho = (A.rho + b.rho) * Real(0.5);
-            o.p = (A.p + b.p) * Real(0.5);
-            o.un = (A.un + b.un) * Real(0.5);
-            o.ut = (A.ut + b.ut) * Real(0.5);
-            store_cell(a.dst, x, y, 2, 3, o);
-        }
+        return Cell<Real>{(A.rho + b.rho) * Real(0.5), (A.p + b.p) * Real(0.5), (A.un + b.un) * Real(0.5),
+                          (A.ut + b.ut) * Real(0.5)};
+    };
+    auto note = [&](const Cell<Real> &o) {
         vmax = fmax(vmax, wave_speed(o.rho, o.p, o.un, o.ut, a.gamma));
         bad |= !(o.rho > Real(0) && o.p > Real(0));  // NaN fails both tests
+    };
+    auto finish = [&](int r, int c, auto b) {
+        const int x = x0 - 2 + c, y = y0 - 2 + r;
+        if constexpr (kResidual) {
+            const Real *const ra = sU + r * RS + c;
+            const Cell<double> d = join_cell(Cell<Real>{ra[0], ra[NC], ra[2 * NC], ra[3 * NC]},
+                                             parts(lU[r * T::kLo + c], 2, 3));
+            note(store_split(a.dst, x, y, 2, 3,
+                             Cell<double>{(d.rho + b.rho) * 0.5, (d.p + b.p) * 0.5, (d.un + b.un) * 0.5,
+                                          (d.ut + b.ut) * 0.5}));
+        } else {
+            const Cell<Real> o = average(r, c, b);
+            store_cell(a.dst, x, y, 2, 3, o);
+            note(o);
+        }
     };
 
     // tasks along x and along y of the two sweeps of each branch
@@ -378,15 +390,46 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
         __syncthreads();
     }
     if constexpr (MERGE) {
-        const int w = ncol - 4;
-        for (int i = tid; i < T::TY * T::TX; i += T::NT) {
-            const int r = 2 + i / T::TX, c = 2 + i % T::TX;
-            if (c - 2 >= w || r - 2 >= nrow - 4) continue;
+#pragma unroll
+        for (int q = 0; q < TileResults<Real, T>::N; ++q) {
+            const int i = tid + q * T::NT, r = 2 + i / T::TX, c = 2 + i % T::TX;
+            if (i >= T::TX * T::TY || c >= ncol - 2 || r >= nrow - 2) continue;
             const Real *const rb = sR + r * RS + c;
-            const Cell<Real> b = {rb[0], rb[NC], rb[2 * NC], rb[3 * NC]};
-            finish(r, c, b);
+            res.v[q] = average(r, c, Cell<Real>{rb[0], rb[NC], rb[2 * NC], rb[3 * NC]});
+            note(res.v[q]);
         }
     }
+}
+
+// Stores the results of a merged tile.  They come after the block's maximum
+// and ticket: nothing in the step waits for them, and a fence issued behind
+// them would.
+template <typename Real, class Phys, class T>
+__device__ __forceinline__ void tile_store(const TileArgs<Real> &a, int bx, int by, const TileResults<Real, T> &res)
+{
+    if constexpr (T::kMerge && !split_storage<Phys>::value) {
+        const int x0 = 2 + bx * T::TX, y0 = 2 + by * T::TY;
+#pragma unroll
+        for (int q = 0; q < TileResults<Real, T>::N; ++q) {
+            const int i = threadIdx.x + q * T::NT, x = x0 + i % T::TX, y = y0 + i / T::TX;
+            if (i < T::TX * T::TY && x <= a.nx - 3 && y <= a.ny - 3) store_cell(a.dst, x, y, 2, 3, res.v[q]);
+        }
+    }
+}
+
+// Largest value of a warp's lanes, all non-negative (NaN loses): as unsigned
+// integers, high words first.
+__device__ __forceinline__ double warp_max(double v)
+{
+#if defined(__CUDA_ARCH__)
+    const unsigned long long b = v > 0.0 ? (unsigned long long)__double_as_longlong(v) : 0ull;
+    const unsigned hi = unsigned(b >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, hi == top ? unsigned(b) : 0u);
+    return __longlong_as_double((long long)((unsigned long long)top << 32 | lo));
+#else
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+#endif
 }
 
 // Ends a step in tiles (its last block): commits it as finish_step does, with
@@ -419,16 +462,12 @@ __device__ __forceinline__ void end_tile(double vmax, int bad, StepControl *ctl,
 {
     __shared__ double red[NT / 32];
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicCAS(&ctl->first_bad, 0, c.steps + 1);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-    if ((threadIdx.x & 31) == 0) {
-        red[threadIdx.x / 32] = vmax;
-        if (bad) __threadfence();
-    }
+    vmax = warp_max(vmax);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = vmax;
     __syncthreads();
+    if (threadIdx.x >= 32) return;
+    vmax = warp_max(threadIdx.x < NT / 32 ? red[threadIdx.x] : 0.0);
     if (threadIdx.x != 0) return;
-#pragma unroll
-    for (int w = 1; w < NT / 32; ++w) vmax = fmax(vmax, red[w]);
     if (vmax > 0.0) atomicMax(&ctl->smax_bits, (unsigned long long)__double_as_longlong(vmax));
     __threadfence();
     if (atomicAdd(&ctl->ticket, 1u) == nblocks - 1) {
@@ -456,8 +495,10 @@ __global__ void __launch_bounds__(T::NT, MINB) step_tile_kernel(TileArgs<Real> a
     double vmax = 0.0;
     int bad = 0;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
-    tile_step<Real, Phys, T>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, c.ring_due, c.t);
+    TileResults<Real, T> res;
+    tile_step<Real, Phys, T>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, res, c.ring_due, c.t);
     end_tile<T::NT>(vmax, bad, a.ctl, c, a.plan, gridDim.x * gridDim.y);
+    tile_store<Real, Phys, T>(a, blockIdx.x, blockIdx.y, res);
 }
 
 // A taped step, from src to dst whatever the parity; fill: the ring of src is
@@ -475,8 +516,10 @@ __global__ void __launch_bounds__(T::NT, MINB) step_tape_kernel(TileArgs<Real> a
     double vmax = 0.0;
     int bad = 0;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
-    tile_step<Real, Phys, T, true>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, fill != 0, c.t, &tape);
+    TileResults<Real, T> res;
+    tile_step<Real, Phys, T, true>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, res, fill != 0, c.t, &tape);
     end_tile<T::NT>(vmax, bad, a.ctl, c, a.plan, gridDim.x * gridDim.y);
+    tile_store<Real, Phys, T>(a, blockIdx.x, blockIdx.y, res);
 }
 
 // Stores the ghost ring after steps in tiles (src: the state if the parity
