@@ -36,6 +36,7 @@ struct BatchArgs {
     // steps in tiles: [np + 1] first tile of each problem (null: steps sweep by
     // sweep); a problem's state is in its region b while its parity is odd
     const long long *t0 = nullptr;
+    int step = 0;  // the step's place in its group (end_steps: the group's steps)
 };
 
 // Largest p with first[p] <= item (first[] ascending, first[0] = 0).
@@ -204,14 +205,13 @@ __global__ void __launch_bounds__(NT) batch_ghost_kernel(BatchArgs<Real> b)
 }
 
 #ifdef __CUDACC__
-// Problem p's arguments of a step in tiles, its state in src.
+// Problem p's arguments of a step in tiles from a state of parity `odd`.
 template <typename Real>
-__device__ __forceinline__ TileArgs<Real> batch_tile_args(const BatchArgs<Real> &b, int p)
+__device__ __forceinline__ TileArgs<Real> batch_tile_args(const BatchArgs<Real> &b, int p, int odd)
 {
     const BatchProblem &P = b.prob[p];
     TileArgs<Real> a;
     a.ctl = b.ctl + p;
-    const int odd = a.ctl->parity;
     a.src.base = b.base + (odd ? P.b : P.u);
     a.dst.base = b.base + (odd ? P.u : P.b);
     a.src.plane = a.dst.plane = P.plane;
@@ -236,33 +236,32 @@ __global__ void __launch_bounds__(T::NT, MINB) batch_tile_kernel(BatchArgs<Real>
     extern __shared__ __align__(16) unsigned char tile_smem[];
     pdl_launch();
     const int p = find_problem(b.t0, b.np, (long long)blockIdx.x);
-    StepControl *ctl = b.ctl + p;
     pdl_wait();
-    __shared__ StepControl c;
-    if (threadIdx.x == 0) c = *ctl;
-    __syncthreads();
-    if (!c.active) return;
-    const TileArgs<Real> a = batch_tile_args(b, p);
+    // a problem steps on every launch until its loop ends, so its parity as
+    // the group began gives the one now, without waiting for its last step's
+    const TileArgs<Real> a = batch_tile_args(b, p, (b.ctl[p].parity + b.step) & 1);
     const int ntx = (a.nx - 4 + T::TX - 1) / T::TX, k = int(blockIdx.x - b.t0[p]);
-    double vmax = 0.0;
+    double vmax = k == 0 && threadIdx.x == 0 ? ring_speed<Real>(a.strategy, a.gamma) : 0.0;
     int bad = 0;
-    if (k == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
-    TileResults<Real, T> res;
-    tile_step<Real, Phys, T>(a, c.dt, k % ntx, k / ntx, tile_smem, vmax, bad, res, c.ring_due, c.t);
-    end_tile<T::NT>(vmax, bad, ctl, c, a.plan, unsigned(b.t0[p + 1] - b.t0[p]));
-    tile_store<Real, Phys, T>(a, k % ntx, k / ntx, res);
+    if (tile_step<Real, Phys, T>(a, k % ntx, k / ntx, tile_smem,
+                                 [&] { return begin_tile(a.ctl, b.step & 1, a.plan, k == 0); }, b.step > 0, vmax, bad))
+        end_tile<T::NT>(vmax, bad, a.ctl, reinterpret_cast<TileHead<Real> *>(tile_smem)->step.steps);
 }
 
-// Stores the ghost rings after steps in tiles.
+// Ends a group of steps in tiles (end_steps_kernel).
 template <typename Real, int NT>
-__global__ void __launch_bounds__(NT) batch_fill_ring_kernel(BatchArgs<Real> b)
+__global__ void __launch_bounds__(NT) batch_end_steps_kernel(BatchArgs<Real> b)
 {
     pdl_launch();
     const int p = find_problem(b.rb0, b.np, int(blockIdx.x));
     pdl_wait();
-    if (!b.ctl[p].ring_due) return;
-    const int k = (int(blockIdx.x) - b.rb0[p]) * NT + threadIdx.x;
-    if (k < b.prob[p].ring) ghost_cell(ring_args(batch_tile_args(b, p)), k, b.ctl[p].t);
+    StepControl *const ctl = b.ctl + p;
+    const TileRecord r = fold_record(ctl, b.step & 1, b.prob[p].plan);
+    if (r.ring_due) {
+        const int k = (int(blockIdx.x) - b.rb0[p]) * NT + threadIdx.x;
+        if (k < b.prob[p].ring) ghost_cell(ring_args(batch_tile_args(b, p, r.parity)), k, r.t);
+    }
+    if (last_of_blocks(&ctl->ticket, unsigned(b.rb0[p + 1] - b.rb0[p]))) commit_record(ctl, r);
 }
 #endif
 
@@ -292,6 +291,7 @@ __global__ void __launch_bounds__(NT) batch_init_kernel(BatchArgs<Real> b)
         ctl->smax_bits = 0ull;
         ctl->ticket = 0u;
         plan_step(ctl, P.plan);
+        open_record(ctl);
     }
 }
 

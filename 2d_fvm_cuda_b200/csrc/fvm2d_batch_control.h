@@ -33,11 +33,12 @@ struct BatchLaunch {
     long long x_total, y_total;
     int ring_blocks, init_blocks;
     int grid_x, grid_y;        // sweep grids (blocks); 0 = all resident blocks
-    // steps in tiles of shape `tile_shape` (tile_cells of this build): [np + 1]
+    // steps in tiles of shape `tile_shape` (batch_tile_shape): [np + 1]
     // tile prefix counts; null: steps sweep by sweep
     const long long *t0;
     long long tile_total;
     int tile_shape;
+    int step;                  // the step's place in its group (for end_steps: the group's steps)
 };
 
 #define FVM2D_DECLARE_BATCH_VARIANT(ns)                                        \
@@ -46,7 +47,7 @@ struct BatchLaunch {
     cudaError_t batch_enqueue_init(const BatchLaunch &L, cudaStream_t s);      \
     cudaError_t batch_enqueue_plan(const BatchLaunch &L, cudaStream_t s);      \
     cudaError_t batch_enqueue_step(const BatchLaunch &L, cudaStream_t s);      \
-    cudaError_t batch_enqueue_fill_ring(const BatchLaunch &L, cudaStream_t s); \
+    cudaError_t batch_enqueue_end_steps(const BatchLaunch &L, cudaStream_t s); \
     /* the tile shape for problems of these sizes, and its tiles of one */     \
     int batch_tile_shape(int np, const int *nx, const int *ny);                \
     long long batch_tiles(int shape, int nx, int ny);                          \

@@ -12,7 +12,7 @@
 // that faster.)  Steps in tiles are enqueued up to 16 at a time (a launch costs
 // the host less than any step the device), sweeps as CUDA graphs of 16 steps
 // and 1 step, until no problem has a step in flight; after each group the
-// control records are read back (64 bytes per problem).  fvm2d_batch_autotune times
+// control records are read back (192 bytes per problem).  fvm2d_batch_autotune times
 // candidate y-segment lengths and sweep grid sizes on the batch itself and
 // keeps the fastest.
 //
@@ -60,23 +60,23 @@ struct BatchVariant {
     cudaError_t (*init)(const BatchLaunch &, cudaStream_t);
     cudaError_t (*plan)(const BatchLaunch &, cudaStream_t);
     cudaError_t (*step)(const BatchLaunch &, cudaStream_t);
-    cudaError_t (*fill_ring)(const BatchLaunch &, cudaStream_t);
+    cudaError_t (*end_steps)(const BatchLaunch &, cudaStream_t);
     int (*tile_shape)(int, const int *, const int *);
     long long (*tiles)(int, int, int);
 };
 
 const BatchVariant kBatchVariants[] = {
     {fvm2d::fp64::batch_prepare, fvm2d::fp64::batch_enqueue_init, fvm2d::fp64::batch_enqueue_plan,
-     fvm2d::fp64::batch_enqueue_step, fvm2d::fp64::batch_enqueue_fill_ring, fvm2d::fp64::batch_tile_shape, fvm2d::fp64::batch_tiles},
+     fvm2d::fp64::batch_enqueue_step, fvm2d::fp64::batch_enqueue_end_steps, fvm2d::fp64::batch_tile_shape, fvm2d::fp64::batch_tiles},
     {fvm2d::fp64_strict::batch_prepare, fvm2d::fp64_strict::batch_enqueue_init, fvm2d::fp64_strict::batch_enqueue_plan,
      fvm2d::fp64_strict::batch_enqueue_step,
-     fvm2d::fp64_strict::batch_enqueue_fill_ring, fvm2d::fp64_strict::batch_tile_shape, fvm2d::fp64_strict::batch_tiles},
+     fvm2d::fp64_strict::batch_enqueue_end_steps, fvm2d::fp64_strict::batch_tile_shape, fvm2d::fp64_strict::batch_tiles},
     {fvm2d::fp64_reforder::batch_prepare, fvm2d::fp64_reforder::batch_enqueue_init,
      fvm2d::fp64_reforder::batch_enqueue_plan, fvm2d::fp64_reforder::batch_enqueue_step,
-     fvm2d::fp64_reforder::batch_enqueue_fill_ring,
+     fvm2d::fp64_reforder::batch_enqueue_end_steps,
      fvm2d::fp64_reforder::batch_tile_shape, fvm2d::fp64_reforder::batch_tiles},
     {fvm2d::fp32::batch_prepare, fvm2d::fp32::batch_enqueue_init, fvm2d::fp32::batch_enqueue_plan,
-     fvm2d::fp32::batch_enqueue_step, fvm2d::fp32::batch_enqueue_fill_ring, fvm2d::fp32::batch_tile_shape, fvm2d::fp32::batch_tiles},
+     fvm2d::fp32::batch_enqueue_step, fvm2d::fp32::batch_enqueue_end_steps, fvm2d::fp32::batch_tile_shape, fvm2d::fp32::batch_tiles},
 };
 constexpr int kNumBatchVariants = sizeof(kBatchVariants) / sizeof(kBatchVariants[0]);
 
@@ -324,9 +324,10 @@ struct fvm2d_batch {
         for (;;) {
             if (use_tiles) {
                 const int n = (int)std::max(1ll, std::min(ahead, budget));
-                for (int k = 0; k < n; ++k) CK(kBatchVariants[precision].step(L, stream));
+                for (L.step = 0; L.step < n; ++L.step) CK(kBatchVariants[precision].step(L, stream));
+                CK(kBatchVariants[precision].end_steps(L, stream));
                 budget -= n;
-                launches += n;
+                launches += n + 1;
             } else {
                 const int which = budget >= kGraphSteps[0] ? 0 : 1;
                 CK(cudaGraphLaunch(graph[which], stream));
@@ -345,11 +346,8 @@ struct fvm2d_batch {
                 if (ctl_h[p].active) left = std::max(left, (t_end[p] - ctl_h[p].t) / ctl_h[p].dt);
             ahead = left < kGraphSteps[0] ? (long long)left + 1 : kGraphSteps[0];
         }
-        if (use_tiles) {
-            CK(kBatchVariants[precision].fill_ring(L, stream));
-            ++launches;
+        if (use_tiles)
             for (int p = 0; p < np; ++p) flip[p] = ctl_h[p].parity;
-        }
         CK(cudaEventRecord(ev1, stream));
         CK(cudaEventSynchronize(ev1));
         auto t1 = std::chrono::high_resolution_clock::now();

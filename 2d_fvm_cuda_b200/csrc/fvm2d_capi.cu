@@ -89,13 +89,13 @@ struct Variant {
     cudaError_t (*plan)(const LaunchConfig &, cudaStream_t);
     cudaError_t (*step)(const LaunchConfig &, cudaStream_t, cudaEvent_t *);       // in place, five kernels
     cudaError_t (*tile_step)(const LaunchConfig &, cudaStream_t);                 // pair[parity] to the other
-    cudaError_t (*fill_ring)(const LaunchConfig &, cudaStream_t);                 // after steps in tiles
+    cudaError_t (*end_steps)(const LaunchConfig &, cudaStream_t);                 // after a group of steps in tiles
     cudaError_t (*plan_from)(const LaunchConfig &, cudaStream_t, const double *);
 };
 
 #define FVM2D_VARIANT_ENTRY(ns)                                                                        \
     {fvm2d::ns::prepare, fvm2d::ns::enqueue_init, fvm2d::ns::enqueue_plan, fvm2d::ns::enqueue_step,     \
-     fvm2d::ns::enqueue_tile_step, fvm2d::ns::enqueue_fill_ring, fvm2d::ns::enqueue_plan_from}
+     fvm2d::ns::enqueue_tile_step, fvm2d::ns::enqueue_end_steps, fvm2d::ns::enqueue_plan_from}
 const Variant kVariants[] = {FVM2D_VARIANT_ENTRY(fp64), FVM2D_VARIANT_ENTRY(fp64_strict),
                              FVM2D_VARIANT_ENTRY(fp64_reforder), FVM2D_VARIANT_ENTRY(fp32),
                              FVM2D_VARIANT_ENTRY(fp32r)};
@@ -168,17 +168,11 @@ struct fvm2d_solver {
     double *scratch = nullptr;  // the other two: A then B
     StepControl *ctl = nullptr;
     StepControl *ctl_h = nullptr;  // pinned mirror
-    // replayed graphs: kGraphSteps[g] steps each; built on first use for the
-    // current precision and parameters, dropped by every setter
-    static constexpr int kGraphs = 3;
-    static constexpr int kGraphSteps[kGraphs] = {16, 4, 1};
     // steps enqueued between two reads of the control record, at most: a run
     // that ends early leaves up to that many empty steps
     static constexpr int kStepsPerRead = 128;
-    cudaGraphExec_t graph[kGraphs] = {};
-    cudaGraphExec_t slab_graph = nullptr;  // one step in place, for fvm2d_slab_step
+    cudaGraphExec_t slab_graph = nullptr;  // one step in place, for fvm2d_slab_step, dropped by every setter
     int slab_flip = 0;                     // the state's buffer it was captured with
-    int graph_variant = -1;
     bool have_state = false;
     bool need_init = true;
     double fixed_dt = 0.0;        // > 0: differentiation runs step with this constant dt
@@ -197,10 +191,9 @@ struct fvm2d_solver {
     int ck_count = 0, ck_len = 0, fwd_steps = -1, fwd_precision = -1;
     bool full_tape = false;       // the last fvm2d_forward kept every step's tape
     // the graphs of a full checkpoint segment: its taped recompute into tape
-    // buffer b ([b]), its reverse from tape buffer b ([2 + b]), and its untaped
-    // forward steps ([4], for fvm2d_forward); built for vjp_len steps and
-    // vjp_bufs tape buffers
-    cudaGraphExec_t vjp_graph[5] = {};
+    // buffer b ([b]) and its reverse from tape buffer b ([2 + b]); built for
+    // vjp_len steps and vjp_bufs tape buffers
+    cudaGraphExec_t vjp_graph[4] = {};
     int vjp_len = 0, vjp_bufs = 0;
     bool last_taped = false;      // the checkpointed forward taped its last segment (fvm2d_vjp skips its recompute)
     bool vjp_overlap = true;      // fvm2d_set_vjp_overlap: two tape buffers where they fit
@@ -228,10 +221,9 @@ struct fvm2d_solver {
     // (its halo rows pass through the sweeps, and its caller enqueues steps
     // without knowing whether the loop has ended).
     bool tiles() const { return ny_global == 0; }
-    cudaError_t enqueue_step(const LaunchConfig &c, cudaStream_t s) const;
-    // Stores the ghost ring that steps in tiles leave unfilled: after every
-    // group of steps whose state something else will read.
-    cudaError_t fill_ring(const LaunchConfig &c, cudaStream_t s) const;
+    // Enqueues n steps and, in tiles, their end (the record committed and the
+    // ghost ring stored): a group of steps.
+    int enqueue_steps(long long n, cudaEvent_t *ev = nullptr);
     int step_kernels() const { return tiles() ? 1 : fvm2d::kStepKernels; }
     // m steps were enqueued, all of which run
     void stepped(int m)
@@ -251,6 +243,7 @@ struct fvm2d_solver {
         c.B = scratch + 4 * plane;
         c.pair[0] = base;
         c.pair[1] = base + 8 * plane;
+        c.parity = flip;
         c.ctl = ctl;
         c.hx = width / double(nx);
         c.hy = height / double(ny_global > 0 ? ny_global : ny);  // a slab keeps the problem's row spacing
@@ -282,13 +275,8 @@ struct fvm2d_solver {
 
     void drop_graph()
     {
-        for (auto &g : graph) {
-            if (g) cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
         if (slab_graph) cudaGraphExecDestroy(slab_graph);
         slab_graph = nullptr;
-        graph_variant = -1;
         drop_vjp_graphs();
         discard_tape();
     }
@@ -325,21 +313,6 @@ struct fvm2d_solver {
         return FVM2D_OK;
     }
 
-    int build_graphs()
-    {
-        if (graph_variant == precision && graph[0] && graph[1] && graph[2]) return FVM2D_OK;
-        drop_graph();
-        const LaunchConfig c = config();
-        for (int which = 0; which < kGraphs; ++which)
-            if (int rc = capture(&graph[which], [&] {
-                    for (int k = 0; k < kGraphSteps[which]; ++k) CK(enqueue_step(c, stream));
-                    return FVM2D_OK;
-                }))
-                return rc;
-        graph_variant = precision;
-        return FVM2D_OK;
-    }
-
     int build_slab_graph()
     {
         if (slab_graph && slab_flip == flip) return FVM2D_OK;
@@ -353,36 +326,29 @@ struct fvm2d_solver {
         });
     }
 
-    // Enqueues n steps as graph replays.
-    int replay(long long n)
-    {
-        for (int which = 0; which < kGraphs; ++which)
-            for (; n >= kGraphSteps[which]; n -= kGraphSteps[which]) CK(cudaGraphLaunch(graph[which], stream));
-        return FVM2D_OK;
-    }
-
-    // Replays the step graphs until the control record says no step is in
+    // Enqueues groups of steps until the control record says no step is in
     // flight.  The record on the device must already be planned; `first`
     // kernels (init or plan) were enqueued just before.  `budget` bounds the
     // steps this loop may start.  The record is read after as many steps as
     // the run is known to have left: the budget, or the remaining time over
-    // the last step size, and at most kStepsPerRead.
+    // the last step size, and at most kStepsPerRead.  Steps are launched one
+    // by one: a launch takes the host 2 us and the smallest step the device
+    // 6, and the graphs that would stand for them cost a handle's first run
+    // 0.3 ms.
     int loop(int first, long long budget)
     {
-        int rc = build_graphs();
-        if (rc) return rc;
         auto t0 = std::chrono::high_resolution_clock::now();
         long long launches = first;
-        long long ahead = budget < LLONG_MAX ? kStepsPerRead : kGraphSteps[0];
+        long long ahead = budget < LLONG_MAX ? kStepsPerRead : 16;
         for (;;) {
             const long long n = std::max(1ll, std::min(ahead, budget));
-            if ((rc = replay(n))) return rc;
-            CK(fill_ring(config(), stream));
+            if (int rc = enqueue_steps(n)) return rc;
             budget -= n;
             launches += n * step_kernels() + tiles();
             CK(cudaEventRecord(ev_end, stream));
             CK(cudaMemcpyAsync(ctl_h, ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, stream));
             CK(cudaStreamSynchronize(stream));
+            if (tiles()) set_flip(ctl_h->parity);
             if (!ctl_h->active) break;
             ahead = kStepsPerRead;
             if (fixed_dt == 0.0) {
@@ -390,7 +356,6 @@ struct fvm2d_solver {
                 if (left < kStepsPerRead) ahead = (long long)left + 1;
             }
         }
-        if (tiles()) set_flip(ctl_h->parity);
         auto t1 = std::chrono::high_resolution_clock::now();
         last_ms = std::chrono::duration_cast<std::chrono::microseconds>(t1 - t0).count() / 1000.0;
         float dms = 0.f;
@@ -404,21 +369,27 @@ struct fvm2d_solver {
     int upload_control(int parity)
     {
         ctl_h->parity = parity;
-        ctl_h->ring_due = 0;
+        open_record(ctl_h);
         CK(cudaMemcpyAsync(ctl, ctl_h, sizeof(StepControl), cudaMemcpyHostToDevice, stream));
         return FVM2D_OK;
     }
 };
 
-cudaError_t fvm2d_solver::enqueue_step(const LaunchConfig &c, cudaStream_t s) const
+int fvm2d_solver::enqueue_steps(long long n, cudaEvent_t *ev)
 {
     const Variant &v = kVariants[precision];
-    return tiles() ? v.tile_step(c, s) : v.step(c, s, nullptr);
-}
-
-cudaError_t fvm2d_solver::fill_ring(const LaunchConfig &c, cudaStream_t s) const
-{
-    return tiles() ? kVariants[precision].fill_ring(c, s) : cudaSuccess;
+    LaunchConfig c = config();
+    if (!tiles()) {
+        for (long long k = 0; k < n; ++k) CK(v.step(c, stream, ev));
+        return FVM2D_OK;
+    }
+    if (ev)
+        for (int q = 0; q < 4; ++q) CK(cudaEventRecord(ev[q], stream));
+    for (; c.step < n; ++c.step) CK(v.tile_step(c, stream));
+    if (ev) CK(cudaEventRecord(ev[4], stream));
+    CK(v.end_steps(c, stream));
+    if (ev) CK(cudaEventRecord(ev[5], stream));
+    return FVM2D_OK;
 }
 
 namespace {
@@ -736,7 +707,6 @@ int fvm2d_solve(fvm2d_solver *s)
     std::memset(c, 0, sizeof(StepControl));
     c->step_limit = INT_MAX;
     const LaunchConfig cfg = s->config();
-    if (int rc = s->build_graphs()) return rc;
     if (s->record_on) {
         if (int rc = solve_recording(s)) return rc;
         s->total_steps += c->steps;
@@ -765,7 +735,6 @@ int fvm2d_advance(fvm2d_solver *s, int nsteps, int *steps_done)
     c->active = 0;
     if (int rc = s->upload_control()) return rc;
     const LaunchConfig cfg = s->config();
-    if (int rc = s->build_graphs()) return rc;
     CK(cudaEventRecord(s->ev_begin, s->stream));
     if (s->need_init) {
         CK(kVariants[s->precision].init(cfg, s->stream));
@@ -786,7 +755,6 @@ int fvm2d_advance_dt(fvm2d_solver *s, double dt)
     if (!s->have_state) return fail(FVM2D_ERR_STATE, "no state has been set");
     if (!(dt > 0.0) || !std::isfinite(dt)) return fail(FVM2D_ERR_INVALID, "dt must be positive and finite");
     const LaunchConfig cfg = s->config();
-    if (int rc = s->build_graphs()) return rc;
     StepControl *c = s->ctl_h;
     if (s->need_init) {  // wave-speed max of the fresh state; the device record becomes the reference
         CK(kVariants[s->precision].init(cfg, s->stream));
@@ -800,8 +768,7 @@ int fvm2d_advance_dt(fvm2d_solver *s, double dt)
     c->step_limit = c->steps + 1;
     if (int rc = s->upload_control()) return rc;
     CK(cudaEventRecord(s->ev_begin, s->stream));
-    if (int rc = s->replay(1)) return rc;
-    CK(s->fill_ring(cfg, s->stream));
+    if (int rc = s->enqueue_steps(1)) return rc;
     CK(cudaMemcpyAsync(c, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaEventRecord(s->ev_end, s->stream));
     CK(cudaEventSynchronize(s->ev_end));
@@ -937,7 +904,6 @@ int fvm2d_slab_begin(fvm2d_solver *s, double *smax_out)
     std::memset(c, 0, sizeof(StepControl));
     c->step_limit = INT_MAX;
     if (int rc = s->upload_control()) return rc;
-    if (int rc = s->build_graphs()) return rc;
     if (int rc = s->build_slab_graph()) return rc;
     CK(kVariants[s->precision].init(s->config(), s->stream));
     s->need_init = false;
@@ -951,7 +917,7 @@ int fvm2d_slab_step(fvm2d_solver *s, const double *smax_in, double *smax_out)
     if (!s->have_state) return fail(FVM2D_ERR_STATE, "no state has been set");
     if (!smax_in || !smax_out || !is_device_pointer(smax_in) || !is_device_pointer(smax_out))
         return fail(FVM2D_ERR_INVALID, "smax_in and smax_out must be device memory");
-    if (s->graph_variant != s->precision || !s->slab_graph)
+    if (!s->slab_graph)
         return fail(FVM2D_ERR_STATE, "fvm2d_slab_begin must come first (and again after a setter)");
     if (int rc = s->build_slab_graph()) return rc;  // again if steps since then left the state in the other buffer
     CK(kVariants[s->precision].plan_from(s->config(), s->stream, smax_in));
@@ -1148,15 +1114,7 @@ int fvm2d_profile_kernels(fvm2d_solver *s, int nsteps, double *kernel_ms, int *s
         if ((rc = s->upload_control())) break;
         e = s->need_init ? kVariants[s->precision].init(cfg, s->stream) : kVariants[s->precision].plan(cfg, s->stream);
         s->need_init = false;
-        if (!e && s->tiles()) {
-            for (int q = 0; q < 4; ++q) cudaEventRecord(ev[q], s->stream);
-            e = s->enqueue_step(cfg, s->stream);
-            cudaEventRecord(ev[4], s->stream);
-            if (!e) e = s->fill_ring(cfg, s->stream);
-            cudaEventRecord(ev[5], s->stream);
-        } else if (!e) {
-            e = kVariants[s->precision].step(cfg, s->stream, ev);
-        }
+        if (!e && (rc = s->enqueue_steps(1, ev))) break;
         if (!e) e = cudaMemcpyAsync(c, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream);
         if (!e) e = cudaStreamSynchronize(s->stream);
         if (e) { rc = cuda_fail(e, "profiled step"); break; }
@@ -1285,8 +1243,10 @@ int fvm2d_jvp(fvm2d_solver *s, int nsteps, const double *tangent_in, double *tan
     h->active = 0;
     if (int rc = s->upload_control(0)) return rc;
     CK(kJvp.init(c, s->stream));
-    for (int k = 0; k < nsteps; ++k) CK(s->tiles() ? kJvp.tile_step(c, s->stream) : kJvp.step(c, s->stream, nullptr));
-    if (s->tiles()) CK(kJvp.fill_ring(c, s->stream));
+    c.parity = 0;
+    for (; c.step < nsteps; ++c.step)
+        CK(s->tiles() ? kJvp.tile_step(c, s->stream) : kJvp.step(c, s->stream, nullptr));
+    if (s->tiles()) CK(kJvp.end_steps(c, s->stream));
     CK(cudaMemcpyAsync(h, s->ctl, sizeof(StepControl), cudaMemcpyDeviceToHost, s->stream));
     unpack_dual<<<148 * 4, 256, 0, s->stream>>>(s->tiles() && (nsteps & 1) ? dB : dU, s->U, T, n4);
     CK(cudaGetLastError());
@@ -1318,6 +1278,7 @@ static int taped_steps(fvm2d_solver *s, const LaunchConfig &c, int m, int buf, c
     auto sweep_step = f32 ? fvm2d::fp32::enqueue_step_taped : fvm2d::fp64::enqueue_step_taped;
     for (int j = 0; j < m; ++j) {
         LaunchConfig cj = c;
+        cj.step = j;
         cj.U = tape_at(s, buf, j, 0, sb);
         cj.A = tape_at(s, buf, j, 1, sb);
         cj.B = tape_at(s, buf, j, 2, sb);
@@ -1326,13 +1287,15 @@ static int taped_steps(fvm2d_solver *s, const LaunchConfig &c, int m, int buf, c
         void *const out =
             j + 1 < m ? static_cast<void *>(tape_at(s, buf, j + 1, 0, sb)) : static_cast<void *>(s->base);
         if (s->tiles())
-            CK(tile_step(cj, st, flux, out, j > 0));
+            CK(tile_step(cj, st, flux, out));
         else
             CK(sweep_step(cj, st, flux, out));
     }
+    if (!s->tiles()) return FVM2D_OK;
     LaunchConfig last = c;
+    last.step = m;
     last.pair[0] = last.pair[1] = s->base;
-    CK(s->fill_ring(last, st));
+    CK(kVariants[s->precision].end_steps(last, st));
     return FVM2D_OK;
 }
 
@@ -1355,7 +1318,7 @@ __global__ void segment_control(StepControl *c, double t, double dt)
         c->ticket = 0u;
         c->first_bad = 0;
         c->parity = 0;
-        c->ring_due = 0;
+        open_record(c);
     }
 }
 
@@ -1379,7 +1342,6 @@ static int forward_full_tape(fvm2d_solver *s, int nsteps)
     bool grew;
     if (int rc = ensure(s->tape, s->tape_bytes, need, grew)) return rc;
     if (grew) s->drop_vjp_graphs();
-    if (int rc = s->build_graphs()) return rc;  // as fvm2d_forward, so a later advance keeps the tape
     StepControl *h = s->ctl_h;
     h->step_limit = INT_MAX;
     h->done = 0;
@@ -1493,11 +1455,6 @@ static int vjp_workspace(fvm2d_solver *s, int *bufs)
         s->drop_vjp_graphs();
         const LaunchConfig c = s->config();
         const int len = s->ck_len;
-        if (int rc = s->capture(&s->vjp_graph[4], [&] {
-                for (int j = 0; j < len; ++j) CK(s->enqueue_step(c, s->stream));
-                return FVM2D_OK;
-            }))
-            return rc;
         for (int b = 0; b < *bufs; ++b) {
             if (int rc = s->capture(&s->vjp_graph[b], [&] { return taped_steps(s, c, len, b, s->stream); }))
                 return rc;
@@ -1523,7 +1480,6 @@ int fvm2d_forward(fvm2d_solver *s, int nsteps, int checkpoints)
     const size_t sb = state_bytes_of(s);
     bool grew;
     if (int rc = ensure(s->ckpt, s->ck_bytes, (size_t)count * sb, grew)) return rc;
-    if (int rc = s->build_graphs()) return rc;  // the step graphs of the fixed-dt build
     s->fwd_steps = -1;
     s->full_tape = false;
     s->last_taped = false;
@@ -1558,12 +1514,7 @@ int fvm2d_forward(fvm2d_solver *s, int nsteps, int checkpoints)
             }
             s->set_flip(0);
         } else {
-            if (count > 1 && m == s->vjp_len) {  // a full segment: one graph of its steps
-                CK(cudaGraphLaunch(s->vjp_graph[4], s->stream));
-            } else if (int rc = s->replay(m)) {
-                return rc;
-            }
-            CK(s->fill_ring(c, s->stream));
+            if (int rc = s->enqueue_steps(m)) return rc;
             s->stepped(m);
         }
         for (int q = 0; q < m; ++q) t = t + s->fixed_dt;  // as the device adds

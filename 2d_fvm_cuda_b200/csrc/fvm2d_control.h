@@ -5,6 +5,18 @@
 
 namespace fvm2d {
 
+// What a step in tiles hands the next one: the loop as that step began and,
+// while `pending`, its own commit (t + dt, steps + 1, its wave-speed maximum)
+// and the next plan, which the next kernel makes for itself (fold_record).
+struct TileRecord {
+    double t, dt, smax_last;
+    int steps, active, done;
+    int pending;   // 1: the step of size dt has run and is not committed here
+    int parity;    // which of the two state buffers holds the state
+    int ring_due;  // 1: that state's ghost ring in memory is not filled (steps in
+                   // tiles compute the ring cells they load; the end of a group stores them)
+};
+
 // Device-resident loop state, one per solver handle.  The kernels of a step
 // read the step size from it and the step's last kernel advances it, so the
 // time loop of src/wrappers.cuh:196-284 runs without a host round trip.
@@ -21,9 +33,30 @@ struct StepControl {
     int first_bad;                 // 1-based step that first left an interior cell with NaN or
                                    // non-positive density or pressure; 0: none
     int parity;                    // steps in tiles: which of the two state buffers holds the state
-    int ring_due;                  // 1: the state's ghost ring in memory is not filled yet (steps in
-                                   // tiles fill the ring cells they load; fill_ring stores them)
+    // Steps in tiles, between the record as planned (open_record) and the end
+    // of their group (end_steps): step k of a group reads rec[k % 2] and writes
+    // rec[(k + 1) % 2]; a step from n committed steps gathers its wave-speed
+    // maximum in smax[(n + 1) % 4] and clears smax[(n + 2) % 4].
+    TileRecord rec[2];
+    unsigned long long smax[4];
 };
+
+// Begins a group of steps in tiles at the record as it stands.
+__host__ __device__ inline void open_record(StepControl *c)
+{
+    TileRecord r;
+    r.t = c->t;
+    r.dt = c->dt;
+    r.smax_last = c->smax_last;
+    r.steps = c->steps;
+    r.active = c->active;
+    r.done = c->done;
+    r.pending = 0;
+    r.parity = c->parity;
+    r.ring_due = 0;
+    c->rec[0] = c->rec[1] = r;
+    for (int k = 0; k < 4; ++k) c->smax[k] = 0ull;
+}
 
 struct PlanParams {
     double t_end;     // end time
@@ -37,8 +70,11 @@ struct LaunchConfig {
     int nx, ny, pitch;
     long long plane;       // elements between field planes
     void *U, *A, *B;       // state buffers: U holds the state, A and B are sweep scratch
-    void *pair[2] = {nullptr, nullptr};  // steps in tiles go from pair[parity] to pair[1 - parity]
-                                         // (parity: the control record's), so neither is swept in place
+    // steps in tiles: the two state buffers a step goes from one to the other
+    // of, the one (0, 1) that holds the state as the group of steps begins,
+    // and the step's place in its group (for end_steps: the group's steps)
+    void *pair[2] = {nullptr, nullptr};
+    int parity = 0, step = 0;
     StepControl *ctl;
     double hx, hy;         // width/nx, height/ny
     double rhx, rhy;       // 1.0/hx, 1.0/hy
@@ -54,8 +90,8 @@ struct LaunchConfig {
 };
 
 // Kernels per step: sweep X, sweep Y, sweep Y, sweep X + average, ghost ring.
-// A step in tiles is one kernel, and one more stores the ghost ring after a
-// group of them.
+// A step in tiles is one kernel, and one more commits a group of them and
+// stores the ghost ring.
 constexpr int kStepKernels = 5;
 
 // x-sweep work items: a warp walks `chunks` chunks of 32 cells of one row and
@@ -86,7 +122,7 @@ inline int x_chunks_for(long long rows, int nx, long long resident_warps)
     cudaError_t enqueue_plan_from(const LaunchConfig &c, cudaStream_t s, const double *smax); \
     cudaError_t enqueue_step(const LaunchConfig &c, cudaStream_t s, cudaEvent_t *ev); \
     cudaError_t enqueue_tile_step(const LaunchConfig &c, cudaStream_t s);      \
-    cudaError_t enqueue_fill_ring(const LaunchConfig &c, cudaStream_t s);      \
+    cudaError_t enqueue_end_steps(const LaunchConfig &c, cudaStream_t s);      \
     }
 
 FVM2D_DECLARE_VARIANT(fp64)
@@ -101,13 +137,12 @@ FVM2D_DECLARE_VARIANT(jvp)
 // X of B), each stored at the interface's right cell in planes mass, normal
 // momentum, energy, tangential momentum.  The step reads c.U and writes its
 // result to `out`.  In tiles (whole problems) the result's ghost ring is left
-// to the next taped step, which fills it (`fill`) as it loads it, or to
-// enqueue_fill_ring; the step sweep by sweep is for row slabs.
+// to the next taped step of its group, which fills it as it loads it, or to
+// enqueue_end_steps; the step sweep by sweep is for row slabs.
 #define FVM2D_DECLARE_TAPED(ns)                                                                             \
     namespace ns {                                                                                          \
     cudaError_t enqueue_step_taped(const LaunchConfig &c, cudaStream_t s, void *const flux[4], void *out);  \
-    cudaError_t enqueue_tile_step_taped(const LaunchConfig &c, cudaStream_t s, void *const flux[4], void *out, \
-                                        bool fill);                                                         \
+    cudaError_t enqueue_tile_step_taped(const LaunchConfig &c, cudaStream_t s, void *const flux[4], void *out); \
     }
 
 FVM2D_DECLARE_TAPED(fp64)

@@ -37,11 +37,12 @@ namespace FVM2D_VARIANT {
 // dt = min(CFL h / smax, t_end - t); stop when t >= t_end or h/smax < 1e-20.
 // With a fixed step size (differentiation runs) dt is that constant and only
 // the step limit ends the loop.
-__device__ __forceinline__ void plan_step(StepControl *c, const PlanParams &p)
+template <class Record>
+__device__ __forceinline__ void plan_step(Record *c, int step_limit, const PlanParams &p)
 {
     c->active = 0;
     if (c->done) return;
-    if (c->steps >= c->step_limit) return;
+    if (c->steps >= step_limit) return;
     if (p.fixed_dt > 0.0) {  // differentiation runs: a constant step size, bounded by the step count only
         c->dt = p.fixed_dt;
         c->active = 1;
@@ -63,9 +64,14 @@ __device__ __forceinline__ void plan_step(StepControl *c, const PlanParams &p)
     c->active = 1;
 }
 
+__device__ __forceinline__ void plan_step(StepControl *c, const PlanParams &p) { plan_step(c, c->step_limit, p); }
+
 __global__ void plan_kernel(StepControl *c, PlanParams p)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) plan_step(c, p);
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        plan_step(c, p);
+        open_record(c);
+    }
 }
 
 // A row slab of a problem split across devices plans its step from the
@@ -190,6 +196,7 @@ __global__ void __launch_bounds__(NT) init_kernel(Field<Real> U, int nx, int ny,
         ctl->smax_bits = 0ull;
         ctl->ticket = 0u;
         plan_step(ctl, p);
+        open_record(ctl);
     }
 }
 

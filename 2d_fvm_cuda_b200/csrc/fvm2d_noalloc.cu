@@ -72,7 +72,6 @@ __global__ void reset_control(fvm2d::StepControl *c, double t0, int nsteps)
     c->ticket = 0u;
     c->first_bad = 0;
     c->parity = 0;
-    c->ring_due = 0;
 }
 
 // Once per device, with that device current: the device address of
@@ -172,14 +171,15 @@ int fvm2d_advance_noalloc(const double *state_in, double *state_out, int nx, int
     int queued = 0;
     do {
         const int n = (nsteps - queued < kStepsPerCheck) ? nsteps - queued : kStepsPerCheck;
-        for (int k = 0; k < n; ++k)
+        for (c.step = 0; c.step < n; ++c.step)
             if ((e = fvm2d::fp64::enqueue_tile_step(c, s))) return cuda_fail(e, "step kernels");
+        if ((e = fvm2d::fp64::enqueue_end_steps(c, s))) return cuda_fail(e, "end of the steps");
         queued += n;
         if ((e = cudaMemcpyAsync(&out, c.ctl, sizeof(out), cudaMemcpyDeviceToHost, s)))
             return cuda_fail(e, "control read");
         if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "cudaStreamSynchronize");
+        c.parity = out.parity;
     } while (out.active && queued < nsteps);
-    if ((e = fvm2d::fp64::enqueue_fill_ring(c, s))) return cuda_fail(e, "ghost ring");
     if (out.parity) {  // an odd number of steps: the result is in the scratch
         if ((e = cudaMemcpyAsync(state_out, c.A, sizeof(double) * 4 * plane, cudaMemcpyDeviceToDevice, s)))
             return cuda_fail(e, "copy of the result");

@@ -65,10 +65,23 @@ __device__ __forceinline__ Real alpha_rh(const TileConsts<Real> &K) { return K.r
 template <typename Real>
 __device__ __forceinline__ Real half_k(const TileConsts<Real> &K) { return K.hk; }
 
+// The step a block runs, from its control record.
+struct TileStep {
+    double t, dt;
+    int active, steps;  // steps committed before it
+};
+
+// What comes first in a block's shared memory.
+template <typename Real>
+struct TileHead {
+    TileConsts<Real> K[2];  // along x, along y
+    TileStep step;
+    double pad;
+};
+
 template <typename Real>
 struct TileArgs {
-    Field<Real> src, dst;  // state read and state written (different buffers); the other way round
-                           // if the control record's parity is odd
+    Field<Real> src, dst;  // state read and state written (different buffers)
     int nx, ny;
     double hx, hy, rhx, rhy;
     double alpha, gamma;
@@ -154,7 +167,7 @@ struct Tile {
     template <typename Real, class Phys>
     static constexpr size_t bytes()
     {
-        return 2 * sizeof(TileConsts<Real>) + (kElems + 1) / 2 * 2 * sizeof(Real) +
+        return sizeof(TileHead<Real>) + (kElems + 1) / 2 * 2 * sizeof(Real) +
                (split_storage<Phys>::value ? kLoWords * sizeof(unsigned long long) : 0);
     }
 };
@@ -168,28 +181,33 @@ __device__ __forceinline__ void tile_copy(Real *dst_shared, const Real *src)
         *dst_shared = *src;
 }
 
-// Results of a merged tile a thread holds until it stores them (tile_store).
-template <typename Real, class T>
-struct TileResults {
-    static constexpr int N = (T::TX * T::TY + T::NT - 1) / T::NT;
-    Cell<Real> v[N];
-};
+// Do the presets' ring values depend on time?  (row_rule: the rows above a
+// double Mach reflection)
+__device__ __forceinline__ bool ring_timed(int strategy)
+{
+    return !(strategy == OUTFLOW || strategy == PERIODIC || strategy == REFLECTIVE_TB || strategy == JET ||
+             strategy == JET800);
+}
 
-// One step of tile (bx, by), by the Tile::NT threads of a block; fill: the
-// state's ring cells are computed for time t, else read.  TAPE: the step also
-// writes its tape (and the ring it fills, into the state it reads).
-template <typename Real, class Phys, class T, bool TAPE = false>
-__device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, int bx, int by, unsigned char *smem,
-                                          double &vmax, int &bad, TileResults<Real, T> &res, bool fill = false,
-                                          double t = 0.0, const TapeArgs<Real> *tape = nullptr)
+// One step of tile (bx, by), by the Tile::NT threads of a block; false, and
+// nothing written, if there is none to run.  begin(): the step, called by the
+// last warp while the copies of the tile are under way (the record's loads
+// and the plan's divisions then cost a step nothing), or before them where
+// ring cells depend on its time.  fill: the state's ring cells are computed,
+// else read.  TAPE: the step also writes its tape (and the ring it fills,
+// into the state it reads).
+template <typename Real, class Phys, class T, bool TAPE = false, class Begin>
+__device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int by, unsigned char *smem, Begin &&begin,
+                                          bool fill, double &vmax, int &bad, const TapeArgs<Real> *tape = nullptr)
 {
     constexpr bool kResidual = split_storage<Phys>::value;
     using Word = unsigned long long;
     constexpr int NC = T::NC, RS = T::RS;
     // (a residual build's branch B is averaged before it is split)
     constexpr bool MERGE = T::kMerge && !kResidual;
-    TileConsts<Real> *const KK = reinterpret_cast<TileConsts<Real> *>(smem);
-    Real *const sU = reinterpret_cast<Real *>(KK + 2);
+    TileHead<Real> *const head = reinterpret_cast<TileHead<Real> *>(smem);
+    TileConsts<Real> *const KK = head->K;
+    Real *const sU = reinterpret_cast<Real *>(head + 1);
     Real *const sA = sU + T::NR * RS;
     Real *const sB = sA + (T::NR - 2) * RS;  // rows 2 .. TY+1 of B1 (rows 0, 1 are not kept)
     Real *const sR = sB + T::TY * RS;        // the same rows of RB
@@ -205,6 +223,31 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
     auto owns_x = [&](int x) { return (x >= x0 || bx == 0) && (x < x0 + T::TX || last_x); };
     auto owns_y = [&](int y) { return (y >= y0 || by == 0) && (y < y0 + T::TY || last_y); };
     const Cell<Real> none = {Real(0), Real(0), Real(0), Real(0)};
+    auto start = [&] {
+        const TileStep now = begin();
+        if (lane == 0) head->step = now;
+        if (lane >= 2) return;
+        TileConsts<Real> K;
+        const double h = lane == 0 ? a.hx : a.hy;
+        K.h = Real(h);
+        K.rh = Real(lane == 0 ? a.rhx : a.rhy);
+        K.alpha = Real(a.alpha);
+        set_gamma_consts(K, a.gamma);
+        K.k = Real(now.dt);
+        K.lambda = Real(now.dt / h);
+        K.lambda_lo = Real(lo_part<Real>(now.dt / h));
+        K.hh = K.h * Real(0.5);
+        K.hrh = K.rh * Real(0.5);
+        K.rha = K.rh * K.alpha;
+        K.hk = K.k * Real(0.5);
+        KK[lane] = K;
+    };
+    const bool timed = fill && by == 0 && ring_timed(a.strategy);
+    if (timed) {
+        if (warp == T::NW - 1) start();
+        __syncthreads();
+    }
+    const double t = timed ? head->step.t : 0.0;
     // does the loaded tile reach the ring?
     const bool edge = fill && (bx == 0 || by == 0 || x0 - 2 + NC > a.nx - 2 || y0 - 2 + T::NR > a.ny - 2);
     for (int i = tid; i < T::NR * NC; i += T::NT) {
@@ -229,24 +272,10 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
         if constexpr (kResidual) async_copy(lU + r * T::kLo + c, &lo_cell(a.src, x, y));
     }
     async_commit();
-    if (tid < 2) {
-        TileConsts<Real> K;
-        const double h = tid == 0 ? a.hx : a.hy;
-        K.h = Real(h);
-        K.rh = Real(tid == 0 ? a.rhx : a.rhy);
-        K.alpha = Real(a.alpha);
-        set_gamma_consts(K, a.gamma);
-        K.k = Real(dt);
-        K.lambda = Real(dt / h);
-        K.lambda_lo = Real(lo_part<Real>(dt / h));
-        K.hh = K.h * Real(0.5);
-        K.hrh = K.rh * Real(0.5);
-        K.rha = K.rh * K.alpha;
-        K.hk = K.k * Real(0.5);
-        KK[tid] = K;
-    }
+    if (!timed && warp == T::NW - 1) start();
     async_wait<0>();
     __syncthreads();
+    if (!head->step.active) return false;
     if constexpr (TAPE) {  // the ring's part: sweeps across it pass its cells through
         for (int i = tid; i < T::NR * NC; i += T::NT) {
             const int r = i / NC, c = i - r * NC, x = x0 - 2 + c, y = y0 - 2 + r;
@@ -272,30 +301,25 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
     };
     // the step's result at tile cell (r, c): branch A (sU, lU) averaged with
     // branch B in primitive variables (src/basicFuns.cuh:264-274)
-    auto average = [&](int r, int c, const Cell<Real> &b) {
-        const Real *const ra = sU + r * RS + c;
-        const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
-        return Cell<Real>{(A.rho + b.rho) * Real(0.5), (A.p + b.p) * Real(0.5), (A.un + b.un) * Real(0.5),
-                          (A.ut + b.ut) * Real(0.5)};
-    };
-    auto note = [&](const Cell<Real> &o) {
-        vmax = fmax(vmax, wave_speed(o.rho, o.p, o.un, o.ut, a.gamma));
-        bad |= !(o.rho > Real(0) && o.p > Real(0));  // NaN fails both tests
-    };
     auto finish = [&](int r, int c, auto b) {
         const int x = x0 - 2 + c, y = y0 - 2 + r;
+        const Real *const ra = sU + r * RS + c;
+        const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
+        Cell<Real> o;
         if constexpr (kResidual) {
-            const Real *const ra = sU + r * RS + c;
-            const Cell<double> d = join_cell(Cell<Real>{ra[0], ra[NC], ra[2 * NC], ra[3 * NC]},
-                                             parts(lU[r * T::kLo + c], 2, 3));
-            note(store_split(a.dst, x, y, 2, 3,
-                             Cell<double>{(d.rho + b.rho) * 0.5, (d.p + b.p) * 0.5, (d.un + b.un) * 0.5,
-                                          (d.ut + b.ut) * 0.5}));
+            const Cell<double> d = join_cell(A, parts(lU[r * T::kLo + c], 2, 3));
+            o = store_split(a.dst, x, y, 2, 3,
+                            Cell<double>{(d.rho + b.rho) * 0.5, (d.p + b.p) * 0.5, (d.un + b.un) * 0.5,
+                                         (d.ut + b.ut) * 0.5});
         } else {
-            const Cell<Real> o = average(r, c, b);
+            o.rho = (A.rho + b.rho) * Real(0.5);
+            o.p = (A.p + b.p) * Real(0.5);
+            o.un = (A.un + b.un) * Real(0.5);
+            o.ut = (A.ut + b.ut) * Real(0.5);
             store_cell(a.dst, x, y, 2, 3, o);
-            note(o);
         }
+        vmax = fmax(vmax, wave_speed(o.rho, o.p, o.un, o.ut, a.gamma));
+        bad |= !(o.rho > Real(0) && o.p > Real(0));  // NaN fails both tests
     };
 
     // tasks along x and along y of the two sweeps of each branch
@@ -390,31 +414,14 @@ __device__ __forceinline__ void tile_step(const TileArgs<Real> &a, double dt, in
         __syncthreads();
     }
     if constexpr (MERGE) {
-#pragma unroll
-        for (int q = 0; q < TileResults<Real, T>::N; ++q) {
-            const int i = tid + q * T::NT, r = 2 + i / T::TX, c = 2 + i % T::TX;
-            if (i >= T::TX * T::TY || c >= ncol - 2 || r >= nrow - 2) continue;
+        for (int i = tid; i < T::TX * T::TY; i += T::NT) {
+            const int r = 2 + i / T::TX, c = 2 + i % T::TX;
+            if (c >= ncol - 2 || r >= nrow - 2) continue;
             const Real *const rb = sR + r * RS + c;
-            res.v[q] = average(r, c, Cell<Real>{rb[0], rb[NC], rb[2 * NC], rb[3 * NC]});
-            note(res.v[q]);
+            finish(r, c, Cell<Real>{rb[0], rb[NC], rb[2 * NC], rb[3 * NC]});
         }
     }
-}
-
-// Stores the results of a merged tile.  They come after the block's maximum
-// and ticket: nothing in the step waits for them, and a fence issued behind
-// them would.
-template <typename Real, class Phys, class T>
-__device__ __forceinline__ void tile_store(const TileArgs<Real> &a, int bx, int by, const TileResults<Real, T> &res)
-{
-    if constexpr (T::kMerge && !split_storage<Phys>::value) {
-        const int x0 = 2 + bx * T::TX, y0 = 2 + by * T::TY;
-#pragma unroll
-        for (int q = 0; q < TileResults<Real, T>::N; ++q) {
-            const int i = threadIdx.x + q * T::NT, x = x0 + i % T::TX, y = y0 + i / T::TX;
-            if (i < T::TX * T::TY && x <= a.nx - 3 && y <= a.ny - 3) store_cell(a.dst, x, y, 2, 3, res.v[q]);
-        }
-    }
+    return true;
 }
 
 // Largest value of a warp's lanes, all non-negative (NaN loses): as unsigned
@@ -432,109 +439,126 @@ __device__ __forceinline__ double warp_max(double v)
 #endif
 }
 
-// Ends a step in tiles (its last block): commits it as finish_step does, with
-// the state now in the other buffer and its ring unfilled.  `c` is the record
-// as the step began, of which a step changes nothing but smax_bits, ticket
-// and first_bad, so the only value waited for is the maximum.
-__device__ __forceinline__ void finish_tile_step(StepControl *ctl, StepControl c, const PlanParams &plan)
+// The record of the step in place `slot` (0, 1) of a group, with the step
+// before it committed and the next one planned as finish_step does.  Every
+// block of a step makes it for itself, the whole warp alike.  (Of smax a
+// value being gathered or cleared is read as well, and not used.)
+__device__ __forceinline__ TileRecord fold_record(const StepControl *ctl, int slot, const PlanParams &plan)
 {
-    c.smax_last = __longlong_as_double((long long)*(volatile unsigned long long *)&ctl->smax_bits);
-    ctl->smax_bits = 0ull;
-    c.t = c.t + c.dt;
-    c.steps += 1;
-    plan_step(&c, plan);
-    ctl->ticket = 0u;
-    ctl->t = c.t;
-    ctl->dt = c.dt;
-    ctl->smax_last = c.smax_last;
-    ctl->steps = c.steps;
-    ctl->active = c.active;
-    ctl->done = c.done;
-    ctl->parity = c.parity ^ 1;
-    ctl->ring_due = 1;
+    TileRecord r = ctl->rec[slot];
+    unsigned long long m[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) m[k] = ctl->smax[k];
+    const int limit = ctl->step_limit;
+    if (r.pending) {
+        const int k = (r.steps + 1) & 3;
+        r.smax_last = __longlong_as_double((long long)(k < 2 ? (k ? m[1] : m[0]) : (k == 2 ? m[2] : m[3])));
+        r.t = r.t + r.dt;
+        r.steps += 1;
+        r.pending = 0;
+        r.parity ^= 1;
+        r.ring_due = 1;
+        plan_step(&r, limit, plan);
+    }
+    return r;
 }
 
-// Folds the block's maxima into the record and ends the step in the last of
-// the nblocks blocks of its problem.
+// The step of a group in place `slot`, for tile_step; in the first block of
+// its problem the record is also handed on.
+__device__ __forceinline__ TileStep begin_tile(StepControl *ctl, int slot, const PlanParams &plan, bool first)
+{
+    TileRecord r = fold_record(ctl, slot, plan);
+    const TileStep now = {r.t, r.dt, r.active, r.steps};
+    if (first && (threadIdx.x & 31) == 0) {
+        r.pending = r.active;
+        ctl->rec[slot ^ 1] = r;
+        ctl->smax[(r.steps + 2) & 3] = 0ull;
+    }
+    return now;
+}
+
+// Folds the block's wave-speed maximum and health into the record of the step
+// that follows `steps` committed ones.  Nothing waits for them: the next
+// kernel starts when this one has ended.
 template <int NT>
-__device__ __forceinline__ void end_tile(double vmax, int bad, StepControl *ctl, const StepControl &c,
-                                         const PlanParams &plan, unsigned nblocks)
+__device__ __forceinline__ void end_tile(double vmax, int bad, StepControl *ctl, int steps)
 {
     __shared__ double red[NT / 32];
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicCAS(&ctl->first_bad, 0, c.steps + 1);
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicCAS(&ctl->first_bad, 0, steps + 1);
     vmax = warp_max(vmax);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = vmax;
     __syncthreads();
     if (threadIdx.x >= 32) return;
     vmax = warp_max(threadIdx.x < NT / 32 ? red[threadIdx.x] : 0.0);
-    if (threadIdx.x != 0) return;
-    if (vmax > 0.0) atomicMax(&ctl->smax_bits, (unsigned long long)__double_as_longlong(vmax));
-    __threadfence();
-    if (atomicAdd(&ctl->ticket, 1u) == nblocks - 1) {
-        __threadfence();
-        finish_tile_step(ctl, c, plan);
-    }
+    if (threadIdx.x == 0 && vmax > 0.0)
+        atomicMax(&ctl->smax[(steps + 1) & 3], (unsigned long long)__double_as_longlong(vmax));
+}
+
+// Ends a group of steps: commits record `r`, folded from the group's last
+// step, and opens the next group.  One thread, after every block's fold.
+__device__ __forceinline__ void commit_record(StepControl *ctl, const TileRecord &r)
+{
+    ctl->t = r.t;
+    ctl->dt = r.dt;
+    ctl->smax_last = r.smax_last;
+    ctl->steps = r.steps;
+    ctl->active = r.active;
+    ctl->done = r.done;
+    ctl->parity = r.parity;
+    ctl->smax_bits = 0ull;
+    ctl->ticket = 0u;
+    open_record(ctl);
 }
 
 #ifdef __CUDACC__  // (host builds of this file call tile_step)
+// Step `place` of its group.
 template <typename Real, class Phys, class T, int MINB>
-__global__ void __launch_bounds__(T::NT, MINB) step_tile_kernel(TileArgs<Real> a)
+__global__ void __launch_bounds__(T::NT, MINB) step_tile_kernel(TileArgs<Real> a, int place)
 {
     extern __shared__ __align__(16) unsigned char tile_smem[];
     pdl_launch();
     pdl_wait();
-    __shared__ StepControl c;
-    if (threadIdx.x == 0) c = *a.ctl;
-    __syncthreads();
-    if (!c.active) return;
-    if (c.parity) {
-        const Field<Real> f = a.src;
-        a.src = a.dst;
-        a.dst = f;
-    }
-    double vmax = 0.0;
+    const bool first = blockIdx.x == 0 && blockIdx.y == 0;
+    double vmax = first && threadIdx.x == 0 ? ring_speed<Real>(a.strategy, a.gamma) : 0.0;
     int bad = 0;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
-    TileResults<Real, T> res;
-    tile_step<Real, Phys, T>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, res, c.ring_due, c.t);
-    end_tile<T::NT>(vmax, bad, a.ctl, c, a.plan, gridDim.x * gridDim.y);
-    tile_store<Real, Phys, T>(a, blockIdx.x, blockIdx.y, res);
+    if (tile_step<Real, Phys, T>(a, blockIdx.x, blockIdx.y, tile_smem,
+                                 [&] { return begin_tile(a.ctl, place & 1, a.plan, first); }, place > 0, vmax, bad))
+        end_tile<T::NT>(vmax, bad, a.ctl, reinterpret_cast<TileHead<Real> *>(tile_smem)->step.steps);
 }
 
-// A taped step, from src to dst whatever the parity; fill: the ring of src is
-// not filled yet (the steps of a tape but its first).
+// A taped step.
 template <typename Real, class Phys, class T, int MINB>
-__global__ void __launch_bounds__(T::NT, MINB) step_tape_kernel(TileArgs<Real> a, TapeArgs<Real> tape, int fill)
+__global__ void __launch_bounds__(T::NT, MINB) step_tape_kernel(TileArgs<Real> a, TapeArgs<Real> tape, int place)
 {
     extern __shared__ __align__(16) unsigned char tile_smem[];
     pdl_launch();
     pdl_wait();
-    __shared__ StepControl c;
-    if (threadIdx.x == 0) c = *a.ctl;
-    __syncthreads();
-    if (!c.active) return;
-    double vmax = 0.0;
+    const bool first = blockIdx.x == 0 && blockIdx.y == 0;
+    double vmax = first && threadIdx.x == 0 ? ring_speed<Real>(a.strategy, a.gamma) : 0.0;
     int bad = 0;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) vmax = ring_speed<Real>(a.strategy, a.gamma);
-    TileResults<Real, T> res;
-    tile_step<Real, Phys, T, true>(a, c.dt, blockIdx.x, blockIdx.y, tile_smem, vmax, bad, res, fill != 0, c.t, &tape);
-    end_tile<T::NT>(vmax, bad, a.ctl, c, a.plan, gridDim.x * gridDim.y);
-    tile_store<Real, Phys, T>(a, blockIdx.x, blockIdx.y, res);
+    if (tile_step<Real, Phys, T, true>(a, blockIdx.x, blockIdx.y, tile_smem,
+                                       [&] { return begin_tile(a.ctl, place & 1, a.plan, first); }, place > 0, vmax, bad,
+                                       &tape))
+        end_tile<T::NT>(vmax, bad, a.ctl, reinterpret_cast<TileHead<Real> *>(tile_smem)->step.steps);
 }
 
-// Stores the ghost ring after steps in tiles (src: the state if the parity
-// is even, dst: if odd).  One thread per ring cell.
+// Ends a group of `steps` steps in tiles (src, dst: the state if the parity
+// is even, odd): stores the ghost ring, one thread per ring cell, and, in the
+// last block, commits the record.
 template <typename Real, int NT>
-__global__ void __launch_bounds__(NT) fill_ring_kernel(TileArgs<Real> a, int residual)
+__global__ void __launch_bounds__(NT) end_steps_kernel(TileArgs<Real> a, int steps, int residual)
 {
     pdl_launch();
     pdl_wait();
-    if (!a.ctl->ring_due) return;
-    if (a.ctl->parity) a.src = a.dst;
-    GhostArgs<Real> g = ring_args(a);
-    g.residual = residual;
-    const int k = blockIdx.x * NT + threadIdx.x;
-    if (k < 4 * a.nx + 4 * (a.ny - 4)) ghost_cell(g, k, a.ctl->t);
+    const TileRecord r = fold_record(a.ctl, steps & 1, a.plan);
+    if (r.ring_due) {
+        if (r.parity) a.src = a.dst;
+        GhostArgs<Real> g = ring_args(a);
+        g.residual = residual;
+        const int k = blockIdx.x * NT + threadIdx.x;
+        if (k < 4 * a.nx + 4 * (a.ny - 4)) ghost_cell(g, k, r.t);
+    }
+    if (last_block_done(&a.ctl->ticket)) commit_record(a.ctl, r);
 }
 #endif
 

@@ -39,10 +39,8 @@ int step(const double *in, double *out, int nx, int ny, double width, double hei
     std::vector<double> v(T::NT, 0.0);
     std::vector<int> b(T::NT, 0);
     emu::launch(dim3((nx - 4 + T::TX - 1) / T::TX, (ny - 4 + T::TY - 1) / T::TY), dim3(T::NT), true, [&] {
-        TileResults<double, T> res;
-        tile_step<double, Phys, T>(a, dt, int(blockIdx.x), int(blockIdx.y),
-                                   reinterpret_cast<unsigned char *>(smem.data()), v[threadIdx.x], b[threadIdx.x], res);
-        tile_store<double, Phys, T>(a, int(blockIdx.x), int(blockIdx.y), res);
+        tile_step<double, Phys, T>(a, int(blockIdx.x), int(blockIdx.y), reinterpret_cast<unsigned char *>(smem.data()),
+                                   [&] { return TileStep{0.0, dt, 1, 0}; }, false, v[threadIdx.x], b[threadIdx.x]);
     });
     *vmax = 0.0;
     *bad = 0;
@@ -95,11 +93,9 @@ long tape(const double *cells, int nx, int ny, int strategy, double t, double dt
     emu::launch(dim3((nx - 4 + T::TX - 1) / T::TX, (ny - 4 + T::TY - 1) / T::TY), dim3(T::NT), true, [&] {
         double vm = 0.0;
         int bad = 0;
-        TileResults<double, T> res;
-        tile_step<double, RefOrder, T, true>(a, dt, int(blockIdx.x), int(blockIdx.y),
-                                             reinterpret_cast<unsigned char *>(smem.data()), vm, bad, res, fill != 0, t,
-                                             &tp);
-        tile_store<double, RefOrder, T>(a, int(blockIdx.x), int(blockIdx.y), res);
+        tile_step<double, RefOrder, T, true>(a, int(blockIdx.x), int(blockIdx.y),
+                                             reinterpret_cast<unsigned char *>(smem.data()),
+                                             [&] { return TileStep{t, dt, 1, 0}; }, fill != 0, vm, bad, &tp);
     });
     long diff = 0;
     auto same = [&](double x, double y) { diff += !(x == y); };
