@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(T::NT, MINB) batch_tile_kernel(BatchArgs<Real>
     int bad = 0;
     if (tile_step<Real, Phys, T>(a, k % ntx, k / ntx, tile_smem,
                                  [&] { return begin_tile(a.ctl, b.step & 1, a.plan, k == 0); }, b.step > 0, vmax, bad))
-        end_tile<T::NT>(vmax, bad, a.ctl, reinterpret_cast<TileHead<Real> *>(tile_smem)->step.steps);
+        end_tile<T::NT>(vmax, bad, a.ctl, reinterpret_cast<TileHead<Real, Phys> *>(tile_smem)->step.steps);
 }
 
 // Ends a group of steps in tiles (end_steps_kernel).

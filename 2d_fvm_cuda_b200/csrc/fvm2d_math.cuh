@@ -427,6 +427,13 @@ template <typename Real>
 __device__ __forceinline__ Real alpha_rh(const SweepConsts<Real> &K) { return K.rh * K.alpha; }
 template <typename Real>
 __device__ __forceinline__ Real half_k(const SweepConsts<Real> &K) { return K.k * Real(0.5); }
+// and the constants kept as hi + lo pairs, joined
+template <typename Real>
+__device__ __forceinline__ double joined_lambda(const SweepConsts<Real> &K) { return double(K.lambda) + double(K.lambda_lo); }
+template <typename Real>
+__device__ __forceinline__ double joined_igm1(const SweepConsts<Real> &K) { return double(K.igm1) + double(K.igm1_lo); }
+template <typename Real>
+__device__ __forceinline__ double joined_gm1(const SweepConsts<Real> &K) { return double(K.gm1) + double(K.gm1_lo); }
 
 // Every sum of a product below is written as an fma or as two roundings, and
 // the FP64 build is compiled without contraction, so each copy of this

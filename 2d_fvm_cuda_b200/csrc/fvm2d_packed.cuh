@@ -108,15 +108,14 @@ struct PackedCompensated : HoistedCompensated {
 // is otherwise idle in these sweeps.)
 struct PackedResidual : PackedCompensated {
     static constexpr bool kSplitStorage = true;
-    template <class Consts>
+    template <class Flux, class Consts>
     __device__ static __forceinline__ Cell<double> update_split(const Cell<float> &U, const Cell<float> &L,
-                                                                const Cell<float> &FL, const Cell<float> &FR,
+                                                                const Cell<Flux> &FL, const Cell<Flux> &FR,
                                                                 const Consts &K)
     {
         const double rho = double(U.rho) + double(L.rho), p = double(U.p) + double(L.p);
         const double un = double(U.un) + double(L.un), ut = double(U.ut) + double(L.ut);
-        const double lam = double(K.lambda) + double(K.lambda_lo);
-        const double igm1 = double(K.igm1) + double(K.igm1_lo), gm1 = double(K.gm1) + double(K.gm1_lo);
+        const double lam = joined_lambda(K), igm1 = joined_igm1(K), gm1 = joined_gm1(K);
         double m0 = rho, m1 = rho * un, m3 = rho * ut;
         double m2 = fma(p, igm1, 0.5 * (m1 * un + m3 * ut));
         // W - lambda (F_R - F_L), the flux differences exact in FP64 (FP32
