@@ -276,25 +276,37 @@ __device__ __forceinline__ unsigned long long &lo_cell(const Field<Real> &F, int
     return reinterpret_cast<unsigned long long *>(residual_block(F.base, F.plane))[y * F.pitch + x];
 }
 
-// the residuals of a cell, as values of the arithmetic type
-template <typename Real>
-__device__ __forceinline__ Cell<Real> load_lo(const Field<Real> &F, int x, int y, int fn, int ft)
+// the residuals of a cell's word (divided by kResidualScale); swap: un is
+// field 3
+__device__ __forceinline__ Cell<double> lo_parts(unsigned long long w, bool swap)
 {
-    const unsigned long long w = lo_cell(F, x, y);
-    auto part = [&](int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
-    Cell<Real> c;
-    c.rho = part(0);
-    c.p = part(1);
-    c.un = part(fn);
-    c.ut = part(ft);
-    return c;
+    const unsigned int a = (unsigned int)w, b = swap_halves((unsigned int)(w >> 32), swap);
+    return {scaled_residual(a << 16), scaled_residual(a), scaled_residual(b << 16), scaled_residual(b)};
 }
 
 template <typename Real>
-__device__ __forceinline__ Cell<double> join_cell(const Cell<Real> &hi, const Cell<Real> &lo)
+__device__ __forceinline__ Cell<double> load_lo(const Field<Real> &F, int x, int y, int fn)
 {
-    return {double(hi.rho) + double(lo.rho), double(hi.p) + double(lo.p), double(hi.un) + double(lo.un),
-            double(hi.ut) + double(lo.ut)};
+    return lo_parts(lo_cell(F, x, y), fn == 3);
+}
+
+// hi + lo of a cell, lo as lo_parts gives it (the product is exact)
+template <typename Real>
+__device__ __forceinline__ Cell<double> join_cell(const Cell<Real> &hi, const Cell<double> &lo)
+{
+    return {fma(lo.rho, kResidualScale, double(hi.rho)), fma(lo.p, kResidualScale, double(hi.p)),
+            fma(lo.un, kResidualScale, double(hi.un)), fma(lo.ut, kResidualScale, double(hi.ut))};
+}
+
+// v as FP32 values (returned) and the residual word; swap: un is field 3
+template <typename Real>
+__device__ __forceinline__ Cell<Real> split_cell(const Cell<double> &v, bool swap, unsigned long long &w)
+{
+    float h[4];
+    const unsigned int l0 = split_bits(v.rho, h[0]), l1 = split_bits(v.p, h[1]);
+    const unsigned int l2 = split_bits(v.un, h[2]), l3 = split_bits(v.ut, h[3]);
+    w = (unsigned long long)swap_halves(l2 >> 16 | l3, swap) << 32 | (l0 >> 16 | l1);
+    return {Real(h[0]), Real(h[1]), Real(h[2]), Real(h[3])};
 }
 
 // v split into the FP32 planes and the cell's residual word; returns the
@@ -303,15 +315,9 @@ template <typename Real>
 __device__ __forceinline__ Cell<Real> store_split(const Field<Real> &F, int x, int y, int fn, int ft,
                                                   const Cell<double> &v)
 {
-    float h[4];
-    unsigned short l[4];
-    split_value(v.rho, h[0], l[0]);
-    split_value(v.p, h[1], l[1]);
-    split_value(v.un, h[2], l[fn]);
-    split_value(v.ut, h[3], l[ft]);
-    lo_cell(F, x, y) = (unsigned long long)l[0] | (unsigned long long)l[1] << 16 | (unsigned long long)l[2] << 32 |
-                       (unsigned long long)l[3] << 48;
-    const Cell<Real> hi = {Real(h[0]), Real(h[1]), Real(h[2]), Real(h[3])};
+    unsigned long long w;
+    const Cell<Real> hi = split_cell<Real>(v, fn == 3, w);
+    lo_cell(F, x, y) = w;
     store_cell(F, x, y, fn, ft, hi);
     return hi;
 }
@@ -504,10 +510,11 @@ __device__ __forceinline__ void x_item(const SweepArgs<Real> &a, const SweepCons
             c0 = ld(c);
             cp1 = ld(c + 1);
         }
-        Cell<Real> A, Alo, Ulo;
+        Cell<Real> A;
+        Cell<double> Alo, Ulo;
         if (FINAL) A = load_cell(a.comb, min(max(u, 0), nx - 1), y, 2, 3);  // branch A, loaded early
-        if (FINAL && kResidual) Alo = load_lo(a.comb, min(max(u, 0), nx - 1), y, 2, 3);
-        if (kResidual) Ulo = load_lo(a.src, min(max(u, 0), nx - 1), y, 2, 3);  // the updated cell's, early
+        if (FINAL && kResidual) Alo = load_lo(a.comb, min(max(u, 0), nx - 1), y, 2);
+        if (kResidual) Ulo = load_lo(a.src, min(max(u, 0), nx - 1), y, 2);  // the updated cell's, early
         const Cell<Real> s0 = Phys::slope(cm1, c0, cp1, K);                // slope of cell c
         Cell<Real> sm1 = shfl_up(s0);                                     // slope of cell c-1
         if (lane == 0) sm1 = cs;
@@ -518,7 +525,7 @@ __device__ __forceinline__ void x_item(const SweepArgs<Real> &a, const SweepCons
         if (lane == 0) FL = cF;
         if ((j > 0 || lane >= 2) && u <= last) {
             if constexpr (kResidual)
-                emit_split(u, Phys::update_split(cm1, Ulo, FL, F, K), join_cell(A, Alo));
+                emit_split(u, Phys::update_split(join_cell(cm1, Ulo), FL, F, K), join_cell(A, Alo));
             else
                 emit(u, Phys::update(cm1, FL, F, K), A);
         }
@@ -534,9 +541,9 @@ __device__ __forceinline__ void x_item(const SweepArgs<Real> &a, const SweepCons
         Cell<Real> Ab;
         if (FINAL) Ab = load_cell(a.comb, x, y, 2, 3);
         if constexpr (kResidual) {
-            Cell<Real> Ablo;
-            if (FINAL) Ablo = load_lo(a.comb, x, y, 2, 3);
-            emit_split(x, join_cell(ld(x), load_lo(a.src, x, y, 2, 3)), join_cell(Ab, Ablo));
+            Cell<double> Ablo;
+            if (FINAL) Ablo = load_lo(a.comb, x, y, 2);
+            emit_split(x, join_cell(ld(x), load_lo(a.src, x, y, 2)), join_cell(Ab, Ablo));
         } else {
             emit(x, ld(x), Ab);
         }
@@ -619,7 +626,7 @@ __device__ __forceinline__ void y_item(const SweepArgs<Real> &a, const SweepCons
             if (tape && col) store_cell(a.flux, x, ny - 1 - l, 2, 3, F);  // interface l-1/2 at line position l
             if (l > l0 && col) {  // cell l-1
                 if constexpr (kResidual)
-                    store_split(a.dst, x, ny - l, 3, 2, Phys::update_split(cm1, load_lo(a.src, x, ny - l, 3, 2), Fp, F, K));
+                    store_split(a.dst, x, ny - l, 3, 2, Phys::update_split(join_cell(cm1, load_lo(a.src, x, ny - l, 3)), Fp, F, K));
                 else
                     store_cell(a.dst, x, ny - l, 3, 2, Phys::update(cm1, Fp, F, K));
             }
@@ -644,8 +651,7 @@ __device__ __forceinline__ void y_item(const SweepArgs<Real> &a, const SweepCons
         };
         auto get_lo = [&](int l) {  // the residuals of row l, in (rho, p, un, ut) order
             const unsigned long long w = ring_lo[(l & (kYRingRows - 1)) * rs];
-            auto part = [&](int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
-            return Cell<Real>{part(0), part(1), part(3), part(2)};
+            return lo_parts(w, true);
         };
         auto get = [&](int l) {
             const Real *r = ring + (l & (kYRingRows - 1)) * 4 * rs;
@@ -675,7 +681,7 @@ __device__ __forceinline__ void y_item(const SweepArgs<Real> &a, const SweepCons
             if (tape && col) store_cell(a.flux, x, ny - 1 - l, 2, 3, F);
             if (l > l0 && col) {
                 if constexpr (kResidual)
-                    store_split(a.dst, x, ny - l, 3, 2, Phys::update_split(cm1, get_lo(l - 1), Fp, F, K));
+                    store_split(a.dst, x, ny - l, 3, 2, Phys::update_split(join_cell(cm1, get_lo(l - 1)), Fp, F, K));
                 else
                     store_cell(a.dst, x, ny - l, 3, 2, Phys::update(get(l - 1), Fp, F, K));
             }

@@ -109,12 +109,10 @@ struct PackedCompensated : HoistedCompensated {
 struct PackedResidual : PackedCompensated {
     static constexpr bool kSplitStorage = true;
     template <class Flux, class Consts>
-    __device__ static __forceinline__ Cell<double> update_split(const Cell<float> &U, const Cell<float> &L,
-                                                                const Cell<Flux> &FL, const Cell<Flux> &FR,
-                                                                const Consts &K)
+    __device__ static __forceinline__ Cell<double> update_split(const Cell<double> &U, const Cell<Flux> &FL,
+                                                                const Cell<Flux> &FR, const Consts &K)
     {
-        const double rho = double(U.rho) + double(L.rho), p = double(U.p) + double(L.p);
-        const double un = double(U.un) + double(L.un), ut = double(U.ut) + double(L.ut);
+        const double rho = U.rho, p = U.p, un = U.un, ut = U.ut;
         const double lam = joined_lambda(K), igm1 = joined_igm1(K), gm1 = joined_gm1(K);
         double m0 = rho, m1 = rho * un, m3 = rho * ut;
         double m2 = fma(p, igm1, 0.5 * (m1 * un + m3 * ut));

@@ -317,11 +317,6 @@ __device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int b
         }
     }
 
-    // residual word -> the residuals of fields 0, 1, f2, f3
-    auto parts = [](Word w, int f2, int f3) {
-        auto part = [&](int f) { return Real(bf16_value((unsigned short)(w >> (16 * f)))); };
-        return Cell<Real>{part(0), part(1), part(f2), part(f3)};
-    };
     // the step's result at tile cell (r, c): branch A (sU, lU) averaged with
     // branch B in primitive variables (src/basicFuns.cuh:264-274)
     auto finish = [&](int r, int c, auto b) {
@@ -330,7 +325,7 @@ __device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int b
         const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
         Cell<Real> o;
         if constexpr (kResidual) {
-            const Cell<double> d = join_cell(A, parts(lU[r * T::kLo + c], 2, 3));
+            const Cell<double> d = join_cell(A, lo_parts(lU[r * T::kLo + c], false));
             o = store_split(a.dst, x, y, 2, 3,
                             Cell<double>{(d.rho + b.rho) * 0.5, (d.p + b.p) * 0.5, (d.un + b.un) * 0.5,
                                          (d.ut + b.ut) * 0.5});
@@ -397,12 +392,11 @@ __device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int b
                 if (mine && k >= 1 && in) store_cell(tape->F[phase == 0 ? (xdir ? 0 : 1) : xdir ? 3 : 2], x, y, 2, 3, F);
             }
             if (!mine || k < 2) continue;
-            const int fn = xdir ? 2 : 3;
             auto updated = [&] {
                 if constexpr (kResidual)
-                    return Phys::update_split(get(q - s),
-                                              parts((phase == 0 ? lU : xdir ? lB : lA)[ru * T::kLo + cu], fn, 5 - fn),
-                                              FL, FR, K);
+                    return Phys::update_split(
+                        join_cell(get(q - s), lo_parts((phase == 0 ? lU : xdir ? lB : lA)[ru * T::kLo + cu], !xdir)), FL,
+                        FR, K);
                 else
                     return Phys::update(get(q - s), FL, FR, K);
             };
@@ -413,18 +407,12 @@ __device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int b
             Real *const d = (phase == 0 ? (xdir ? sA : sB) : xdir ? sR : sU) + ru * RS + cu;
             const auto v = updated();
             if constexpr (kResidual) {
-                float h[4];
-                unsigned short l[4];
-                split_value(v.rho, h[0], l[0]);
-                split_value(v.p, h[1], l[1]);
-                split_value(v.un, h[2], l[fn]);
-                split_value(v.ut, h[3], l[5 - fn]);
-                (phase == 0 ? (xdir ? lA : lB) : lU)[ru * T::kLo + cu] =
-                    (Word)l[0] | (Word)l[1] << 16 | (Word)l[2] << 32 | (Word)l[3] << 48;
-                d[0] = h[0];
-                d[NC] = h[1];
-                d[on] = h[2];
-                d[ot] = h[3];
+                const Cell<Real> h =
+                    split_cell<Real>(v, !xdir, (phase == 0 ? (xdir ? lA : lB) : lU)[ru * T::kLo + cu]);
+                d[0] = h.rho;
+                d[NC] = h.p;
+                d[on] = h.un;
+                d[ot] = h.ut;
             } else {
                 d[0] = v.rho;
                 d[NC] = v.p;
