@@ -150,7 +150,6 @@ struct fvm2d_batch {
             xchunks /= 2;
         }
         if ((int)listed.size() != np) listed.assign(np, 1);
-        tile_shape = kBatchVariants[precision].tile_shape(np, nx.data(), ny.data());
         // offsets in elements of the storage type: FP32 planes start at the
         // same byte addresses as FP64 planes would (the layout is in doubles)
         const long long scale = (precision == FVM2D_FP32) ? 2 : 1;
@@ -211,9 +210,14 @@ struct fvm2d_batch {
     long long y_items(int p) const { return (long long)((nx[p] + 31) / 32) * y_segments(ny[p], T); }
     long long tiles(int p) const { return kBatchVariants[precision].tiles(tile_shape, nx[p], ny[p]); }
 
-    // Tile prefix counts of the listed problems -> device.
+    // The tile shape for the listed problems, and their tile prefix counts ->
+    // device.
     int upload_tiles()
     {
+        std::vector<int> lx, ly;
+        for (int p = 0; p < np; ++p)
+            if (listed[p]) lx.push_back(nx[p]), ly.push_back(ny[p]);
+        L.tile_shape = tile_shape = kBatchVariants[precision].tile_shape((int)lx.size(), lx.data(), ly.data());
         std::vector<long long> t0(np + 1, 0);
         for (int p = 0; p < np; ++p) t0[p + 1] = t0[p] + (listed[p] ? tiles(p) : 0);
         CK(cudaMemcpyAsync(t0_d, t0.data(), sizeof(long long) * (np + 1), cudaMemcpyHostToDevice, stream));
@@ -236,13 +240,14 @@ struct fvm2d_batch {
         L.x_total = x0[np];
         L.y_total = y0[np];
         L.t0 = use_tiles ? t0_d : nullptr;
-        L.tile_shape = tile_shape;
         return FVM2D_OK;
     }
 
     // After a group of steps: drops the problems whose loop has ended from the
     // lists once they hold at least an eighth of the listed tiles, or a
-    // quarter of the listed x items (whose lists the graphs hold).
+    // quarter of the listed x items (whose lists the graphs hold).  Those left
+    // get the tile shape that suits them: 20 problems of 64^2 .. 384^2 that
+    // end after 18 to 111 steps, 9.55 ms in the first shape, 9.37 so.
     int compact_items()
     {
         long long ended = 0;
