@@ -1,5 +1,6 @@
 // fvm2d_batch.cuh -- batched kernels: many independent problems of different
-// sizes advance together, one launch per stage of the step.
+// sizes advance together, one launch per step in tiles (batch_tile_kernel, a
+// block per tile of any problem) or one per stage of the step.
 //
 // Each problem keeps its own state buffers, step-control record (its own dt,
 // time and end time) and ghost preset.  The work items of a stage -- x-sweep

@@ -10,10 +10,10 @@
 //            are `scratch`: the sweeps' A and B and the staging area for
 //            uploads and downloads;
 //   ctl      the device-resident StepControl of the time loop;
-//   CUDA graphs of 16, 4 and 1 steps replayed until the control record says
-//   the loop has ended; the only host round trip is one 64-byte read per
-//   group of replays (the reference reads the max wave speed back and
-//   synchronizes 17 times per step, src/wrappers.cuh:196-284);
+//            steps are enqueued in groups until it says the loop has ended,
+//            and the only host round trip is one read of it per group (the
+//            reference reads the max wave speed back and synchronizes 17
+//            times per step, src/wrappers.cuh:196-284);
 //   and, allocated on first use, the differentiation workspaces (dual-number
 //   states of fvm2d_jvp; checkpoints, one segment's tape (or, for a
 //   full-tape forward, every step's) and the adjoint states of

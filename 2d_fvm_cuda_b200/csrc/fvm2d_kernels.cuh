@@ -1,9 +1,12 @@
 // fvm2d_kernels.cuh -- the sm_100a kernels of one split step.
 //
 // A step is  U <- ghost( (Y(X(U)) + X(Y(U))) / 2 )  with one dt
-// (src/wrappers.cuh:196-284).  It runs as five kernels, all reading the step
-// size from a device-resident control record so the loop never waits on the
-// host:
+// (src/wrappers.cuh:196-284).  Whole problems take it in tiles, one kernel a
+// step (fvm2d_tile.cuh, which uses the arithmetic, records and ghost rules
+// here).  A row slab, whose halo rows pass through the sweeps, and a batch
+// that was tuned to it run the five kernels of this file, all reading the
+// step size from a device-resident control record so the loop never waits on
+// the host:
 //
 //   sweep_x        U -> A         first sweep of branch A
 //   sweep_y        U -> B         first sweep of branch B

@@ -524,7 +524,11 @@ struct Hoisted {
             o.p_t = -fma(u_r, pi_rx, (c_r * sr) * u_rx);
         } else {
             const Real u = (fma(u_l, c_l, u_r * c_r) - dp) * isum;
-            const Real pm = fma(du * c_l, c_r, fma(c_l, pi_r, c_r * pi_l)) * isum;
+            Real pm;
+            if constexpr (std::is_same<Real, float>::value)  // the small term first: one full-size rounding less
+                pm = fma(c_r, pi_l, fma(c_l, pi_r, (du * c_l) * c_r)) * isum;
+            else
+                pm = fma(du * c_l, c_r, fma(c_l, pi_r, c_r * pi_l)) * isum;
             // b_l = -s_l k_l, b_r = s_r k_r, nDp = -Dpi_Dt
             const Real b_l = sl * fma(half * u_l, c_lx, fma(c_l, u_lx, pi_lx));
             const Real b_r = sr * fma(half * u_r, c_rx, fma(c_r, u_rx, -pi_rx));
@@ -578,13 +582,24 @@ struct Hoisted {
     {
         const Real hk = half_k(K), half = Real(0.5);
         const Real m = w.rho * w.un, m_t = fma(w.rho, w.un_t, w.un * w.rho_t);
-        const Real M = fma(hk, m_t, m), Q = fma(hk, w.p_t, w.p), hm = hk * m;
+        const Real M = fma(hk, m_t, m), hm = hk * m;
         const Real es = fma(half, fma(w.un, w.un, w.ut * w.ut), w.e);
         const Real et = fma(w.un, w.un_t, fma(w.ut, w.ut_t, w.e_t));
         Cell<Real> F;
         F.rho = M;
-        F.p = fma(M, w.un, fma(hm, w.un_t, Q));
-        F.un = fma(es, M, fma(hm, et, fma(w.un, Q, (hk * w.p) * w.un_t)));
+        if constexpr (std::is_same<Real, float>::value) {
+            // the time derivatives' parts, small where the flow is smooth, are
+            // summed first: two full-size roundings a flux instead of three
+            // and four (with Q, a residual build's velocities ended 20% further
+            // from FP64 on a shock-bubble flow; 0.7% of its step)
+            const Real dp = hk * w.p_t;
+            F.p = fma(M, w.un, w.p) + fma(hm, w.un_t, dp);
+            F.un = fma(es, M, fma(w.un, w.p, fma(hm, et, fma(w.un, dp, (hk * w.p) * w.un_t))));
+        } else {
+            const Real Q = fma(hk, w.p_t, w.p);
+            F.p = fma(M, w.un, fma(hm, w.un_t, Q));
+            F.un = fma(es, M, fma(hm, et, fma(w.un, Q, (hk * w.p) * w.un_t)));
+        }
         F.ut = fma(M, w.ut, hm * w.ut_t);
         return F;
     }

@@ -9,8 +9,9 @@
 // own device memory; this entry point advances it using only memory that
 // exists for the whole life of the library.
 //
-// The sweeps need two state-sized intermediate buffers and the step-control
-// record.  Here they live in one file-scope device array, `g_scratch`, sized
+// The steps go back and forth between the caller's buffer and a scratch
+// state, under a step-control record.  Room for two such states and the
+// record lives in one file-scope device array, `g_scratch`, sized
 // for at most kNoAllocMaxCells cells; every GPU that loads the library holds
 // that array (16 MiB + 256 B) until the process exits.  Every call uses the
 // same array: calls whose work overlaps on the GPU (on different streams, or
