@@ -255,17 +255,18 @@ int fvm2d_get_time_stages_count(fvm2d_solver *s, long long *count);
 int fvm2d_get_time(fvm2d_solver *s, double *t, int *steps, double *last_dt);
 
 /* CUDA-event time (on the handle's stream) of the last solve()/advance()
- * loop, and the number of kernels it launched (graph replays launch every
- * captured kernel; steps after the loop ends exit at once).  No reference
+ * loop, and the number of kernels it launched (steps enqueued past the
+ * loop's end exit at once).  No reference
  * counterpart: the reference times its loop on the host only
  * (src/wrappers.cuh:193,286-288). */
 int fvm2d_get_run_stats(fvm2d_solver *s, double *device_ms, long long *kernel_launches);
 
-/* Runs up to nsteps steps one at a time outside the graph, with CUDA events
+/* Runs up to nsteps steps in groups of one, with CUDA events
  * between the kernels of a step; kernel_ms[0..4] receive their mean durations
  * in milliseconds and *steps_done the steps taken.  A whole problem steps in
  * tiles, all four sweeps and the average in one kernel: [3] is that kernel,
- * [4] the ghost ring's, [0..2] next to nothing.  A row slab's step has five:
+ * [4] the one that commits it and stores the ghost ring, [0..2] next to
+ * nothing.  A row slab's step has five:
  * sweep X, sweep Y, sweep Y, final sweep X + average, ghost ring.  Advances the state like
  * fvm2d_advance.  No reference counterpart (diagnostics). */
 int fvm2d_profile_kernels(fvm2d_solver *s, int nsteps, double *kernel_ms, int *steps_done);
@@ -332,10 +333,10 @@ int fvm2d_vjp(fvm2d_solver *s, const double *cotangent_in, double *cotangent_out
 int fvm2d_set_vjp_overlap(fvm2d_solver *s, int on);
 
 /* ---- batched form (no reference counterpart) -------------------------------
- * Many independent problems of different sizes advance together: every stage
- * of the step is one launch covering all problems, each problem with its own
- * dt, end time and ghost preset, and the time loop is captured in CUDA
- * graphs.  Results match the same problems solved one by one with the same
+ * Many independent problems of different sizes advance together: a step is
+ * one launch covering all problems, each problem with its own dt, end time
+ * and ghost preset, and the host only reads the control records now and
+ * then.  Results match the same problems solved one by one with the same
  * precision bit for bit. */
 typedef struct fvm2d_batch fvm2d_batch;
 
