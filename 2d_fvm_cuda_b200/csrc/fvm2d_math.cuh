@@ -627,12 +627,13 @@ struct Hoisted {
                                                         const Cell<Real> &FR, const Consts &K)
     {
         const Real half = Real(0.5);
-        const Real r1 = U.rho * U.un, r3 = U.rho * U.ut;
-        const Real r2 = fma(U.p, K.igm1, half * fma(r1, U.un, r3 * U.ut));
+        // W + lambda (F_L - F_R), the change rounded before the conserved value
+        // it joins: one rounding of each component
         const Real m0 = fma(FL.rho - FR.rho, K.lambda, U.rho);
-        const Real m1 = fma(FL.p - FR.p, K.lambda, r1);
-        const Real m2 = fma(FL.un - FR.un, K.lambda, r2);
-        const Real m3 = fma(FL.ut - FR.ut, K.lambda, r3);
+        const Real m1 = fma(U.rho, U.un, (FL.p - FR.p) * K.lambda);
+        const Real m2 = fma(U.p, K.igm1,
+                            fma(FL.un - FR.un, K.lambda, (half * U.rho) * fma(U.un, U.un, U.ut * U.ut)));
+        const Real m3 = fma(U.rho, U.ut, (FL.ut - FR.ut) * K.lambda);
         const Real ir = rrcp(m0);
         Cell<Real> o;
         o.rho = m0;
