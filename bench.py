@@ -379,7 +379,7 @@ def product_arm(args, rank, world, local_rank):
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": {"workload": f"four_quadrant_{n}x{n}_fp64", "nx": n, "ny": n, "ghost": "outflow",
                        "cfl": CFG["cfl"], "alpha": CFG["alpha"], "gamma": CFG["gamma"], "seed": "rank",
-                       "arithmetic": "FP64, FMA contraction (nvcc default)",
+                       "arithmetic": "FP64 with FMA",
                        "l2": "inputs larger than L2 (537 MB state buffers)",
                        "parallelism": f"replicas x{world}"},
             "l1_rel_vs_reference_order": {"fields": ["rho", "p", "u", "v"], "value": l1,
@@ -479,7 +479,7 @@ def slab_arm(args, rank, world, local_rank):
             "config": {"workload": f"four_quadrant_slabs_{n}x{ny}_fp64", "nx": n, "ny": ny,
                        "rows_per_gpu": owned, "ghost": "outflow", "cfl": CFG["cfl"], "alpha": CFG["alpha"],
                        "gamma": CFG["gamma"], "seed": "tile k seeded with k",
-                       "arithmetic": "FP64, FMA contraction (nvcc default)",
+                       "arithmetic": "FP64 with FMA",
                        "l2": "inputs larger than L2 (three 537 MB state buffers per GPU)",
                        "parallelism": f"row slabs x{world}: NCCL halo exchange (2 rows per neighbour) "
                                       "+ 8-byte max all-reduce per step, enqueued on the solver stream"},
