@@ -286,16 +286,74 @@ __device__ __forceinline__ void sound_adjoint(const Side &S, SideAdjoint &b, A g
     b.px = fma(S.r, t, b.px);
 }
 
+// The sides' i, cx, c, ic and s, the arguments of max(0, .) and 1/(c_l + c_r),
+// each with the forward's own roundings, so that the reverse takes its
+// branches: Hoisted::grp's grouping, in single precision Hoisted::fan.
+template <typename Real>
+__device__ __forceinline__ void side_speeds(Side &l, Side &r, const Cell<Real> &sL, const Cell<Real> &sR,
+                                            const SweepConsts<Real> &K, Real du, Real dp, Real &zl, Real &zr, Real &isum)
+{
+    if constexpr (std::is_same<Real, float>::value) {
+        const auto w = Hoisted::fan(Cell<Real>{l.r, l.p, l.u, l.v}, Cell<Real>{r.r, r.p, r.u, r.v}, sL, sR, K);
+        l.i = w.il, l.cx = w.c_lx, l.c = w.c_l, l.ic = w.icl, l.s = w.sl;
+        r.i = w.ir, r.cx = w.c_rx, r.c = w.c_r, r.ic = w.icr, r.s = w.sr;
+        zl = w.zl, zr = w.zr, isum = w.isum;
+    } else {
+        const Real zero = Real(0), kappa = K.kappa, hg = Real(0.5) * K.g;
+        l.i = rrsqrt(l.gp * l.r), r.i = rrsqrt(r.gp * r.r);
+        l.cx = l.Y * (hg * l.i), r.cx = r.Y * (hg * r.i);
+        if (r.p >= l.p) {
+            zl = fma(dp, r.i, du);
+            l.s = fma(kappa, rmax(zero, zl), l.gp * l.i);
+            l.c = l.r * l.s;
+            l.ic = rrcp(l.c);
+            zr = fma(-dp, l.ic, du);
+            r.s = fma(kappa, rmax(zero, zr), r.gp * r.i);
+            r.c = r.r * r.s;
+            const Real sc = l.c + r.c, q = rrcp(r.c * sc);
+            r.ic = sc * q;
+            isum = r.c * q;
+        } else {
+            zr = fma(-dp, l.i, du);
+            r.s = fma(kappa, rmax(zero, zr), r.gp * r.i);
+            r.c = r.r * r.s;
+            r.ic = rrcp(r.c);
+            zl = fma(dp, r.ic, du);
+            l.s = fma(kappa, rmax(zero, zl), l.gp * l.i);
+            l.c = l.r * l.s;
+            const Real sc = l.c + r.c, q = rrcp(l.c * sc);
+            l.ic = sc * q;
+            isum = l.c * q;
+        }
+    }
+}
+template <typename Real>
+__device__ __forceinline__ Real contact_speed(const Side &l, const Side &r, Real dp, Real isum)
+{
+    if constexpr (std::is_same<Real, float>::value)
+        return Hoisted::contact_speed(l.u, l.c, l.p, r.u, r.c, r.p, isum);
+    else
+        return (fma(l.u, l.c, r.u * r.c) - dp) * isum;
+}
+template <typename Real>
+__device__ __forceinline__ Real contact_pressure(const Side &l, const Side &r, Real du, Real isum)
+{
+    if constexpr (std::is_same<Real, float>::value)
+        return Hoisted::contact_pressure(du, l.c, l.p, r.c, r.p, isum);
+    else
+        return fma(du * l.c, r.c, fma(l.c, r.p, r.c * l.p)) * isum;
+}
+
 // Adjoint of Hoisted::interface_flux(UL, UR, sL, sR): given the flux adjoint
 // Fb (slots mass, normal momentum, energy, tangential momentum), adds the
 // adjoints of the two cells and the two slopes.  The forward is recomputed
-// with Hoisted::grp's grouping, and the reverse follows it.
+// as Hoisted::grp has it, so the reverse takes the forward's branches.
 __device__ __forceinline__ void interface_flux_adjoint(const Cell<A> &UL, const Cell<A> &UR, const Cell<A> &sL,
                                                        const Cell<A> &sR, const SweepConsts<A> &K, const Cell<A> &Fb,
                                                        Cell<A> &ULb, Cell<A> &URb, Cell<A> &sLb, Cell<A> &sRb)
 {
     const A half = A(0.5), zero = A(0);
-    const A g = K.g, igm1 = K.igm1, kappa = K.kappa, hk = K.k * half, hh = K.h * half, hg = half * g;
+    const A g = K.g, igm1 = K.igm1, kappa = K.kappa, hk = K.k * half, hh = K.h * half;
     Side l, r;
     l.r = fma(sL.rho, hh, UL.rho), l.p = fma(sL.p, hh, UL.p), l.u = fma(sL.un, hh, UL.un), l.v = fma(sL.ut, hh, UL.ut);
     r.r = fma(-sR.rho, hh, UR.rho), r.p = fma(-sR.p, hh, UR.p), r.u = fma(-sR.un, hh, UR.un);
@@ -303,35 +361,11 @@ __device__ __forceinline__ void interface_flux_adjoint(const Cell<A> &UL, const 
     l.rx = sL.rho, l.px = sL.p, l.ux = sL.un, l.vx = sL.ut;
     r.rx = sR.rho, r.px = sR.p, r.ux = sR.un, r.vx = sR.ut;
     l.gp = g * l.p, r.gp = g * r.p;
-    l.i = rrsqrt(l.gp * l.r), r.i = rrsqrt(r.gp * r.r);
     l.Y = fma(l.p, l.rx, l.r * l.px), r.Y = fma(r.p, r.rx, r.r * r.px);
-    l.cx = l.Y * (hg * l.i), r.cx = r.Y * (hg * r.i);
     const A du = l.u - r.u, dp = r.p - l.p;
     const bool left_first = r.p >= l.p;
     A zl, zr, isum;
-    if (left_first) {
-        zl = fma(dp, r.i, du);
-        l.s = fma(kappa, rmax(zero, zl), l.gp * l.i);
-        l.c = l.r * l.s;
-        l.ic = rrcp(l.c);
-        zr = fma(-dp, l.ic, du);
-        r.s = fma(kappa, rmax(zero, zr), r.gp * r.i);
-        r.c = r.r * r.s;
-        const A sc = l.c + r.c, q = rrcp(r.c * sc);
-        r.ic = sc * q;
-        isum = r.c * q;
-    } else {
-        zr = fma(-dp, l.i, du);
-        r.s = fma(kappa, rmax(zero, zr), r.gp * r.i);
-        r.c = r.r * r.s;
-        r.ic = rrcp(r.c);
-        zl = fma(dp, r.ic, du);
-        l.s = fma(kappa, rmax(zero, zl), l.gp * l.i);
-        l.c = l.r * l.s;
-        const A sc = l.c + r.c, q = rrcp(l.c * sc);
-        l.ic = sc * q;
-        isum = l.c * q;
-    }
+    side_speeds(l, r, sL, sR, K, du, dp, zl, zr, isum);
     SideAdjoint lb, rb;
     A dub = zero, dpb = zero;
     if (l.u - l.s >= zero) {
@@ -339,8 +373,8 @@ __device__ __forceinline__ void interface_flux_adjoint(const Cell<A> &UL, const 
     } else if (r.u + r.s <= zero) {
         one_sided_adjoint(r, rb, igm1, hk, Fb);
     } else {
-        const A u = (fma(l.u, l.c, r.u * r.c) - dp) * isum;
-        const A pm = fma(du * l.c, r.c, fma(l.c, r.p, r.c * l.p)) * isum;
+        const A u = contact_speed(l, r, dp, isum);
+        const A pm = contact_pressure(l, r, du, isum);
         const A Bl = fma(half * l.u, l.cx, fma(l.c, l.ux, l.px)), Br = fma(half * r.u, r.cx, fma(r.c, r.ux, -r.px));
         const A b_l = l.s * Bl, b_r = r.s * Br, nD = fma(r.c, b_l, l.c * b_r) * isum;
         A ub, pmb, nDb, blb, brb, xb;

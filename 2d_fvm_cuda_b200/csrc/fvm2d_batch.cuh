@@ -10,10 +10,11 @@
 // meets few problem boundaries, so the final sweep folds its wave-speed max
 // into a problem's record once per boundary).  Items of problems whose loop has
 // ended are skipped.  The per-item arithmetic is the single-problem kernels'
-// (x_item, y_item, ghost_cell).  In the contraction-free build a problem
-// advanced in a batch matches the same problem advanced alone bit for bit; in
-// the builds with FMA contraction the compiler may contract the inlined copies
-// of that arithmetic differently in the two kernels, and the two agree to
+// (x_item, y_item, ghost_cell).  In the FP64 product and contraction-free
+// builds a problem advanced in a batch matches the same problem advanced alone
+// bit for bit; in FP32 one rounding along y is the batch's own (PackedBatch),
+// and in the build in reference order the compiler may contract the inlined
+// copies of its arithmetic differently in the two kernels: these agree to
 // rounding.
 #pragma once
 

@@ -16,10 +16,9 @@
 // candidate y-segment lengths and sweep grid sizes on the batch itself and
 // keeps the fastest.
 //
-// Per problem, a batch gives the bits of a single solve in the
-// contraction-free build; in the builds with FMA contraction the two agree to
-// rounding (the compiler may contract the same inlined arithmetic differently
-// in the batched and the single-problem kernels).
+// Per problem, a batch gives the bits of a single solve in the FP64 product
+// and contraction-free builds; in the others the two agree to rounding
+// (fvm2d_batch.cuh).
 #include <nvtx3/nvToolsExt.h>
 #include "../../include/fvm2d.h"
 #include "fvm2d_batch_control.h"

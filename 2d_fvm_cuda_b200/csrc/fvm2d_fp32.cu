@@ -8,6 +8,7 @@
 #define FVM2D_VARIANT fp32
 #define FVM2D_REAL float
 #define FVM2D_PHYS PackedCompensated
+#define FVM2D_BATCH_PHYS PackedBatch
 #define FVM2D_TAPED_STEP  // also the taped step of FP32 differentiation runs
 // the FP64 wave speed from reciprocal square roots (fvm2d_math.cuh)
 #define FVM2D_FAST_RCP

@@ -1,6 +1,6 @@
-// fvm2d_fp64.cu -- FP64 kernels with hoisted reciprocals and FMA contraction:
-// the product default (FVM2D_FP64).  Checked against the reference within a
-// relative L1 tolerance.
+// fvm2d_fp64.cu -- FP64 kernels with hoisted reciprocals and every FMA written
+// out (compiled without contraction): the product default (FVM2D_FP64).
+// Checked against the reference within a relative L1 tolerance.
 #define FVM2D_VARIANT fp64
 #define FVM2D_REAL double
 #define FVM2D_PHYS Hoisted

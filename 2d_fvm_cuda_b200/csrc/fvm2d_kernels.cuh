@@ -272,6 +272,23 @@ struct split_storage : std::false_type {};
 template <class P>
 struct split_storage<P, std::void_t<decltype(P::kSplitStorage)>> : std::integral_constant<bool, P::kSplitStorage> {};
 
+// The interface flux of a sweep along x or y; last: of X(B), the step's last.
+// A physics with sweep_flux rounds some sweeps differently.
+template <class P, class = void>
+struct own_sweep_flux : std::false_type {};
+template <class P>
+struct own_sweep_flux<P, std::void_t<decltype(&P::template sweep_flux<SweepConsts<float>>)>> : std::true_type {};
+
+template <class Phys, typename Real, class Consts>
+__device__ __forceinline__ Cell<Real> sweep_flux(bool y, bool last, const Cell<Real> &UL, const Cell<Real> &UR,
+                                                 const Cell<Real> &sL, const Cell<Real> &sR, const Consts &K)
+{
+    if constexpr (own_sweep_flux<Phys>::value)
+        return Phys::sweep_flux(y, last, UL, UR, sL, sR, K);
+    else
+        return Phys::interface_flux(UL, UR, sL, sR, K);
+}
+
 // the 8-byte word of a cell's 4 residuals (field f in bits 16 f .. 16 f + 15)
 template <typename Real>
 __device__ __forceinline__ unsigned long long &lo_cell(const Field<Real> &F, int x, int y)
@@ -451,19 +468,17 @@ __device__ __forceinline__ void x_item(const SweepArgs<Real> &a, const SweepCons
             store_cell(a.dst, x, y, 2, 3, U);
         }
     };
-    // residual builds: U and Ab as hi + lo; the wave speed from the FP32 part
+    // residual builds: the value averaged already; the wave speed from the FP32 part
     // as stored (as the init and ghost kernels see it)
-    auto emit_split = [&](int x, const Cell<double> &U, const Cell<double> &Ab) {
+    auto emit_split = [&](int x, const Cell<double> &o) {
         if (FINAL) {
-            const Cell<double> o = {(Ab.rho + U.rho) * 0.5, (Ab.p + U.p) * 0.5, (Ab.un + U.un) * 0.5,
-                                    (Ab.ut + U.ut) * 0.5};
             const Cell<Real> h = store_split(a.dst, x, y, 2, 3, o);
             if (x >= 2 && x <= nx - 3 && y >= 2 && y <= ny - 3) {
                 vmax = fmax(vmax, wave_speed(h.rho, h.p, h.un, h.ut, a.gamma));
                 bad |= !(h.rho > Real(0) && h.p > Real(0));
             }
         } else {
-            store_split(a.dst, x, y, 2, 3, U);
+            store_split(a.dst, x, y, 2, 3, o);
         }
     };
     // chunk m's cell of this lane into its ring slot
@@ -522,13 +537,13 @@ __device__ __forceinline__ void x_item(const SweepArgs<Real> &a, const SweepCons
         Cell<Real> sm1 = shfl_up(s0);                                     // slope of cell c-1
         if (lane == 0) sm1 = cs;
         Cell<Real> F = {Real(0), Real(0), Real(0), Real(0)};
-        if (c <= nx - 2) F = Phys::interface_flux(cm1, c0, sm1, s0, K);   // interface c-1/2
+        if (c <= nx - 2) F = sweep_flux<Phys>(false, FINAL, cm1, c0, sm1, s0, K);   // interface c-1/2
         if (tape && (j > 0 || lane >= 1) && c <= nx - 2) store_cell(a.flux, c, y, 2, 3, F);  // at cell c
         Cell<Real> FL = shfl_up(F);                                       // interface c-3/2
         if (lane == 0) FL = cF;
         if ((j > 0 || lane >= 2) && u <= last) {
             if constexpr (kResidual)
-                emit_split(u, Phys::update_split(join_cell(cm1, Ulo), FL, F, K), join_cell(A, Alo));
+                emit_split(u, Phys::template update_split<FINAL>(join_cell(cm1, Ulo), FL, F, K, join_cell(A, Alo)));
             else
                 emit(u, Phys::update(cm1, FL, F, K), A);
         }
@@ -546,7 +561,12 @@ __device__ __forceinline__ void x_item(const SweepArgs<Real> &a, const SweepCons
         if constexpr (kResidual) {
             Cell<double> Ablo;
             if (FINAL) Ablo = load_lo(a.comb, x, y, 2);
-            emit_split(x, join_cell(ld(x), load_lo(a.src, x, y, 2)), join_cell(Ab, Ablo));
+            const Cell<double> U = join_cell(ld(x), load_lo(a.src, x, y, 2)), B = join_cell(Ab, Ablo);
+            if (FINAL)
+                emit_split(x, Cell<double>{(B.rho + U.rho) * 0.5, (B.p + U.p) * 0.5, (B.un + U.un) * 0.5,
+                                           (B.ut + U.ut) * 0.5});
+            else
+                emit_split(x, U);
         } else {
             emit(x, ld(x), Ab);
         }
@@ -625,7 +645,7 @@ __device__ __forceinline__ void y_item(const SweepArgs<Real> &a, const SweepCons
         for (int l = l0; l <= lend; ++l) {
             const Cell<Real> cp2 = ld(min(l + 2, ny - 1));  // next iteration's cell, loaded one interface ahead
             const Cell<Real> s0 = Phys::slope(cm1, c0, cp1, K);
-            const Cell<Real> F = Phys::interface_flux(cm1, c0, sm1, s0, K);
+            const Cell<Real> F = sweep_flux<Phys>(true, false, cm1, c0, sm1, s0, K);
             if (tape && col) store_cell(a.flux, x, ny - 1 - l, 2, 3, F);  // interface l-1/2 at line position l
             if (l > l0 && col) {  // cell l-1
                 if constexpr (kResidual)
@@ -680,7 +700,7 @@ __device__ __forceinline__ void y_item(const SweepArgs<Real> &a, const SweepCons
             async_wait<RING>();   // rows up to l+1 have landed
             const Cell<Real> cm1 = get(l - 1), c0 = get(l), cp1 = get(l + 1);
             const Cell<Real> s0 = Phys::slope(cm1, c0, cp1, K);
-            const Cell<Real> F = Phys::interface_flux(cm1, c0, sm1, s0, K);
+            const Cell<Real> F = sweep_flux<Phys>(true, false, cm1, c0, sm1, s0, K);
             if (tape && col) store_cell(a.flux, x, ny - 1 - l, 2, 3, F);
             if (l > l0 && col) {
                 if constexpr (kResidual)

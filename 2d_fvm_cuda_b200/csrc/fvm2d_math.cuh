@@ -524,11 +524,7 @@ struct Hoisted {
             o.p_t = -fma(u_r, pi_rx, (c_r * sr) * u_rx);
         } else {
             const Real u = (fma(u_l, c_l, u_r * c_r) - dp) * isum;
-            Real pm;
-            if constexpr (std::is_same<Real, float>::value)  // the small term first: one full-size rounding less
-                pm = fma(c_r, pi_l, fma(c_l, pi_r, (du * c_l) * c_r)) * isum;
-            else
-                pm = fma(du * c_l, c_r, fma(c_l, pi_r, c_r * pi_l)) * isum;
+            const Real pm = fma(du * c_l, c_r, fma(c_l, pi_r, c_r * pi_l)) * isum;
             // b_l = -s_l k_l, b_r = s_r k_r, nDp = -Dpi_Dt
             const Real b_l = sl * fma(half * u_l, c_lx, fma(c_l, u_lx, pi_lx));
             const Real b_r = sr * fma(half * u_r, c_rx, fma(c_r, u_rx, -pi_rx));
@@ -574,6 +570,162 @@ struct Hoisted {
         return o;
     }
 
+    // Single precision keeps the formulas term by term, and each rounding where
+    // it was: the midpoint flux jumps where the contact speed u (or a fan edge's
+    // speed) crosses zero, the star density and tangential velocity changing
+    // sides and k/2 rho u_t with them.  Where such a speed is within FP32
+    // rounding of zero the order of the operations decides, and cells there
+    // change by 1e-5 to 1e-4, so the order is part of what these builds return.
+    // Every fma is written (cfma) and they are compiled without contraction: left
+    // to the compiler, tiles and sweeps chose differently (17% of the velocities
+    // of one step apart in the last bit).  Two roundings belong to some sweeps,
+    // whose results keep them: `sound`, the sound speed's product rounded by
+    // itself in the impedances (PackedResidual); `once`, c_r u_rx - p_rx rounded
+    // once (PackedBatch).
+    // (host builds, for tests, round the product and the sum as the formulas read)
+    __device__ static __forceinline__ float cfma(float a, float b, float c)
+    {
+#if defined(__CUDA_ARCH__)
+        return fmaf(a, b, c);
+#else
+        return a * b + c;
+#endif
+    }
+    struct Fan {  // the two fans' speeds, as forward and adjoint take them
+        float irl, irr, il, ir, c_lx, c_rx, zl, zr, c_l, c_r, icl, icr, isum, sl, sr;
+    };
+    template <class Consts>
+    __device__ static __forceinline__ Fan fan(const Cell<float> &L, const Cell<float> &R, const Cell<float> &sL,
+                                              const Cell<float> &sR, const Consts &K, bool sound = false)
+    {
+        const float zero = 0.f, kappa = K.kappa, hg = 0.5f * K.g;
+        Fan w;
+        // 1/rho_l and 1/rho_r from one division
+        const float irlr = rrcp(L.rho * R.rho);
+        w.irl = R.rho * irlr;
+        w.irr = L.rho * irlr;
+        // 1/(rho a) = 1/sqrt(g p rho) and a = sqrt(g p / rho) = g p / sqrt(g p rho):
+        // one reciprocal square root per side
+        const float gpl = K.g * L.p, gpr = K.g * R.p;
+        w.il = rrsqrt(gpl * L.rho);
+        w.ir = rrsqrt(gpr * R.rho);
+        w.c_lx = hg * cfma(L.p, sL.rho, L.rho * sL.p) * w.il;
+        w.c_rx = hg * cfma(R.p, sR.rho, R.rho * sR.p) * w.ir;
+        const float du = L.un - R.un, dp = R.p - L.p;
+        auto speed = [&](float gp, float i, float z) {  // a + kappa max(0, z)
+            return sound ? cfma(kappa, rmax(zero, z), gp * i) : cfma(gp, i, kappa * rmax(zero, z));
+        };
+        // the side computed second gets its reciprocal and 1/(c_l + c_r)
+        // from one division
+        if (R.p >= L.p) {
+            w.zl = cfma(dp, w.ir, du);
+            w.c_l = L.rho * speed(gpl, w.il, w.zl);
+            w.icl = rrcp(w.c_l);
+            w.zr = cfma(-dp, w.icl, du);
+            w.c_r = R.rho * speed(gpr, w.ir, w.zr);
+            const float sc = w.c_l + w.c_r, q = rrcp(w.c_r * sc);
+            w.icr = sc * q;
+            w.isum = w.c_r * q;
+        } else {
+            w.zr = cfma(-dp, w.il, du);
+            w.c_r = R.rho * speed(gpr, w.ir, w.zr);
+            w.icr = rrcp(w.c_r);
+            w.zl = cfma(dp, w.icr, du);
+            w.c_l = L.rho * speed(gpl, w.il, w.zl);
+            const float sc = w.c_l + w.c_r, q = rrcp(w.c_l * sc);
+            w.icl = sc * q;
+            w.isum = w.c_l * q;
+        }
+        w.sl = w.c_l * w.irl;  // c/rho: the fan's edge speeds relative to u
+        w.sr = w.c_r * w.irr;
+        return w;
+    }
+    __device__ static __forceinline__ float contact_speed(float u_l, float c_l, float p_l, float u_r, float c_r, float p_r,
+                                                          float isum)
+    {
+        return (cfma(u_l, c_l, u_r * c_r) + p_l - p_r) * isum;
+    }
+    __device__ static __forceinline__ float contact_pressure(float du, float c_l, float p_l, float c_r, float p_r,
+                                                             float isum)
+    {
+        return cfma(c_r, p_l, cfma(c_l, p_r, du * c_l * c_r)) * isum;
+    }
+    template <class Consts>
+    __device__ static __forceinline__ Interface<float> grp(const Cell<float> &L, const Cell<float> &R,
+                                                           const Cell<float> &sL, const Cell<float> &sR,
+                                                           const Consts &K, bool sound = false, bool once = false)
+    {
+        const float one = 1.f, half = 0.5f, zero = 0.f, igm1 = K.igm1;
+        const float rho_l = L.rho, pi_l = L.p, u_l = L.un, v_l = L.ut;
+        const float rho_r = R.rho, pi_r = R.p, u_r = R.un, v_r = R.ut;
+        const float rho_lx = sL.rho, pi_lx = sL.p, u_lx = sL.un, v_lx = sL.ut;
+        const float rho_rx = sR.rho, pi_rx = sR.p, u_rx = sR.un, v_rx = sR.ut;
+        const Fan w = fan(L, R, sL, sR, K, sound);
+        const float irl = w.irl, irr = w.irr, c_lx = w.c_lx, c_rx = w.c_rx, c_l = w.c_l, c_r = w.c_r;
+        const float icl = w.icl, icr = w.icr, isum = w.isum, sl = w.sl, sr = w.sr;
+        const float e_l = pi_l * irl * igm1, e_r = pi_r * irr * igm1;
+        // (gamma - 1) e_x
+        const float g_lx = cfma(-(pi_l * rho_lx), irl, pi_lx) * irl, g_rx = cfma(-(pi_r * rho_rx), irr, pi_rx) * irr;
+        Interface<float> o;
+        if (u_l - sl >= zero) {
+            o.rho = rho_l; o.p = pi_l; o.un = u_l; o.ut = v_l; o.e = e_l;
+            o.rho_t = cfma(-rho_l, u_lx, -(u_l * rho_lx));
+            o.un_t = cfma(-u_l, u_lx, -(pi_lx * irl));
+            o.e_t = cfma(-u_l, g_lx * igm1, -(pi_l * irl * u_lx));
+            o.ut_t = -u_l * v_lx;
+            o.p_t = cfma(-u_l, pi_lx, -(c_l * sl * u_lx));
+        } else if (u_r + sr <= zero) {
+            o.rho = rho_r; o.p = pi_r; o.un = u_r; o.ut = v_r; o.e = e_r;
+            o.rho_t = cfma(-rho_r, u_rx, -(u_r * rho_rx));
+            o.un_t = cfma(-u_r, u_rx, -(pi_rx * irr));
+            o.e_t = cfma(-u_r, g_rx * igm1, -(pi_r * irr * u_rx));
+            o.ut_t = -u_r * v_rx;
+            o.p_t = cfma(-u_r, pi_rx, -(c_r * sr * u_rx));
+        } else {
+            const float u = contact_speed(u_l, c_l, pi_l, u_r, c_r, pi_r, isum);
+            const float pm = contact_pressure(u_l - u_r, c_l, pi_l, c_r, pi_r, isum);
+            const float cu_l = c_l * u_lx, cu_r = c_r * u_rx;
+            const float f_r = once ? cfma(c_r, u_rx, -pi_rx) : cu_r - pi_rx;
+            const float k_l = cfma(-(half * u_l), c_lx, -pi_lx - cu_l);
+            const float k_r = cfma(half * u_r, c_rx, f_r);
+            const float d_l = sl * cfma(-2.f, cu_l + pi_lx, -(u_l * c_lx));
+            const float d_r = sr * cfma(u_r, c_rx, 2.f * f_r);
+            const float Dp = cfma(c_r, d_l, -(c_l * d_r)) * half * isum;
+            o.p = pm;
+            o.un = u;
+            if (u <= zero) {
+                const float irho = (u_r - u + sr) * icr;
+                const float rho = rrcp(irho), icr2 = icr * icr;
+                const float e = cfma((pm - pi_r) * (pm + pi_r) * half, icr2, e_r);
+                const float rho3 = rho * rho * rho, urho = u * rho;
+                const float h_l = cfma(urho, icr, one), h_r = cfma(-urho, icl, one);
+                const float S = cfma(1.5f * (u - u_r), c_rx, cfma(sr * sr, rho_rx, -cu_r));
+                const float G = cfma(2.f * (e_r - e) * c_rx, icr, cfma(g_rx, igm1, -(pi_r * pi_rx * icr2)));
+                o.rho = rho; o.e = e; o.ut = v_r;
+                o.rho_t = cfma(rho3 * icr2 * icr * cfma(c_r, irho, u), Dp, -u * rho3 * irr * icr2 * S);
+                o.p_t = isum * cfma(c_r * sl * h_l, k_l, -(c_l * sr * h_r * k_r));
+                o.un_t = isum * cfma(sl * h_l, k_l, sr * cfma(-(urho * c_l), icr2, one) * k_r);
+                o.e_t = cfma(-urho * irr, G, pm * icr2 * o.p_t);
+                o.ut_t = -urho * irr * v_rx;
+            } else {
+                const float irho = (u - u_l + sl) * icl;
+                const float rho = rrcp(irho), icl2 = icl * icl;
+                const float e = cfma((pm - pi_l) * (pm + pi_l) * half, icl2, e_l);
+                const float rho3 = rho * rho * rho, urho = u * rho;
+                const float h_l = cfma(urho, icr, one), h_r = cfma(-urho, icl, one);
+                const float S = cfma(1.5f * (u - u_l), c_lx, cfma(sl * sl, rho_lx, cu_l));
+                const float G = cfma(2.f * (e_l - e) * c_lx, icl, cfma(g_lx, igm1, -(pi_l * pi_lx * icl2)));
+                o.rho = rho; o.e = e; o.ut = v_l;
+                o.rho_t = cfma(-u * rho3 * irl * icl2, S, -(rho3 * icl2 * icl * cfma(-c_l, irho, u) * Dp));
+                o.p_t = isum * cfma(c_r * sl * h_l, k_l, -(c_l * sr * h_r * k_r));
+                o.un_t = isum * cfma(sr * h_r, k_r, sl * cfma(urho * c_r, icl2, one) * k_l);
+                o.e_t = cfma(-urho * irl, G, pm * icl2 * o.p_t);
+                o.ut_t = -urho * irl * v_lx;
+            }
+        }
+        return o;
+    }
+
     // F + k/2 dF/dt through m = rho u and m_t = d(rho u)/dt (the product rule
     // applied to src/basicFuns.cuh:28-33), gathered around the midpoint mass
     // flux M = m + k/2 m_t and pressure Q = p + k/2 p_t.
@@ -587,20 +739,25 @@ struct Hoisted {
         const Real et = fma(w.un, w.un_t, fma(w.ut, w.ut_t, w.e_t));
         Cell<Real> F;
         F.rho = M;
-        if constexpr (std::is_same<Real, float>::value) {
-            // the time derivatives' parts, small where the flow is smooth, are
-            // summed first: two full-size roundings a flux instead of three
-            // and four (with Q, a residual build's velocities ended 20% further
-            // from FP64 on a shock-bubble flow; 0.7% of its step)
-            const Real dp = hk * w.p_t;
-            F.p = fma(M, w.un, w.p) + fma(hm, w.un_t, dp);
-            F.un = fma(es, M, fma(w.un, w.p, fma(hm, et, fma(w.un, dp, (hk * w.p) * w.un_t))));
-        } else {
-            const Real Q = fma(hk, w.p_t, w.p);
-            F.p = fma(M, w.un, fma(hm, w.un_t, Q));
-            F.un = fma(es, M, fma(hm, et, fma(w.un, Q, (hk * w.p) * w.un_t)));
-        }
+        const Real Q = fma(hk, w.p_t, w.p);
+        F.p = fma(M, w.un, fma(hm, w.un_t, Q));
+        F.un = fma(es, M, fma(hm, et, fma(w.un, Q, (hk * w.p) * w.un_t)));
         F.ut = fma(M, w.ut, hm * w.ut_t);
+        return F;
+    }
+    // and term by term in single precision (grp)
+    template <class Consts>
+    __device__ static __forceinline__ Cell<float> flux_of(const Interface<float> &w, const Consts &K)
+    {
+        const float hk = half_k(K);
+        const float m = w.rho * w.un, m_t = cfma(w.un, w.rho_t, w.rho * w.un_t);
+        const float es = cfma(0.5f, cfma(w.un, w.un, w.ut * w.ut), w.e);
+        const float et = cfma(w.ut, w.ut_t, cfma(w.un, w.un_t, w.e_t));
+        Cell<float> F;
+        F.rho = cfma(hk, m_t, m);
+        F.p = cfma(hk, cfma(m, w.un_t, m_t * w.un) + w.p_t, cfma(m, w.un, w.p));
+        F.un = cfma(hk, cfma(w.p, w.un_t, cfma(w.p_t, w.un, cfma(m_t, es, m * et))), cfma(w.p, w.un, m * es));
+        F.ut = cfma(m, w.ut, hk * cfma(m, w.ut_t, m_t * w.ut));
         return F;
     }
 

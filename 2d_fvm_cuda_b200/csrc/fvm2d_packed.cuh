@@ -7,7 +7,9 @@
 // pairs or the relaxation GRP's left/right set-up as well was measured
 // slower (the pairing moves and registers cost more than they save), so the
 // GRP and limiter stay those of HoistedCompensated.  Same mathematics as
-// HoistedCompensated; rounding differs at the FP32 ulp level.
+// HoistedCompensated; rounding differs at the FP32 ulp level.  Steps in tiles
+// at 4096^2 (varied four-quadrant flow): 1.20 ms in FP32, where the shared
+// grouping of the FP64 build (Hoisted::grp) took 1.09 with other roundings.
 #pragma once
 
 #include "fvm2d_math.cuh"
@@ -34,7 +36,7 @@ struct PackedCompensated : HoistedCompensated {
     template <class Consts>
     __device__ static __forceinline__ Cell<float> interface_flux(const Cell<float> &UL, const Cell<float> &UR,
                                                                  const Cell<float> &sL, const Cell<float> &sR,
-                                                                 const Consts &K)
+                                                                 const Consts &K, bool sound = false, bool once = false)
     {
         const float h2 = half_h(K);
         const float2 hh = p2(h2, h2), mh = p2(-h2, -h2);
@@ -43,7 +45,7 @@ struct PackedCompensated : HoistedCompensated {
         const float2 r01 = fma2(p2(sR.rho, sR.p), mh, p2(UR.rho, UR.p));
         const float2 r23 = fma2(p2(sR.un, sR.ut), mh, p2(UR.un, UR.ut));
         const Cell<float> fL = {l01.x, l01.y, l23.x, l23.y}, fR = {r01.x, r01.y, r23.x, r23.y};
-        return flux_of(grp(fL, fR, sL, sR, K), K);
+        return flux_of(grp(fL, fR, sL, sR, K, sound, once), K);
     }
 
     // HoistedCompensated::update with the conserved vector handled as the
@@ -99,6 +101,17 @@ struct PackedCompensated : HoistedCompensated {
     }
 };
 
+// The FP32 physics of batches: the solver's but for one rounding along y.
+struct PackedBatch : PackedCompensated {
+    template <class Consts>
+    __device__ static __forceinline__ Cell<float> sweep_flux(bool y, bool, const Cell<float> &UL, const Cell<float> &UR,
+                                                             const Cell<float> &sL, const Cell<float> &sR,
+                                                             const Consts &K)
+    {
+        return interface_flux(UL, UR, sL, sR, K, false, y);
+    }
+};
+
 // The FP32 physics of the build with residual planes (FVM2D_FP32_RESIDUAL):
 // slopes and fluxes from the FP32 values as PackedCompensated computes them;
 // the conservative update of a cell from its stored hi + lo in FP64, with
@@ -108,9 +121,18 @@ struct PackedCompensated : HoistedCompensated {
 // is otherwise idle in these sweeps.)
 struct PackedResidual : PackedCompensated {
     static constexpr bool kSplitStorage = true;
-    template <class Flux, class Consts>
+    template <class Consts>
+    __device__ static __forceinline__ Cell<float> sweep_flux(bool, bool last, const Cell<float> &UL,
+                                                             const Cell<float> &UR, const Cell<float> &sL,
+                                                             const Cell<float> &sR, const Consts &K)
+    {
+        return interface_flux(UL, UR, sL, sR, K, !last);
+    }
+    // (average: the mean of the result and branch A, the step's last sweep)
+    template <bool AVERAGE = false, class Flux, class Consts>
     __device__ static __forceinline__ Cell<double> update_split(const Cell<double> &U, const Cell<Flux> &FL,
-                                                                const Cell<Flux> &FR, const Consts &K)
+                                                                const Cell<Flux> &FR, const Consts &K,
+                                                                const Cell<double> &branch_a = {})
     {
         const double rho = U.rho, p = U.p, un = U.un, ut = U.ut;
         const double lam = joined_lambda(K), igm1 = joined_igm1(K), gm1 = joined_gm1(K);
@@ -129,7 +151,11 @@ struct PackedResidual : PackedCompensated {
         o.rho = m0;
         o.un = m1 * ir;
         o.ut = m3 * ir;
-        o.p = gm1 * fma(-0.5, fma(m1, o.un, m3 * o.ut), m2);
+        const double ei = fma(-0.5, fma(m1, o.un, m3 * o.ut), m2);
+        if constexpr (AVERAGE)
+            return {(branch_a.rho + o.rho) * 0.5, fma(gm1, ei, branch_a.p) * 0.5, (branch_a.un + o.un) * 0.5,
+                    (branch_a.ut + o.ut) * 0.5};
+        o.p = gm1 * ei;
         return o;
     }
 };

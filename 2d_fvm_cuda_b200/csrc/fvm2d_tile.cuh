@@ -321,19 +321,24 @@ __device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int b
         }
     }
 
-    // the step's result at tile cell (r, c): branch A (sU, lU) averaged with
-    // branch B in primitive variables (src/basicFuns.cuh:264-274)
-    auto finish = [&](int r, int c, auto b) {
-        const int x = x0 - 2 + c, y = y0 - 2 + r;
+    // branch A's result at tile cell (r, c)
+    auto branch_a = [&](int r, int c) {
         const Real *const ra = sU + r * RS + c;
         const Cell<Real> A = {ra[0], ra[NC], ra[2 * NC], ra[3 * NC]};
+        if constexpr (kResidual)
+            return join_cell(A, lo_parts(lU[r * T::kLo + c], false));
+        else
+            return A;
+    };
+    // the step's result there: branch A averaged with branch B in primitive
+    // variables (src/basicFuns.cuh:264-274); residual builds: averaged already
+    auto finish = [&](int r, int c, auto b) {
+        const int x = x0 - 2 + c, y = y0 - 2 + r;
         Cell<Real> o;
         if constexpr (kResidual) {
-            const Cell<double> d = join_cell(A, lo_parts(lU[r * T::kLo + c], false));
-            o = store_split(a.dst, x, y, 2, 3,
-                            Cell<double>{(d.rho + b.rho) * 0.5, (d.p + b.p) * 0.5, (d.un + b.un) * 0.5,
-                                         (d.ut + b.ut) * 0.5});
+            o = store_split(a.dst, x, y, 2, 3, b);
         } else {
+            const Cell<Real> A = branch_a(r, c);
             o.rho = (A.rho + b.rho) * Real(0.5);
             o.p = (A.p + b.p) * Real(0.5);
             o.un = (A.un + b.un) * Real(0.5);
@@ -379,7 +384,7 @@ __device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int b
             {
                 const Cell<Real> cm1 = get(q - s), c0 = get(q);
                 s0 = Phys::slope(cm1, c0, get(q + s), K);
-                F = Phys::interface_flux(cm1, c0, shfl_up(s0), s0, K);
+                F = sweep_flux<Phys>(!xdir, phase == 2, cm1, c0, shfl_up(s0), s0, K);
             }
             // (a residual build's update takes them in FP64: widened once, four
             // conversions a task less than after the shuffle)
@@ -396,16 +401,24 @@ __device__ __forceinline__ bool tile_step(const TileArgs<Real> &a, int bx, int b
                 if (mine && k >= 1 && in) store_cell(tape->F[phase == 0 ? (xdir ? 0 : 1) : xdir ? 3 : 2], x, y, 2, 3, F);
             }
             if (!mine || k < 2) continue;
+            auto old = [&] {
+                if constexpr (kResidual)
+                    return join_cell(get(q - s), lo_parts((phase == 0 ? lU : xdir ? lB : lA)[ru * T::kLo + cu], !xdir));
+                else
+                    return get(q - s);
+            };
             auto updated = [&] {
                 if constexpr (kResidual)
-                    return Phys::update_split(
-                        join_cell(get(q - s), lo_parts((phase == 0 ? lU : xdir ? lB : lA)[ru * T::kLo + cu], !xdir)), FL,
-                        FR, K);
+                    return Phys::update_split(old(), FL, FR, K);
                 else
-                    return Phys::update(get(q - s), FL, FR, K);
+                    return Phys::update(old(), FL, FR, K);
             };
             if (!MERGE && phase == 2) {
-                if (x0 - 2 + cu <= a.nx - 3) finish(ru, cu, updated());
+                if (x0 - 2 + cu > a.nx - 3) continue;
+                if constexpr (kResidual)
+                    finish(ru, cu, Phys::template update_split<true>(old(), FL, FR, K, branch_a(ru, cu)));
+                else
+                    finish(ru, cu, updated());
                 continue;
             }
             Real *const d = (phase == 0 ? (xdir ? sA : sB) : xdir ? sR : sU) + ru * RS + cu;

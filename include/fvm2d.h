@@ -337,7 +337,8 @@ int fvm2d_set_vjp_overlap(fvm2d_solver *s, int on);
  * one launch covering all problems, each problem with its own dt, end time
  * and ghost preset, and the host only reads the control records now and
  * then.  Results match the same problems solved one by one with the same
- * precision bit for bit. */
+ * precision, bit for bit with FVM2D_FP64 and FVM2D_FP64_STRICT, to rounding
+ * with the others. */
 typedef struct fvm2d_batch fvm2d_batch;
 
 /* A batch of nproblems problems; problem p is nx[p] x ny[p] cells (ghosts
