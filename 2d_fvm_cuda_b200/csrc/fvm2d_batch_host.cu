@@ -527,8 +527,9 @@ int fvm2d_batch_set_precision(fvm2d_batch *b, int precision)
     if (precision < 0 || precision >= kNumBatchVariants) return fail(FVM2D_ERR_INVALID, "unknown precision");
     if ((precision == FVM2D_FP32) != (b->precision == FVM2D_FP32)) {
         if (int rc = b->convert_states(precision)) return rc;
-        b->dirty = true;  // element offsets depend on the storage type
     }
+    // element offsets depend on the storage type, tiles on the build
+    if (precision != b->precision) b->dirty = true;
     b->precision = precision;
     b->drop_graphs();
     return FVM2D_OK;
