@@ -542,6 +542,19 @@ __device__ __forceinline__ void commit_record(StepControl *ctl, const TileRecord
 }
 
 #ifdef __CUDACC__  // (host builds of this file call tile_step)
+// A block per tile.  A grid's second dimension ends at 65535; the tile rows of
+// an array of more (30 cells each: 1,966,054 rows) go on in the third, whose
+// last layer has blocks past the end.  (One dimension and a division per block
+// measured 0.3% slower at 4096^2.)
+constexpr int kTileRowsPerLayer = 65535;
+template <class T>
+dim3 tile_grid(int nx, int ny)
+{
+    const int rows = (ny - 4 + T::TY - 1) / T::TY, layers = (rows + kTileRowsPerLayer - 1) / kTileRowsPerLayer;
+    return dim3((nx - 4 + T::TX - 1) / T::TX, rows < kTileRowsPerLayer ? rows : kTileRowsPerLayer, layers);
+}
+__device__ __forceinline__ int tile_row() { return int(blockIdx.y) + kTileRowsPerLayer * int(blockIdx.z); }
+
 // Step `place` of its group.
 template <typename Real, class Phys, class T, int MINB>
 __global__ void __launch_bounds__(T::NT, MINB) step_tile_kernel(TileArgs<Real> a, int place)
@@ -549,10 +562,12 @@ __global__ void __launch_bounds__(T::NT, MINB) step_tile_kernel(TileArgs<Real> a
     extern __shared__ __align__(16) unsigned char tile_smem[];
     pdl_launch();
     pdl_wait();
-    const bool first = blockIdx.x == 0 && blockIdx.y == 0;
+    const int by = tile_row();
+    if (by >= (a.ny - 4 + T::TY - 1) / T::TY) return;
+    const bool first = blockIdx.x == 0 && by == 0;
     double vmax = first && threadIdx.x == 0 ? ring_speed<Real>(a.strategy, a.gamma) : 0.0;
     int bad = 0;
-    if (tile_step<Real, Phys, T>(a, blockIdx.x, blockIdx.y, tile_smem,
+    if (tile_step<Real, Phys, T>(a, blockIdx.x, by, tile_smem,
                                  [&] { return begin_tile(a.ctl, place & 1, a.plan, first); }, place > 0, vmax, bad))
         end_tile<T::NT>(vmax, bad, a.ctl, reinterpret_cast<TileHead<Real, Phys> *>(tile_smem)->step.steps);
 }
@@ -564,10 +579,12 @@ __global__ void __launch_bounds__(T::NT, MINB) step_tape_kernel(TileArgs<Real> a
     extern __shared__ __align__(16) unsigned char tile_smem[];
     pdl_launch();
     pdl_wait();
-    const bool first = blockIdx.x == 0 && blockIdx.y == 0;
+    const int by = tile_row();
+    if (by >= (a.ny - 4 + T::TY - 1) / T::TY) return;
+    const bool first = blockIdx.x == 0 && by == 0;
     double vmax = first && threadIdx.x == 0 ? ring_speed<Real>(a.strategy, a.gamma) : 0.0;
     int bad = 0;
-    if (tile_step<Real, Phys, T, true>(a, blockIdx.x, blockIdx.y, tile_smem,
+    if (tile_step<Real, Phys, T, true>(a, blockIdx.x, by, tile_smem,
                                        [&] { return begin_tile(a.ctl, place & 1, a.plan, first); }, place > 0, vmax, bad,
                                        &tape))
         end_tile<T::NT>(vmax, bad, a.ctl, reinterpret_cast<TileHead<Real, Phys> *>(tile_smem)->step.steps);
