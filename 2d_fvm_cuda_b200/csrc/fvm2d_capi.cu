@@ -405,8 +405,8 @@ int check(fvm2d_solver *s)
 int upload(fvm2d_solver *s, const double *cells, int stride)
 {
     const double *src = cells;
-    if (!is_memory_of(cells, s->device)) {
-        const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
+    const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
+    if (!is_memory_of(cells, bytes, s->device)) {
         const cudaMemcpyKind kind = is_device_pointer(cells) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         CK(cudaMemcpyAsync(s->scratch, cells, bytes, kind, s->stream));
         src = s->scratch;
@@ -580,8 +580,9 @@ int fvm2d_set_state_planes(fvm2d_solver *s, const double *planes)
     if (int rc = check(s)) return rc;
     if (!planes) return fail(FVM2D_ERR_INVALID, "null state pointer");
     const double *src = planes;
-    if (!is_memory_of(planes, s->device)) {
-        CK(cudaMemcpyAsync(s->scratch, planes, sizeof(double) * 4 * (size_t)s->nx * s->ny, cudaMemcpyDefault, s->stream));
+    const size_t bytes = sizeof(double) * 4 * (size_t)s->nx * s->ny;
+    if (!is_memory_of(planes, bytes, s->device)) {
+        CK(cudaMemcpyAsync(s->scratch, planes, bytes, cudaMemcpyDefault, s->stream));
         src = s->scratch;
     }
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
@@ -630,14 +631,14 @@ int fvm2d_get_state(fvm2d_solver *s, double *cells, int stride)
     if (!cells) return fail(FVM2D_ERR_INVALID, "null state pointer");
     if (stride != 4 && stride != 5) return fail(FVM2D_ERR_INVALID, "stride must be 4 or 5 doubles per cell");
     if (!s->have_state) return fail(FVM2D_ERR_STATE, "no state has been set");
-    const bool direct = is_memory_of(cells, s->device);
+    const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
+    const bool direct = is_memory_of(cells, bytes, s->device);
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
         soa_to_aos<<<148 * 4, 256, 0, s->stream>>>(st, s->nx, s->ny, s->pitch, s->plane, stride,
                                                    direct ? cells : s->scratch);
     });
     CK(cudaGetLastError());
     if (!direct) {
-        const size_t bytes = sizeof(double) * (size_t)s->nx * s->ny * stride;
         const cudaMemcpyKind kind = is_device_pointer(cells) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
         CK(cudaMemcpyAsync(cells, s->scratch, bytes, kind, s->stream));
     }
@@ -830,14 +831,14 @@ static int rows_check(fvm2d_solver *s, int j0, int nrows, const void *buf)
 int fvm2d_get_rows(fvm2d_solver *s, int j0, int nrows, double *rows)
 {
     if (int rc = rows_check(s, j0, nrows, rows)) return rc;
-    const bool direct = is_memory_of(rows, s->device);
+    const size_t bytes = sizeof(double) * 4 * (size_t)nrows * s->nx;
+    const bool direct = is_memory_of(rows, bytes, s->device);
     with_planes(s->precision, s->U, s->plane, [&](auto st) {
         rows_out<<<rows_grid(nrows, s->nx), kRowThreads, 0, s->stream>>>(st, s->plane, s->pitch, j0, nrows, s->nx,
                                                                          direct ? rows : s->scratch);
     });
     CK(cudaGetLastError());
-    if (!direct)
-        CK(cudaMemcpyAsync(rows, s->scratch, sizeof(double) * 4 * (size_t)nrows * s->nx, cudaMemcpyDefault, s->stream));
+    if (!direct) CK(cudaMemcpyAsync(rows, s->scratch, bytes, cudaMemcpyDefault, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return FVM2D_OK;
 }
@@ -846,8 +847,9 @@ int fvm2d_set_rows(fvm2d_solver *s, int j0, int nrows, const double *rows)
 {
     if (int rc = rows_check(s, j0, nrows, rows)) return rc;
     const double *src = rows;
-    if (!is_memory_of(rows, s->device)) {
-        CK(cudaMemcpyAsync(s->scratch, rows, sizeof(double) * 4 * (size_t)nrows * s->nx, cudaMemcpyDefault, s->stream));
+    const size_t bytes = sizeof(double) * 4 * (size_t)nrows * s->nx;
+    if (!is_memory_of(rows, bytes, s->device)) {
+        CK(cudaMemcpyAsync(s->scratch, rows, bytes, cudaMemcpyDefault, s->stream));
         src = s->scratch;
     }
     with_planes(s->precision, s->U, s->plane, [&](auto st) {

@@ -5,6 +5,7 @@
 // whose get/put convert element k to and from double.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <stdint.h>
@@ -148,17 +149,38 @@ inline bool is_device_pointer(const void *p)
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-// True for memory allocated on `device` itself: what a kernel there may read
-// and write in place.  (Memory of another device, managed memory or an odd
-// address goes through a copy.)
-inline bool is_memory_of(const void *p, int device)
+// The bytes from p to the end of the device allocation that holds it (0 where
+// the driver does not say).
+inline size_t bytes_from(const void *p)
+{
+    using Range = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
+    static const Range range = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &found);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<Range>(f) : nullptr;
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+    if (!range || range(&base, &size, at) != CUDA_SUCCESS || at < base || at - base > size) return 0;
+    return size - size_t(at - base);
+}
+
+// True for `bytes` at p of memory allocated on `device` itself: what a kernel
+// there may read and write in place.  Memory of another device, managed memory,
+// an odd address, or a buffer that ends before (or goes on in another mapping)
+// goes through a copy, which checks its ranges.
+inline bool is_memory_of(const void *p, size_t bytes, int device)
 {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == device && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0;
+    return a.type == cudaMemoryTypeDevice && a.device == device && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0 &&
+           bytes_from(p) >= bytes;
 }
 
 } // namespace fvm2d

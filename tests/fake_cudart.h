@@ -4,6 +4,7 @@
 // Linked in place of the runtime with objects that nvcc compiled.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
@@ -20,6 +21,35 @@ inline double clock_ms = 0.0;
 inline int captured = -1;                     // steps captured so far; -1: no capture
 inline cudaError_t (*graph_launch)(long) = nullptr;  // a graph of that many captured steps
 inline int resident = 4;                      // blocks per SM that the occupancy call answers
+
+// buffers that count as a caller's device memory, and the copies from and to them
+struct Range {
+    char *base;
+    size_t size;
+};
+inline std::vector<Range> device;
+inline long device_copies = 0;
+inline Range *holding(const void *p)
+{
+    for (Range &r : device)
+        if (p >= r.base && p < r.base + r.size) return &r;
+    return nullptr;
+}
+// As the runtime's copy checks: both ends inside their allocation.
+inline bool copies(const void *p, size_t n)
+{
+    Range *r = holding(p);
+    if (!r) return true;
+    ++device_copies;
+    return n <= size_t(r->base + r->size - static_cast<const char *>(p));
+}
+inline CUresult address_range(CUdeviceptr *base, size_t *size, CUdeviceptr p)
+{
+    Range *r = holding(reinterpret_cast<void *>(p));
+    if (!r) return CUDA_ERROR_NOT_FOUND;
+    *base = reinterpret_cast<CUdeviceptr>(r->base), *size = r->size;
+    return CUDA_SUCCESS;
+}
 
 // As the runtime's launch checks: the grid's limits.
 inline cudaError_t note(dim3 grid, dim3 block, size_t smem)
@@ -45,9 +75,29 @@ cudaError_t cudaMalloc(void **p, size_t n) { *p = std::calloc(n ? n : 1, 1); ret
 cudaError_t cudaFree(void *p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeHost(void *p) { return cudaFree(p); }
-cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) { std::memmove(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t)
+{
+    if (!fake::copies(d, n) || !fake::copies(s, n)) return cudaErrorInvalidValue;
+    std::memmove(d, s, n);
+    return cudaSuccess;
+}
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t) { std::memset(d, v, n); return cudaSuccess; }
-cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) { std::memset(a, 0, sizeof *a); return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p)
+{
+    std::memset(a, 0, sizeof *a);
+    if (fake::holding(p)) a->type = cudaMemoryTypeDevice;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDriverEntryPoint(const char *name, void **f, unsigned long long, cudaDriverEntryPointQueryResult *found)
+{
+    const bool known = !std::strcmp(name, "cuMemGetAddressRange");
+    *f = known ? reinterpret_cast<void *>(fake::address_range) : nullptr;
+    *found = known ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
+    return cudaSuccess;
+}
+cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { *f = *t = size_t(1) << 33; return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { *e = reinterpret_cast<cudaEvent_t>(new double(0)); return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
