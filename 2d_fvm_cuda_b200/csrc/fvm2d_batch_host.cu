@@ -628,43 +628,48 @@ int fvm2d_batch_autotune(fvm2d_batch *b, int trial_steps, int *segment_interface
         }
         return cudaStreamSynchronize(b->stream);
     };
-    cudaError_t e = copy_states(true);
-    int best_T = b->T, best_g = 0;
-    double best = 1e300;
+    const bool was_tiles = b->use_tiles;
+    const int was_T = b->T, was_x = b->grid_x, was_y = b->grid_y;
     int rc = FVM2D_OK;
-    const int Ts[] = {16, 32, 64};
-    const int mults[] = {1, 2, 4};
-    bool best_tiles = false;
-    double sweeps = 1e300;
-    if (!e) {  // a step in tiles
-        b->use_tiles = true;
+    cudaError_t e = copy_states(true);
+    // a trial's device time; the states are as before it
+    auto trial = [&](double &ms) {
         b->dirty = true;
-        if (!(rc = b->run(trial_steps))) {
-            best = b->last_device_ms;
-            best_tiles = true;
+        if (!e && !rc && !(rc = b->run(trial_steps))) {
+            ms = b->last_device_ms;
             e = copy_states(false);
         }
-        b->use_tiles = false;
-    }
-    for (int ti = 0; ti < 3 && !e && !rc; ++ti)
-        for (int mi = 0; mi < 3 && !e && !rc; ++mi) {
+        return !e && !rc;
+    };
+    int best_T = b->T, best_g = 0;
+    const int Ts[] = {16, 32, 64};
+    const int mults[] = {1, 2, 4};
+    // steps in tiles, once before they are timed: what a first run costs (the
+    // kernels' loading, clocks) is no candidate's
+    double tiles = 1e300, sweeps = 1e300, ms = 0.0;
+    b->use_tiles = true;
+    if (trial(ms)) trial(tiles);
+    b->use_tiles = false;
+    for (int ti = 0; ti < 3; ++ti)
+        for (int mi = 0; mi < 3; ++mi) {
             b->T = Ts[ti];
             b->grid_x = mults[mi] * b->occ_x;
             b->grid_y = mults[mi] * b->occ_y;
-            b->dirty = true;
-            if ((rc = b->run(trial_steps))) break;
-            const double ms = b->last_device_ms;
-            if (ms < sweeps) sweeps = ms, best_T = Ts[ti], best_g = mults[mi];
-            e = copy_states(false);
+            if (trial(ms) && ms < sweeps) sweeps = ms, best_T = Ts[ti], best_g = mults[mi];
         }
     cudaFree(saved);
-    b->use_tiles = best_tiles && best <= sweeps;
-    if (rc) return rc;
-    if (e) return cuda_fail(e, "state copy during tuning");
+    b->dirty = true;  // the last trial's plan is not the one to keep
+    if (rc || e) {
+        b->use_tiles = was_tiles;
+        b->T = was_T;
+        b->grid_x = was_x;
+        b->grid_y = was_y;
+        return rc ? rc : cuda_fail(e, "state copy during tuning");
+    }
+    b->use_tiles = tiles <= sweeps;
     b->T = best_T;
     b->grid_x = best_g * b->occ_x;
     b->grid_y = best_g * b->occ_y;
-    b->dirty = true;
     std::memset(b->ctl_h, 0, sizeof(StepControl) * b->np);
     if (segment_interfaces) *segment_interfaces = best_T;
     if (grid_blocks) *grid_blocks = b->grid_x;

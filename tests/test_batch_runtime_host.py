@@ -69,3 +69,29 @@ def test_steps_follow_the_precision_set_last(lib, batch, apart):
         assert lib.fvm2d_batch_solve(batch) == 0
         got = seen(lib)
         assert got["tiles"] > 0 and got["wrong_plan"] == 0 and got["mixed"] == 0, (precision, got)
+
+
+def test_autotuning_times_no_first_run(lib, batch):
+    """Tiles that are faster are kept although the process's first run, which is
+    in tiles, costs more than any sweep."""
+    lib.br_set(2.0, 1.0, 500.0, -1, 0)
+    assert lib.fvm2d_batch_autotune(batch, 2, None, None) == 0
+    lib.br_set(2.0, 1.0, 0.0, -1, 0)
+    assert lib.fvm2d_batch_solve(batch) == 0
+    assert seen(lib) == {"tiles": 32, "sweeps": 0, "wrong_plan": 0, "mixed": 0}
+    lib.br_set(1.0, 2.0, 0.0, -1, 0)
+    assert lib.fvm2d_batch_autotune(batch, 2, None, None) == 0
+    lib.br_set(1.0, 2.0, 0.0, -1, 0)
+    assert lib.fvm2d_batch_solve(batch) == 0
+    assert seen(lib) == {"tiles": 0, "sweeps": 32, "wrong_plan": 0, "mixed": 0}
+
+
+@pytest.mark.parametrize("trial", [0, 4, 17])
+def test_a_failed_autotuning_leaves_the_batch_as_it_was(lib, batch, trial):
+    """An error in any of the sweeps' trials is returned, and the next solve steps
+    as the ones before."""
+    lib.br_set(2.0, 1.0, 0.0, trial, 0)
+    assert lib.fvm2d_batch_autotune(batch, 2, None, None) != 0
+    lib.br_set(2.0, 1.0, 0.0, -1, 0)
+    assert lib.fvm2d_batch_solve(batch) == 0
+    assert seen(lib) == {"tiles": 32, "sweeps": 0, "wrong_plan": 0, "mixed": 0}
