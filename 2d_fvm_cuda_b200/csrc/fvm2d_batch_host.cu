@@ -324,7 +324,9 @@ struct fvm2d_batch {
         CK(cudaEventRecord(ev0, stream));
         CK(kBatchVariants[precision].init(L, stream));
         long long launches = 1;
-        long long budget = limit, ahead = kGraphSteps[0];
+        long long cells = 0;
+        for (int p = 0; p < np; ++p) cells += (long long)nx[p] * ny[p];
+        long long budget = limit, ahead = fvm2d::first_group(cells);
         for (;;) {
             if (use_tiles) {
                 const int n = (int)std::max(1ll, std::min(ahead, budget));

@@ -154,6 +154,14 @@ void with_planes(int precision, const void *state, long long plane, F &&f)
 
 int fvm2d::report_error(int code, const char *msg) { return fail(code, msg); }
 
+// The record as it stands, to the host's pinned mirror.
+static __global__ void show_record(const StepControl *c, StepControl *host)
+{
+    static_assert(sizeof(StepControl) % 4 == 0 && sizeof(StepControl) / 4 <= 64, "one word a thread");
+    if (threadIdx.x < sizeof(StepControl) / 4)
+        reinterpret_cast<unsigned *>(host)[threadIdx.x] = reinterpret_cast<const unsigned *>(c)[threadIdx.x];
+}
+
 struct fvm2d_solver {
     int device = 0;
     int nx = 0, ny = 0, pitch = 0;
@@ -168,8 +176,7 @@ struct fvm2d_solver {
     double *scratch = nullptr;  // the other two: A then B
     StepControl *ctl = nullptr;
     StepControl *ctl_h = nullptr;  // pinned mirror
-    // steps enqueued between two reads of the control record, at most: a run
-    // that ends early leaves up to that many empty steps
+    // steps enqueued between two reads of the control record, at most
     static constexpr int kStepsPerRead = 128;
     cudaGraphExec_t slab_graph = nullptr;  // one step in place, for fvm2d_slab_step, dropped by every setter
     int slab_flip = 0;                     // the state's buffer it was captured with
@@ -221,9 +228,10 @@ struct fvm2d_solver {
     // (its halo rows pass through the sweeps, and its caller enqueues steps
     // without knowing whether the loop has ended).
     bool tiles() const { return ny_global == 0; }
-    // Enqueues n steps and, in tiles, their end (the record committed and the
-    // ghost ring stored): a group of steps.
-    int enqueue_steps(long long n, cudaEvent_t *ev = nullptr);
+    // Enqueues a group of steps: its steps from .. to - 1 and, in tiles and
+    // unless it is left open for more, their end (the record committed and the
+    // ghost ring stored).
+    int enqueue_steps(long long to, cudaEvent_t *ev = nullptr, long long from = 0, bool open = false);
     int step_kernels() const { return tiles() ? 1 : fvm2d::kStepKernels; }
     // m steps were enqueued, all of which run
     void stepped(int m)
@@ -326,23 +334,45 @@ struct fvm2d_solver {
         });
     }
 
+    // The steps a run has left by its last record at most, as far as its step
+    // size tells.
+    long long steps_left() const
+    {
+        if (fixed_dt > 0.0) return kStepsPerRead;  // ends at its step limit
+        const double left = (t_end - ctl_h->t) / ctl_h->dt;  // NaN: a whole group
+        return left < kStepsPerRead ? (long long)left + 1 : kStepsPerRead;
+    }
+
     // Enqueues groups of steps until the control record says no step is in
     // flight.  The record on the device must already be planned; `first`
     // kernels (init or plan) were enqueued just before.  `budget` bounds the
     // steps this loop may start.  The record is read after as many steps as
     // the run is known to have left: the budget, or the remaining time over
-    // the last step size, and at most kStepsPerRead.  Steps are launched one
-    // by one: a launch takes the host 2 us and the smallest step the device
-    // 6, and the graphs that would stand for them cost a handle's first run
-    // 0.3 ms.
+    // the last step size, and at most kStepsPerRead.  What a run that may end
+    // early has left is read from its first plan while the first few steps are
+    // under way.  Steps are launched one by one: a launch takes the host 2 us
+    // and the smallest step the device 6, and the graphs that would stand for
+    // them cost a handle's first run 0.3 ms.
     int loop(int first, long long budget)
     {
         auto t0 = std::chrono::high_resolution_clock::now();
         long long launches = first;
-        long long ahead = budget < LLONG_MAX ? kStepsPerRead : 16;
-        for (;;) {
-            const long long n = std::max(1ll, std::min(ahead, budget));
-            if (int rc = enqueue_steps(n)) return rc;
+        long long n = std::max(1ll, std::min<long long>(kStepsPerRead, budget));
+        const long long few = fvm2d::first_group((long long)nx * ny);
+        const bool may_end = fixed_dt == 0.0 && n > few;
+        if (may_end) {
+            // (a kernel into pinned memory: with a copy between the plan and the
+            // first step 100^2 solves took 14 us more)
+            show_record<<<1, 64, 0, stream>>>(ctl, ctl_h);
+            CK(cudaGetLastError());
+            CK(cudaEventRecord(ev_end, stream));
+            ++launches;
+            if (int rc = enqueue_steps(few, nullptr, 0, true)) return rc;
+            CK(cudaEventSynchronize(ev_end));
+            n = std::max(few, ctl_h->active ? std::min(budget, steps_left()) : 0);
+        }
+        for (long long from = may_end ? few : 0;; from = 0) {
+            if (int rc = enqueue_steps(n, nullptr, from)) return rc;
             budget -= n;
             launches += n * step_kernels() + tiles();
             CK(cudaEventRecord(ev_end, stream));
@@ -350,11 +380,7 @@ struct fvm2d_solver {
             CK(cudaStreamSynchronize(stream));
             if (tiles()) set_flip(ctl_h->parity);
             if (!ctl_h->active) break;
-            ahead = kStepsPerRead;
-            if (fixed_dt == 0.0) {
-                const double left = (t_end - ctl_h->t) / ctl_h->dt;  // NaN: a whole group
-                if (left < kStepsPerRead) ahead = (long long)left + 1;
-            }
+            n = std::max(1ll, std::min(steps_left(), budget));
         }
         auto t1 = std::chrono::high_resolution_clock::now();
         last_ms = std::chrono::duration_cast<std::chrono::microseconds>(t1 - t0).count() / 1000.0;
@@ -375,17 +401,18 @@ struct fvm2d_solver {
     }
 };
 
-int fvm2d_solver::enqueue_steps(long long n, cudaEvent_t *ev)
+int fvm2d_solver::enqueue_steps(long long to, cudaEvent_t *ev, long long from, bool open)
 {
     const Variant &v = kVariants[precision];
     LaunchConfig c = config();
     if (!tiles()) {
-        for (long long k = 0; k < n; ++k) CK(v.step(c, stream, ev));
+        for (long long k = from; k < to; ++k) CK(v.step(c, stream, ev));
         return FVM2D_OK;
     }
     if (ev)
         for (int q = 0; q < 4; ++q) CK(cudaEventRecord(ev[q], stream));
-    for (; c.step < n; ++c.step) CK(v.tile_step(c, stream));
+    for (c.step = int(from); c.step < to; ++c.step) CK(v.tile_step(c, stream));
+    if (open) return FVM2D_OK;
     if (ev) CK(cudaEventRecord(ev[4], stream));
     CK(v.end_steps(c, stream));
     if (ev) CK(cudaEventRecord(ev[5], stream));

@@ -3,7 +3,7 @@
 // decisions can be tested without a GPU (tests/test_batch_runtime_host.py).
 // Build k's tile of shape s is (k + 1) x (s + 1) tiles a problem; a step takes
 // step_ms[1] in tiles and step_ms[0] sweep by sweep, and the first of the
-// process first_ms more.  Problem p ends after 20 + stagger p steps.
+// process first_ms more.  Problem p ends after ends + stagger p steps.
 #include "fake_cudart.h"
 
 #include "../2d_fvm_cuda_b200/csrc/fvm2d_batch_control.h"
@@ -14,7 +14,7 @@ using fvm2d::StepControl;
 namespace {
 const BatchLaunch *last = nullptr;
 double step_ms[2] = {2.0, 1.0}, first_ms = 0.0;
-int stagger = 0;
+int ends = 20, stagger = 0;
 long fail_at = -1;            // this sweep by sweep group fails
 long groups = 0, bad = 0;     // groups of sweeps; steps whose tile plan was not their build's
 long tile_steps = 0, sweep_steps = 0, mixed = 0;
@@ -28,8 +28,9 @@ void run_steps(long n, int tiles)
         StepControl &c = last->ctl[p];
         if (!c.active) continue;
         c.steps += int(n);
+        c.t += n * c.dt;
         c.parity ^= tiles ? int(n & 1) : 0;
-        const int end = c.step_limit < 20 + stagger * p ? c.step_limit : 20 + stagger * p;
+        const int end = c.step_limit < ends + stagger * p ? c.step_limit : ends + stagger * p;
         if (c.steps >= end) c.steps = end, c.active = 0;
     }
 }
@@ -44,7 +45,7 @@ cudaError_t init(const BatchLaunch &L)
 {
     last = &L;
     fake::graph_launch = graph;
-    for (int p = 0; p < L.np; ++p) L.ctl[p].active = 1, L.ctl[p].dt = 1e-300;
+    for (int p = 0; p < L.np; ++p) L.ctl[p].active = 1, L.ctl[p].dt = L.prob[p].plan.t_end / (ends + stagger * p);
     return cudaSuccess;
 }
 long long tiles_of(int build, int shape) { return (build + 1) * (shape + 1); }
@@ -95,6 +96,7 @@ void br_set(double sweep, double tile, double first, long fail, int apart)
     step_ms[0] = sweep, step_ms[1] = tile, first_ms = first, fail_at = fail;
     groups = bad = tile_steps = sweep_steps = mixed = 0;
 }
+void br_ends(int n) { ends = n; }
 // steps in tiles, steps sweep by sweep, steps whose plan was another build's,
 // calls that mixed the two ways
 void br_seen(long *out) { out[0] = tile_steps, out[1] = sweep_steps, out[2] = bad, out[3] = mixed; }

@@ -9,6 +9,8 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <string>
 #include <vector>
 
 namespace fake {
@@ -21,6 +23,14 @@ inline double clock_ms = 0.0;
 inline int captured = -1;                     // steps captured so far; -1: no capture
 inline cudaError_t (*graph_launch)(long) = nullptr;  // a graph of that many captured steps
 inline int resident = 4;                      // blocks per SM that the occupancy call answers
+
+// the kernels' (mangled) names, and what a test does in a kernel's place
+inline std::map<const void *, std::string> &names()
+{
+    static std::map<const void *, std::string> m;
+    return m;
+}
+inline void (*on_kernel)(const std::string &name, void **args) = nullptr;
 
 // buffers that count as a caller's device memory, and the copies from and to them
 struct Range {
@@ -127,7 +137,12 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const
     *n = fake::resident;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *, dim3 g, dim3 b, void **, size_t m, cudaStream_t) { return fake::note(g, b, m); }
+cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **args, size_t m, cudaStream_t)
+{
+    if (cudaError_t e = fake::note(g, b, m)) return e;
+    if (fake::on_kernel) fake::on_kernel(fake::names()[f], args);
+    return cudaSuccess;
+}
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **)
 {
     return fake::note(c->gridDim, c->blockDim, c->dynamicSmemBytes);
@@ -143,6 +158,9 @@ cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *m, void *s)
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
 void __cudaRegisterFatBinaryEnd(void **) {}
 void __cudaUnregisterFatBinary(void **) {}
-void __cudaRegisterFunction(void **, const char *, char *, const char *, int, void *, void *, void *, void *, int *) {}
+void __cudaRegisterFunction(void **, const char *f, char *, const char *name, int, void *, void *, void *, void *, int *)
+{
+    fake::names()[f] = name;
+}
 void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
 } // extern "C"

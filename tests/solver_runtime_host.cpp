@@ -25,8 +25,14 @@ void plan(StepControl *c, const LaunchConfig &l)
     c->dt = step_dt < l.plan.t_end - c->t ? step_dt : l.plan.t_end - c->t;
     c->active = 1;
 }
+void kernel(const std::string &name, void **args)
+{
+    if (name.find("show_record") != std::string::npos)
+        **static_cast<StepControl **>(args[1]) = **static_cast<const StepControl **>(args[0]);
+}
 cudaError_t init(const LaunchConfig &l)
 {
+    fake::on_kernel = kernel;
     plan(l.ctl, l);
     return cudaSuccess;
 }

@@ -78,7 +78,7 @@ def test_autotuning_times_no_first_run(lib, batch):
     assert lib.fvm2d_batch_autotune(batch, 2, None, None) == 0
     lib.br_set(2.0, 1.0, 0.0, -1, 0)
     assert lib.fvm2d_batch_solve(batch) == 0
-    assert seen(lib) == {"tiles": 32, "sweeps": 0, "wrong_plan": 0, "mixed": 0}
+    assert seen(lib) == {"tiles": 20, "sweeps": 0, "wrong_plan": 0, "mixed": 0}
     lib.br_set(1.0, 2.0, 0.0, -1, 0)
     assert lib.fvm2d_batch_autotune(batch, 2, None, None) == 0
     lib.br_set(1.0, 2.0, 0.0, -1, 0)
@@ -94,4 +94,21 @@ def test_a_failed_autotuning_leaves_the_batch_as_it_was(lib, batch, trial):
     assert lib.fvm2d_batch_autotune(batch, 2, None, None) != 0
     lib.br_set(2.0, 1.0, 0.0, -1, 0)
     assert lib.fvm2d_batch_solve(batch) == 0
-    assert seen(lib) == {"tiles": 32, "sweeps": 0, "wrong_plan": 0, "mixed": 0}
+    assert seen(lib) == {"tiles": 20, "sweeps": 0, "wrong_plan": 0, "mixed": 0}
+
+
+@pytest.mark.parametrize("n", [40, 2100])
+def test_few_steps_are_enqueued_past_the_end(lib, n):
+    b = ctypes.c_void_p()
+    sizes = (ctypes.c_int * 1)(n)
+    assert lib.fvm2d_batch_create(ctypes.byref(b), 1, sizes, sizes) == 0
+    cells = np.ones((n, n, 4))
+    assert lib.fvm2d_batch_set_problem(b, 0, 1.0, 1.0, 1.0, 0.4, 1.9, 1.4, 0) == 0
+    assert lib.fvm2d_batch_set_state(b, 0, ctypes.c_void_p(cells.ctypes.data), 4) == 0
+    for ends in (20, 3):  # steps to the end; a first group of 16 where steps are cheap
+        lib.br_set(2.0, 1.0, 0.0, -1, 0)
+        lib.br_ends(ends)
+        assert lib.fvm2d_batch_solve(b) == 0
+        assert ends <= seen(lib)["tiles"] <= (ends + 1 if n > 2000 else max(16, ends + 1))
+    lib.br_ends(20)
+    lib.fvm2d_batch_destroy(b)

@@ -58,3 +58,35 @@ def test_device_buffers_are_used_in_place_only_if_they_are_long_enough(lib, hand
         assert lib.sr_device_copies() == copies
     lib.sr_device(None, 0)
     assert CALLS[call](lib, handle, ctypes.c_void_p(start)) == OK  # host memory
+
+
+@pytest.mark.parametrize("n,first", [(24, 16), (800, 13), (2100, 1)])  # cells a side; steps before the first look
+@pytest.mark.parametrize("call", ["solve", "advance"])
+def test_few_steps_are_enqueued_past_the_end(lib, n, first, call):
+    """A run that ends early leaves few steps that do nothing: each of them loads
+    the array."""
+    h = ctypes.c_void_p()
+    assert lib.fvm2d_create(ctypes.byref(h), n, n) == OK
+    state, out, done = np.ones((n, n, 4)), (ctypes.c_long * 3)(), ctypes.c_int(0)
+    for steps in (0, 1, 2, 3, 13, 16, 17, 60, 128, 129, 300):
+        lib.sr_run(0.25)  # (exact in binary)
+        assert lib.fvm2d_set_end_time(h, 0.25 * steps) == OK
+        assert lib.fvm2d_set_state(h, ctypes.c_void_p(state.ctypes.data), 4) == OK
+        assert (lib.fvm2d_solve(h) if call == "solve" else lib.fvm2d_advance(h, 1000, ctypes.byref(done))) == OK
+        lib.sr_seen(out)
+        enqueued, ran, groups = out
+        assert ran == steps and (call == "solve" or done.value == steps)
+        assert enqueued <= max(first, steps + 1), (steps, list(out))
+        assert groups <= 2 + steps // 100
+    lib.fvm2d_destroy(h)
+
+
+def test_a_short_advance_is_one_group(lib, handle):
+    state, out, done = np.ones((NY, NX, 4)), (ctypes.c_long * 3)(), ctypes.c_int(0)
+    assert lib.fvm2d_set_end_time(handle, 1e9) == OK
+    assert lib.fvm2d_set_state(handle, ctypes.c_void_p(state.ctypes.data), 4) == OK
+    for n in (1, 2, 16):
+        lib.sr_run(0.25)
+        assert lib.fvm2d_advance(handle, n, ctypes.byref(done)) == OK and done.value == n
+        lib.sr_seen(out)
+        assert list(out) == [n, n, 1]
