@@ -784,19 +784,21 @@ struct Hoisted {
                                                         const Cell<Real> &FR, const Consts &K)
     {
         const Real half = Real(0.5);
-        // W + lambda (F_L - F_R), the change rounded before the conserved value
-        // it joins: one rounding of each component
+        // W + lambda (F_L - F_R): momenta with the change rounded before the
+        // product it joins, one rounding each; the energy with the pressure's
+        // part rounded by itself, as the reference does (with the change rounded
+        // first, pressures ended 1.5 to 2.4 times as far from the formulas in
+        // the reference's order, over 40 steps of four flows)
         const Real m0 = fma(FL.rho - FR.rho, K.lambda, U.rho);
         const Real m1 = fma(U.rho, U.un, (FL.p - FR.p) * K.lambda);
-        const Real m2 = fma(U.p, K.igm1,
-                            fma(FL.un - FR.un, K.lambda, (half * U.rho) * fma(U.un, U.un, U.ut * U.ut)));
+        const Real m2 = fma(FL.un - FR.un, K.lambda, fma(half * U.rho, fma(U.un, U.un, U.ut * U.ut), U.p * K.igm1));
         const Real m3 = fma(U.rho, U.ut, (FL.ut - FR.ut) * K.lambda);
         const Real ir = rrcp(m0);
         Cell<Real> o;
         o.rho = m0;
         o.un = m1 * ir;
         o.ut = m3 * ir;
-        o.p = K.gm1 * fma(-(half * fma(m1, m1, m3 * m3)), ir, m2);
+        o.p = K.gm1 * fma(-(half * fma(m3, m3, m1 * m1)), ir, m2);
         return o;
     }
 };
