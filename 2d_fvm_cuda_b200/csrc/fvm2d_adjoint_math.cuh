@@ -20,20 +20,8 @@ struct Cell5 {
 };
 
 // ---- limiter -------------------------------------------------------------
-// s = Hoisted::slope's limiter (limited_slope_hoisted) on (m, c, p): which
-// difference was selected (0 none, 1 central, 2 backward, 3 forward), for the
-// adjoint.  Same tests and tie order (d1 d2 > 0 alone: it implies dc d2 > 0).
-__device__ __forceinline__ int slope_choice(A m, A c, A p, A rh, A alpha)
-{
-    const A d1 = c - m, d2 = p - c, dc = p - m;
-    if (!(d1 * d2 > A(0))) return 0;
-    const A a1 = fabs(d1), a2 = fabs(d2);
-    const A inner = (rh * alpha) * ((a2 < a1) ? a2 : a1);
-    if (!(inner < fabs(dc) * (rh * A(0.5)))) return 1;
-    return (a2 < a1) ? 3 : 2;
-}
-
-// The slope itself (Hoisted's limiter) with its choice.
+// The slope itself (Hoisted's limiter) with its choice: which difference was
+// selected (0 none, 1 central, 2 backward, 3 forward), for the adjoint.
 __device__ __forceinline__ A slope_with_choice(A m, A c, A p, A hrh, A rha, int &choice)
 {
     const A d1 = c - m, d2 = p - c, dc = p - m;
@@ -54,6 +42,20 @@ __device__ __forceinline__ A slope_parts(int choice, A sbar, A hrh, A rha, A &mb
     return choice & 1 ? x : A(0);
 }
 
+#if !defined(__CUDACC__)  // host builds: the limiter's choice and adjoint each by itself, for tests
+// s = Hoisted::slope's limiter (limited_slope_hoisted) on (m, c, p): which
+// difference was selected (0 none, 1 central, 2 backward, 3 forward), for the
+// adjoint.  Same tests and tie order (d1 d2 > 0 alone: it implies dc d2 > 0).
+__device__ __forceinline__ int slope_choice(A m, A c, A p, A rh, A alpha)
+{
+    const A d1 = c - m, d2 = p - c, dc = p - m;
+    if (!(d1 * d2 > A(0))) return 0;
+    const A a1 = fabs(d1), a2 = fabs(d2);
+    const A inner = (rh * alpha) * ((a2 < a1) ? a2 : a1);
+    if (!(inner < fabs(dc) * (rh * A(0.5)))) return 1;
+    return (a2 < a1) ? 3 : 2;
+}
+
 // Adds the adjoint of one slope component (sbar) to its three cells.
 __device__ __forceinline__ void slope_adjoint(int choice, A sbar, A rh, A alpha, A &mbar, A &cbar, A &pbar)
 {
@@ -68,6 +70,7 @@ __device__ __forceinline__ void slope_adjoint(int choice, A sbar, A rh, A alpha,
         cbar -= rh * alpha * sbar;
     }
 }
+#endif
 
 // ---- conservative update ---------------------------------------------------
 // Adjoint of Hoisted::update.  Given the output adjoint Ub (rho, p, un, ut),
