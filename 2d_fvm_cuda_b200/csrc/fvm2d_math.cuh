@@ -663,22 +663,22 @@ struct Hoisted {
         const Fan w = fan(L, R, sL, sR, K, sound);
         const float irl = w.irl, irr = w.irr, c_lx = w.c_lx, c_rx = w.c_rx, c_l = w.c_l, c_r = w.c_r;
         const float icl = w.icl, icr = w.icr, isum = w.isum, sl = w.sl, sr = w.sr;
-        const float e_l = pi_l * irl * igm1, e_r = pi_r * irr * igm1;
-        // (gamma - 1) e_x
-        const float g_lx = cfma(-(pi_l * rho_lx), irl, pi_lx) * irl, g_rx = cfma(-(pi_r * rho_rx), irr, pi_rx) * irr;
+        // a side's e and (gamma - 1) e_x, wanted on one side only
+        auto energy = [&](float p, float ir) { return p * ir * igm1; };
+        auto energy_x = [&](float p, float rho_x, float p_x, float ir) { return cfma(-(p * rho_x), ir, p_x) * ir; };
         Interface<float> o;
         if (u_l - sl >= zero) {
-            o.rho = rho_l; o.p = pi_l; o.un = u_l; o.ut = v_l; o.e = e_l;
+            o.rho = rho_l; o.p = pi_l; o.un = u_l; o.ut = v_l; o.e = energy(pi_l, irl);
             o.rho_t = cfma(-rho_l, u_lx, -(u_l * rho_lx));
             o.un_t = cfma(-u_l, u_lx, -(pi_lx * irl));
-            o.e_t = cfma(-u_l, g_lx * igm1, -(pi_l * irl * u_lx));
+            o.e_t = cfma(-u_l, energy_x(pi_l, rho_lx, pi_lx, irl) * igm1, -(pi_l * irl * u_lx));
             o.ut_t = -u_l * v_lx;
             o.p_t = cfma(-u_l, pi_lx, -(c_l * sl * u_lx));
         } else if (u_r + sr <= zero) {
-            o.rho = rho_r; o.p = pi_r; o.un = u_r; o.ut = v_r; o.e = e_r;
+            o.rho = rho_r; o.p = pi_r; o.un = u_r; o.ut = v_r; o.e = energy(pi_r, irr);
             o.rho_t = cfma(-rho_r, u_rx, -(u_r * rho_rx));
             o.un_t = cfma(-u_r, u_rx, -(pi_rx * irr));
-            o.e_t = cfma(-u_r, g_rx * igm1, -(pi_r * irr * u_rx));
+            o.e_t = cfma(-u_r, energy_x(pi_r, rho_rx, pi_rx, irr) * igm1, -(pi_r * irr * u_rx));
             o.ut_t = -u_r * v_rx;
             o.p_t = cfma(-u_r, pi_rx, -(c_r * sr * u_rx));
         } else {
@@ -696,11 +696,11 @@ struct Hoisted {
             if (u <= zero) {
                 const float irho = (u_r - u + sr) * icr;
                 const float rho = rrcp(irho), icr2 = icr * icr;
-                const float e = cfma((pm - pi_r) * (pm + pi_r) * half, icr2, e_r);
+                const float e_r = energy(pi_r, irr), e = cfma((pm - pi_r) * (pm + pi_r) * half, icr2, e_r);
                 const float rho3 = rho * rho * rho, urho = u * rho;
                 const float h_l = cfma(urho, icr, one), h_r = cfma(-urho, icl, one);
                 const float S = cfma(1.5f * (u - u_r), c_rx, cfma(sr * sr, rho_rx, -cu_r));
-                const float G = cfma(2.f * (e_r - e) * c_rx, icr, cfma(g_rx, igm1, -(pi_r * pi_rx * icr2)));
+                const float G = cfma(2.f * (e_r - e) * c_rx, icr, cfma(energy_x(pi_r, rho_rx, pi_rx, irr), igm1, -(pi_r * pi_rx * icr2)));
                 o.rho = rho; o.e = e; o.ut = v_r;
                 o.rho_t = cfma(rho3 * icr2 * icr * cfma(c_r, irho, u), Dp, -u * rho3 * irr * icr2 * S);
                 o.p_t = isum * cfma(c_r * sl * h_l, k_l, -(c_l * sr * h_r * k_r));
@@ -710,11 +710,11 @@ struct Hoisted {
             } else {
                 const float irho = (u - u_l + sl) * icl;
                 const float rho = rrcp(irho), icl2 = icl * icl;
-                const float e = cfma((pm - pi_l) * (pm + pi_l) * half, icl2, e_l);
+                const float e_l = energy(pi_l, irl), e = cfma((pm - pi_l) * (pm + pi_l) * half, icl2, e_l);
                 const float rho3 = rho * rho * rho, urho = u * rho;
                 const float h_l = cfma(urho, icr, one), h_r = cfma(-urho, icl, one);
                 const float S = cfma(1.5f * (u - u_l), c_lx, cfma(sl * sl, rho_lx, cu_l));
-                const float G = cfma(2.f * (e_l - e) * c_lx, icl, cfma(g_lx, igm1, -(pi_l * pi_lx * icl2)));
+                const float G = cfma(2.f * (e_l - e) * c_lx, icl, cfma(energy_x(pi_l, rho_lx, pi_lx, irl), igm1, -(pi_l * pi_lx * icl2)));
                 o.rho = rho; o.e = e; o.ut = v_l;
                 o.rho_t = cfma(-u * rho3 * irl * icl2, S, -(rho3 * icl2 * icl * cfma(-c_l, irho, u) * Dp));
                 o.p_t = isum * cfma(c_r * sl * h_l, k_l, -(c_l * sr * h_r * k_r));
