@@ -31,5 +31,9 @@
 #define FVM2D_TILE2_MINB 3
 #define FVM2D_TILE3_WARPS 10
 #define FVM2D_TILE3_MINB 2
+// (us per step around 0.9 x the resident blocks, the NEEDs of fvm2d_variant.inc:
+// 30 x 30 against 30 x 14, 592 blocks: 610^2, 441 tiles, 43.9 / 40.3; 700^2, 576,
+// 43.8 / 50.6.  30 x 14 against 14 x 14, 444: 330^2, 264, 20.2 / 17.7; 400^2, 406,
+// 20.3 / 21.6)
 #include "fvm2d_packed.cuh"
 #include "fvm2d_variant.inc"

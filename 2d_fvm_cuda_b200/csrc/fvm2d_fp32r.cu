@@ -30,6 +30,9 @@
 #define FVM2D_TILE2_MINB 3
 #define FVM2D_TILE3_WARPS 10
 #define FVM2D_TILE3_MINB 2
+// (30 x 30 against 30 x 14 around 1.5 x 296 tiles, us per step: 520^2, 324 tiles,
+// 37.8 / 35.6; 700^2, 576, 51.1 / 56.1; where one wave of 30 x 30 is nearly full
+// the smaller shape loses: 460^2, 256, 27.7 / 32.2)
 #define FVM2D_TILE0_NEED 1.5
 #include "fvm2d_packed.cuh"
 #include "fvm2d_variant.inc"

@@ -26,6 +26,9 @@
 #define FVM2D_TILE2_MINB 1
 #define FVM2D_TILE3_WARPS 10
 #define FVM2D_TILE3_MINB 1
+// 30 x 30 against 30 x 14 around 2 x 148 tiles: 400^2, 196 tiles, 87 / 73; 520^2,
+// 324, 119 / 118; 610^2, 441, 128 / 155.  30 x 14 against 14 x 14 around 2 x 148:
+// 280^2, 200, 50 / 41; 330^2, 264, 50 / 54; 400^2, 406, 73 / 78.
 #define FVM2D_TILE0_NEED 2
 #define FVM2D_TILE1_NEED 2
 #include "fvm2d_quotient.cuh"

@@ -92,7 +92,9 @@ __global__ void plan_from_kernel(StepControl *c, PlanParams p, const double *sma
 // its predecessor on the stream is still running; pdl_wait returns once the
 // predecessor has completed and its writes are visible (at once in a kernel
 // launched without it).  Every thread of such a kernel calls it before it
-// touches global memory, so completion stays in stream order.
+// touches memory that a step writes, so completion stays in stream order.  (The
+// batch's kernels look their problem up before it, in the prefix counts t0 and
+// rb0: the host writes those only between groups, with no step in flight.)
 __device__ __forceinline__ void pdl_wait()
 {
 #if defined(__CUDA_ARCH__)

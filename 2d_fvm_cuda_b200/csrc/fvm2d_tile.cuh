@@ -28,16 +28,17 @@
 //
 // So the four sweeps' intermediate states never leave the SM: 64 bytes per
 // FP64 cell and step in place of 288, one launch in place of five.  Work on
-// the two halo cells is done again by the neighbouring tiles (30 x 30: 128
-// warp tasks for 900 cells, 12% over four sweeps without overlap), which the
-// shorter instruction stream (no global addresses, clamps, carries or ring
-// copies per sweep: 476 slots per task against 430-640 per cell and sweep)
-// repays even where the array is large.  What bounds a tile is FP64 latency
-// and issue: FP64 pipe 59%, issue slots 60% busy at 20 warps per SM.
+// the two halo cells is done again by the neighbouring tiles (30 x 30: 128 warp
+// tasks where four sweeps of 900 cells fill 112.5: 14%), which the shorter
+// instruction stream (no global addresses, clamps, carries or ring copies per
+// sweep: 433 slots per task of 32 interfaces, in the quadrants at 2048^2,
+// against 460-650 per 32 cells of a sweep kernel) repays even where the array is
+// large.  What bounds a tile is FP64 latency and issue: FP64 pipe 57%, issue
+// slots 61% busy at 20 warps per SM.
 //
 // Against the sweep kernels with the same arithmetic (FP64,
 // us per step of a varied four-quadrant flow): 400^2 58 -> 27, 131 x 517
-// 48 -> 16, 1003^2 164 -> 111, 4096^2 1830 -> 1640; FP32 4096^2 1240 -> 1070.
+// 48 -> 16, 1003^2 164 -> 111, 4096^2 1810 -> 1600; FP32 4096^2 1270 -> 1200.
 //
 // A warp task is 32 interfaces, one per lane: a lane holds cell c of a line,
 // computes its limited slope, takes the slope of c-1 from its neighbour by
