@@ -397,8 +397,7 @@ __device__ __forceinline__ Real limited_slope_hoisted(Real m, Real c, Real p, Re
 // hence |dc d2| >= |d1 d2| > 0; then dc != 0 and the result takes its sign.
 // The minima are formed for every cell and selected: four fields without a
 // branch between them overlap their chains (4096^2 step of a varied flow in
-// tiles: 1627 -> 1587 us; a branch around the minima pays only where the
-// flow is constant).
+// tiles: 1627 -> 1587 us).
 __device__ __forceinline__ double limited_slope_hoisted(double m, double c, double p, double hrh, double rha)
 {
     const double d1 = c - m, d2 = p - c, dc = p - m;
@@ -414,6 +413,24 @@ __device__ __forceinline__ float limited_slope_hoisted(float m, float c, float p
     const float d1 = c - m, d2 = p - c, dc = p - m;
     const float a = fminf(fabsf(dc) * hrh, rha * fminf(fabsf(d1), fabsf(d2)));
     return d1 * d2 > 0.f ? copysignf(a, dc) : 0.f;
+}
+
+// The limiter as a kernel with constants of type Consts takes it.  The sweep
+// kernels, which wait more for memory, gain nothing by the select (4096^2 slab
+// step of a varied flow 1816 us with a branch around the minima, 1808 with the
+// select) and lose where the flow is constant (plain quadrants: 1591, 1722): the
+// branch, with the same result.
+template <typename Real, class Consts>
+__device__ __forceinline__ Real limiter(Real m, Real c, Real p, Real hrh, Real rha, const Consts &)
+{
+    return limited_slope_hoisted(m, c, p, hrh, rha);
+}
+__device__ __forceinline__ double limiter(double m, double c, double p, double hrh, double rha,
+                                          const SweepConsts<double> &)
+{
+    const double d1 = c - m, d2 = p - c, dc = p - m;
+    if (d1 * d2 > 0.0) return copysign(rmin(fabs(dc) * hrh, rha * rmin(fabs(d1), fabs(d2))), dc);
+    return 0.0;
 }
 
 // Products of the constants of a sweep, formed where they are used; a kernel
@@ -445,10 +462,10 @@ struct Hoisted {
     {
         Cell<Real> s;
         const Real hrh = half_rh(K), rha = alpha_rh(K);
-        s.rho = limited_slope_hoisted(m.rho, c.rho, p.rho, hrh, rha);
-        s.p = limited_slope_hoisted(m.p, c.p, p.p, hrh, rha);
-        s.un = limited_slope_hoisted(m.un, c.un, p.un, hrh, rha);
-        s.ut = limited_slope_hoisted(m.ut, c.ut, p.ut, hrh, rha);
+        s.rho = limiter(m.rho, c.rho, p.rho, hrh, rha, K);
+        s.p = limiter(m.p, c.p, p.p, hrh, rha, K);
+        s.un = limiter(m.un, c.un, p.un, hrh, rha, K);
+        s.ut = limiter(m.ut, c.ut, p.ut, hrh, rha, K);
         return s;
     }
     // The reference's formulas (src/basicFuns.cuh:86-189) with common parts
